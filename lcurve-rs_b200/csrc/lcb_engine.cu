@@ -2,7 +2,7 @@
 //
 // A batch runs as one launch sequence on the context's stream:
 //   memset(aux, status, counter) -> k_phase -> k_elements -> k_roche (or, for
-//   small batches, k_roche_scan -> k_roche_chop2) -> k_aux -> k_flux -> k_epilogue
+//   small batches, k_roche_scan -> k_roche_chop2) -> k_aux -> k_flux -> k_curve -> k_results
 // For a resident batch (lcb_batch_*) the sequence is captured once in a CUDA
 // graph and replayed; between runs only the model table and the tables
 // derived from it are uploaded, and the graph is rebuilt only when the
@@ -76,11 +76,11 @@ struct DevBuf {
 struct DeviceSet {
     DevBuf models, segs, bands, rings, eblocks, rblocks, ablocks, units, dmodel, dsub0, dsrc, data;
     DevBuf rec, pos, p64, d64, ecl, egrp, aux, status, spe, spphi, sptype, spw, slfac, partial, calc, results, counter,
-        datum, ecount, fcomp, svda, firsthit;
+        datum, ecount, fcomp, svda, firsthit, episum;
     void release() {
         for (DevBuf* b : {&models, &segs, &bands, &rings, &eblocks, &rblocks, &ablocks, &units, &dmodel, &dsub0, &dsrc,
                           &data, &rec, &pos, &p64, &d64, &ecl, &egrp, &aux, &status, &spe, &spphi, &sptype, &spw, &slfac,
-                          &partial, &calc, &results, &counter, &datum, &ecount, &fcomp, &svda, &firsthit})
+                          &partial, &calc, &results, &counter, &datum, &ecount, &fcomp, &svda, &firsthit, &episum})
             b->release();
     }
 };
@@ -135,6 +135,9 @@ namespace {
 // Upload of the plan's tables (and the data) into a device set.
 // Words of the per-group eclipse slot masks (one per kEclGroup elements).
 size_t ecl_groups(const lcb::Plan& P) { return (size_t)((P.nelem + lcb::kEclGroup - 1) / lcb::kEclGroup); }
+
+// Doubles of the epilogue's per-block sums: four per k_curve block, one per k_results block.
+size_t epi_sums(const lcb::Plan& P) { return P.models.size() * (size_t)(4 * P.curve_blocks + P.result_blocks); }
 
 // `prev` (a resident batch's previous plan, its tables already on the device):
 // tables equal to prev's are not uploaded again (a re-parameterised batch of
@@ -197,6 +200,7 @@ void upload_plan(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, const lcb_datum* 
     D.partial.ensure(P.npartial * sizeof(double));
     D.calc.ensure(P.ndatum * sizeof(double));
     D.results.ensure(nm * 12 * sizeof(double));
+    D.episum.ensure(epi_sums(P) * sizeof(double));
     D.counter.ensure(sizeof(int) * 4);
     D.ecount.ensure(sizeof(unsigned long long) * 8);
     const size_t ncomp = P.any_iscale ? (size_t)P.ndatum * 5 : 1;
@@ -206,7 +210,7 @@ void upload_plan(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, const lcb_datum* 
 }
 
 // Parts of the launch sequence: the element stage (grids, continuum, eclipses:
-// k_elements, k_roche) and the rest (k_phase, k_aux, k_flux, k_epilogue).
+// k_elements, k_roche) and the rest (k_phase, k_aux, k_flux, k_curve, k_results).
 constexpr int kStageElements = 1, kStageRest = 2, kStagesAll = 3;
 
 // The device launch sequence of one batch evaluation.  nblk / nrblk (>= 0)
@@ -261,7 +265,9 @@ void enqueue_run(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, int scale, int rd
     lcb::EpiArgs pe{D.models.as<lcb::ModelDev>(), D.datum.as<lcb_datum>(), D.dsub0.as<int64_t>(),
                     D.spphi.as<double>(), D.spw.as<double>(), D.slfac.as<double>(), D.partial.as<double>(),
                     D.aux.as<double>(), D.status.as<int>(), scale, rdata, D.calc.as<double>(),
-                    D.results.as<double>(), D.fcomp.as<double>(), D.svda.as<double>(), nm, sz, D.status.as<int>()};
+                    D.results.as<double>(), D.fcomp.as<double>(), D.svda.as<double>(), D.episum.as<double>(),
+                    D.episum.as<double>() + nm * 4 * P.curve_blocks, nm, P.curve_blocks, P.result_blocks, P.curve_share, sz,
+                    D.status.as<int>()};
     CUDA_TRY(lcb::launch_epilogue(pe, s));
     if (timed) CUDA_TRY(cudaEventRecord(C->ev[6], s));
 }
@@ -1143,6 +1149,7 @@ size_t noalloc_carve(const lcb::Plan& P, unsigned char* base, DeviceSet& D) {
     take(D.partial, P.npartial * sizeof(double));
     take(D.calc, P.ndatum * sizeof(double));
     take(D.results, nm * 12 * sizeof(double));
+    take(D.episum, epi_sums(P) * sizeof(double));
     take(D.counter, sizeof(int) * 4);
     take(D.ecount, sizeof(unsigned long long) * 8);
     const size_t ncomp = P.any_iscale ? (size_t)P.ndatum * 5 : 1;

@@ -34,6 +34,7 @@ enum AuxSlot : int32_t {
     AUX_SPEC0 = 0,           // 0..8: raw comp_star sums at the special phases
     AUX_FG1 = 9, AUX_F1 = 10, AUX_FG2 = 11, AUX_F2 = 12,   // logg sums (flux.rs:288-322)
     AUX_SA1 = 13, AUX_VOL1 = 14, AUX_SA2 = 15, AUX_VOL2 = 16,  // rv sums (flux.rs:347-373)
+    AUX_DONE = 17,           // as unsigned: k_results blocks of the model that have finished
 };
 
 struct RocheEcl {          // constants of a Roche-distorted eclipsing star

@@ -29,11 +29,12 @@
 //                Visibility is decided exactly in FP64 per (element, tile)
 //                and per sub-phase only where an eclipse edge falls inside
 //                the tile.
-//   k_epilogue : one block per model: ginterp scale factors, exposure
-//                smearing, slope/third, chi-squared / re_scale
-//                (orchestration.rs:243-310, 361-401), and with iscale = 1 the
-//                per-component fluxes and their one-sided Jacobi SVD scale
-//                factors (405-436).
+//   k_curve    : per datum, the slots' partial sums under the ginterp scale
+//                factors, exposure smearing, slope/third (orchestration.rs:
+//                243-310), in tiles of 32 data per block.
+//   k_results  : per model, re_scale and chi-squared (361-401), log g, radii,
+//                and with iscale = 1 the per-component fluxes and their
+//                one-sided Jacobi SVD scale factors (405-436).
 #include <algorithm>
 #include <cfloat>
 #include <cstdint>
@@ -1749,7 +1750,7 @@ __global__ void __launch_bounds__(kFluxThreads, 5) k_flux(FluxArgs A) {
 }
 
 // ---------------------------------------------------------------------------
-// k_epilogue
+// k_curve, k_results
 // ---------------------------------------------------------------------------
 struct Gint {  // types.rs:130-202
     double p1, p2, s11, s12, s21, s22;
@@ -1930,111 +1931,210 @@ __device__ void epilogue_iscale(const EpiArgs& A, const ModelDev& M, const Gint&
     }
 }
 
-__global__ void __launch_bounds__(kEpiThreads) k_epilogue(EpiArgs A) {
+// The ginterp scale factors of a model (orchestration.rs:86-131, with the live
+// Ginterp) and its white-dwarf flux.
+__device__ Gint model_gint(const ModelDev& M, const double* aux, double& s_wd) {
+    Gint g{M.phase1, M.phase2, 1.0, 1.0, 1.0, 1.0};
+    auto c1 = [&](int s) { return g.scale1(M.spec[s].phase) * aux[AUX_SPEC0 + s]; };
+    auto c2 = [&](int s) { return g.scale2(M.spec[s].phase) * aux[AUX_SPEC0 + s]; };
+    if (!M.copy1) {
+        g.s11 = c1(M.spec_g11[0]) / c1(M.spec_g11[1]);
+        g.s12 = c1(M.spec_g12[0]) / c1(M.spec_g12[1]);
+    }
+    if (!M.copy2) {
+        g.s21 = c2(M.spec_g21[0]) / c2(M.spec_g21[1]);
+        g.s22 = c2(M.spec_g22[0]) / c2(M.spec_g22[1]);
+    }
+    s_wd = g.scale1(0.5) * aux[AUX_SPEC0 + M.spec_wd];
+    return g;
+}
+
+// Fluxes: per datum, the sum of its slots' partial sums under the ginterp
+// factors, trapezoid over the exposure (orchestration.rs:243-310); and per
+// block the sums that re_scale and the chi-squared need.  A tile is 32 data, a
+// warp's lanes.  Bound by reading the partial sums (8 B a slot and sub-phase).
+// kShare = 1: each warp takes tiles of its own.  kShare = 8 (few tiles: one
+// long light curve): the block's eight warps share a tile's slots, which makes
+// eight times the warps; one block per model took 48.7 ms for 1,240 slots x
+// 110,000 sub-phases (1.74 ms here) and 1.26 ms for 110 x 50,000 (0.05 ms),
+// almost all of it latency of one SM.
+constexpr int kCurveTile = 32;
+
+template <int kShare>
+__global__ void __launch_bounds__(kEpiThreads) k_curve(EpiArgs A) {
+    constexpr int kWarps = kEpiThreads / 32, kTiles = kWarps / kShare;  // tiles a block works on at once
+    static_assert(kShare == 1 || kShare == kWarps, "a block's barriers are inside the tile loop");
     const int64_t m = blockIdx.x;
     const ModelDev& M = A.models[m];
-    double* res = A.results + m * 12;
-    __shared__ double red[kEpiThreads / 32];
-    __shared__ Gint G;
-    __shared__ double s_wd;
     const bool in_range = LCB_IN_BOUNDS(M.pbase + (int64_t)M.nslots * M.nsub <= A.sz.npartial &&
                                             M.datum_begin + M.ndatum <= A.sz.ndatum && M.sub_begin + M.nsub <= A.sz.nsub,
                                         A.bad + m);
     if (M.status < 0 || A.status[m] != 0 || !in_range) {
-        if (threadIdx.x == 0) {
-            for (int k = 0; k < 12; ++k) res[k] = NAN;
-        }
-        for (int64_t d = threadIdx.x; d < M.ndatum; d += blockDim.x) A.calc[M.datum_begin + d] = NAN;
+        for (int64_t d = (int64_t)blockIdx.y * kEpiThreads + threadIdx.x; d < M.ndatum; d += (int64_t)gridDim.y * kEpiThreads)
+            A.calc[M.datum_begin + d] = NAN;
         return;
     }
-    const double* aux = A.aux + m * kNumAux;
-    if (threadIdx.x == 0) {  // orchestration.rs:86-131 with the live Ginterp
-        Gint g{M.phase1, M.phase2, 1.0, 1.0, 1.0, 1.0};
-        auto c1 = [&](int s) { return g.scale1(M.spec[s].phase) * aux[AUX_SPEC0 + s]; };
-        auto c2 = [&](int s) { return g.scale2(M.spec[s].phase) * aux[AUX_SPEC0 + s]; };
-        if (!M.copy1) {
-            g.s11 = c1(M.spec_g11[0]) / c1(M.spec_g11[1]);
-            g.s12 = c1(M.spec_g12[0]) / c1(M.spec_g12[1]);
-        }
-        if (!M.copy2) {
-            g.s21 = c2(M.spec_g21[0]) / c2(M.spec_g21[1]);
-            g.s22 = c2(M.spec_g22[0]) / c2(M.spec_g22[1]);
-        }
-        G = g;
-        s_wd = g.scale1(0.5) * aux[AUX_SPEC0 + M.spec_wd];
+    if (M.iscale) return;  // k_results: its fluxes are per component
+    __shared__ double part[2][kShare][3][32];
+    __shared__ double red[4][kWarps];
+    __shared__ Gint G;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int share = kShare > 1 ? warp : 0;           // the warp's part of a tile's slots
+    const bool lead = share == 0;
+    if (threadIdx.x == 0) {
+        double wd;
+        G = model_gint(M, A.aux + m * kNumAux, wd);
     }
     __syncthreads();
     const Gint g = G;
-    if (M.iscale) {
-        epilogue_iscale(A, M, g, s_wd, aux, res);
-        return;
-    }
     const double* P = A.partial + M.pbase;
-    double chi = 0.0, wnok = 0.0, sdy = 0.0, syy = 0.0;
-    for (int64_t d = threadIdx.x; d < M.ndatum; d += blockDim.x) {
-        const int64_t gd = M.datum_begin + d;
-        const lcb_datum D = A.data[gd];
-        int64_t j = A.dsub0[gd] - M.sub_begin;
+    double v[4] = {0.0, 0.0, 0.0, 0.0};  // chi, wnok, sdy, syy
+    int buf = 0;
+    const int64_t step = (int64_t)gridDim.y * kTiles * kCurveTile;
+    for (int64_t d0 = ((int64_t)blockIdx.y * kTiles + (kShare > 1 ? 0 : warp)) * kCurveTile; d0 < M.ndatum; d0 += step) {
+        const int64_t d = d0 + lane, gd = M.datum_begin + d;
+        const bool on = d < M.ndatum;
+        const int ndiv = on ? A.data[gd].ndiv : 0;
+        const int64_t j0 = on ? A.dsub0[gd] - M.sub_begin : 0;
+        const int most = __reduce_max_sync(0xffffffffu, ndiv);  // the same in every warp that shares the tile
         double sum = 0.0;
-        for (int nd = 0; nd < D.ndiv; ++nd, ++j) {
-            double pn = A.sp_phi[M.sub_begin + j];
-            double s1 = 0.0, s2 = 0.0, s0 = 0.0;
-            for (int s = 0; s < M.g1_end; ++s) s1 += P[(int64_t)s * M.nsub + j];
-            for (int s = M.g1_end; s < M.g2_end; ++s) s2 += P[(int64_t)s * M.nsub + j];
-            for (int s = M.g2_end; s < M.nslots; ++s) s0 += P[(int64_t)s * M.nsub + j];
-            double ss = s1 * g.scale1(pn);
-            ss += g.scale2(pn) * s2;
-            ss += s0;
-            sum += A.sp_w[M.sub_begin + j] * ss;
+        for (int nd = 0; nd < most; ++nd, buf ^= 1) {
+            const bool act = nd < ndiv;
+            double t[3] = {0.0, 0.0, 0.0};
+            if (act) {
+                const double* q = P + j0 + nd;
+                int s = share;
+#pragma unroll 4
+                for (; s < M.g1_end; s += kShare) t[0] += q[(int64_t)s * M.nsub];
+#pragma unroll 4
+                for (; s < M.g2_end; s += kShare) t[1] += q[(int64_t)s * M.nsub];
+#pragma unroll 8
+                for (; s < M.nslots; s += kShare) t[2] += q[(int64_t)s * M.nsub];
+            }
+            if (kShare > 1) {
+                for (int k = 0; k < 3; ++k) part[buf][share][k][lane] = t[k];
+                __syncthreads();  // the other buffer is free: the lead warp read it before it came here
+                if (lead)
+                    for (int k = 0; k < 3; ++k) {
+                        t[k] = 0.0;
+                        for (int w = 0; w < kShare; ++w) t[k] += part[buf][w][k][lane];
+                    }
+            }
+            if (lead && act) {
+                const double pn = A.sp_phi[M.sub_begin + j0 + nd];
+                double ss = t[0] * g.scale1(pn);
+                ss += g.scale2(pn) * t[1];
+                ss += t[2];
+                sum += A.sp_w[M.sub_begin + j0 + nd] * ss;
+            }
         }
-        double c = A.d_slfac[gd] * (sum / (double)max(1, D.ndiv - 1)) + M.third;
-        A.calc[gd] = c;
-        if (D.weight > 0.0) {
-            if (A.scale) {
-                double w = D.weight / sq(D.ferr);
-                sdy += w * D.flux * c;
-                syy += w * c * c;
-                wnok += D.weight;
-            } else if (A.rdata) {
-                wnok += D.weight;
-                chi += D.weight * sq((D.flux - c) / D.ferr);
+        if (lead && on) {
+            const lcb_datum D = A.data[gd];
+            const double c = A.d_slfac[gd] * (sum / (double)max(1, D.ndiv - 1)) + M.third;
+            A.calc[gd] = c;
+            if (D.weight > 0.0) {
+                if (A.scale) {
+                    const double w = D.weight / sq(D.ferr);
+                    v[2] += w * D.flux * c;
+                    v[3] += w * c * c;
+                    v[1] += D.weight;
+                } else if (A.rdata) {
+                    v[1] += D.weight;
+                    v[0] += D.weight * sq((D.flux - c) / D.ferr);
+                }
             }
         }
     }
-    double sfac = 1.0;
+    block_sums(v, red);
+    if (threadIdx.x == 0)
+        for (int k = 0; k < 4; ++k) A.episum[(m * gridDim.y + blockIdx.y) * 4 + k] = v[k];
+}
+
+// Per model: the scale factor and the chi-squared (orchestration.rs:361-401)
+// from k_curve's sums, log g and radii.  gridDim.y > 1 (a light curve of many
+// data, scaled) splits the rescaled pass over blocks; the last one to finish
+// adds their chi-squared parts in block order.
+__global__ void __launch_bounds__(kEpiThreads) k_results(EpiArgs A) {
+    const int64_t m = blockIdx.x;
+    const ModelDev& M = A.models[m];
+    double* res = A.results + m * 12;
+    __shared__ double red[kEpiThreads / 32], red4[4][kEpiThreads / 32];
+    const bool in_range = M.pbase + (int64_t)M.nslots * M.nsub <= A.sz.npartial &&
+                          M.datum_begin + M.ndatum <= A.sz.ndatum && M.sub_begin + M.nsub <= A.sz.nsub;
+    if (M.status < 0 || A.status[m] != 0 || !in_range) {
+        if (blockIdx.y == 0 && threadIdx.x < 12) res[threadIdx.x] = NAN;
+        return;
+    }
+    double* aux = A.aux + m * kNumAux;
+    if (M.iscale) {
+        if (blockIdx.y > 0) return;
+        __shared__ Gint G;
+        __shared__ double s_wd;
+        if (threadIdx.x == 0) G = model_gint(M, aux, s_wd);
+        __syncthreads();
+        const Gint g = G;
+        epilogue_iscale(A, M, g, s_wd, aux, res);
+        return;
+    }
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int64_t k = threadIdx.x; k < A.curve_blocks; k += kEpiThreads)
+        for (int i = 0; i < 4; ++i) v[i] += A.episum[(m * A.curve_blocks + k) * 4 + i];
+    block_sums(v, red4);
+    double chi = v[0], wnok = v[1], sfac = 1.0;
+    const double sdy = v[2], syy = v[3];
+    bool last = blockIdx.y == 0;
     if (A.scale) {  // re_scale (orchestration.rs:361-388)
-        sdy = block_sum(sdy, red);
-        syy = block_sum(syy, red);
-        wnok = block_sum(wnok, red);
+        chi = 0.0;
         if (wnok > 0.0 && syy > 0.0) {
             sfac = sdy / syy;
-            chi = 0.0;
-            for (int64_t d = threadIdx.x; d < M.ndatum; d += blockDim.x) {
+            for (int64_t d = (int64_t)blockIdx.y * kEpiThreads + threadIdx.x; d < M.ndatum;
+                 d += (int64_t)gridDim.y * kEpiThreads) {
                 const int64_t gd = M.datum_begin + d;
                 const lcb_datum D = A.data[gd];
-                double c = A.calc[gd] * sfac;
+                const double c = A.calc[gd] * sfac;
                 A.calc[gd] = c;
                 if (D.weight > 0.0) chi += D.weight * sq((D.flux - c) / D.ferr);
             }
             chi = block_sum(chi, red);
+            if (gridDim.y > 1) {
+                __shared__ bool s_last;
+                if (threadIdx.x == 0) {
+                    A.chipart[m * gridDim.y + blockIdx.y] = chi;
+                    __threadfence();
+                    s_last = atomicAdd(reinterpret_cast<unsigned*>(aux + AUX_DONE), 1u) == gridDim.y - 1;
+                }
+                __syncthreads();
+                last = s_last;
+                if (last) {
+                    __threadfence();
+                    chi = 0.0;
+                    for (int64_t k = threadIdx.x; k < gridDim.y; k += kEpiThreads)
+                        chi += *(volatile double*)(A.chipart + m * gridDim.y + k);
+                    chi = block_sum(chi, red);
+                }
+            }
         } else {
-            chi = 0.0;
             wnok = 0.0;
         }
-    } else {
-        chi = block_sum(chi, red);
-        wnok = block_sum(wnok, red);
     }
-    if (threadIdx.x == 0) {
-        res[0] = s_wd * sfac;
-        res[1] = chi;
-        res[2] = wnok;
-        double fg1 = aux[AUX_FG1], f1 = aux[AUX_F1], fg2 = aux[AUX_FG2], f2 = aux[AUX_F2];
-        res[3] = (M.glogg1 > 0.0 && fg1 > 0.0 && f1 > 0.0) ? log10(M.glogg1 * fg1 / f1) : 0.0;
-        res[4] = (M.glogg2 > 0.0 && fg2 > 0.0 && f2 > 0.0) ? log10(M.glogg2 * fg2 / f2) : 0.0;
-        res[5] = pow(aux[AUX_VOL1] / aux[AUX_SA1], 1.0 / 3.0);
-        res[6] = pow(aux[AUX_VOL2] / aux[AUX_SA2], 1.0 / 3.0);
-        for (int k = 0; k < 5; ++k) res[7 + k] = sfac;
+    if (!last) return;
+    // a warp each for the values that need a logarithm or a power
+    const double fg1 = aux[AUX_FG1], f1 = aux[AUX_F1], fg2 = aux[AUX_FG2], f2 = aux[AUX_F2];
+    switch (threadIdx.x) {
+        case 0: {
+            double s_wd;
+            model_gint(M, aux, s_wd);
+            res[0] = s_wd * sfac;
+            res[1] = chi;
+            res[2] = wnok;
+            for (int k = 0; k < 5; ++k) res[7 + k] = sfac;
+            break;
+        }
+        case 32: res[3] = (M.glogg1 > 0.0 && fg1 > 0.0 && f1 > 0.0) ? log10(M.glogg1 * fg1 / f1) : 0.0; break;
+        case 64: res[4] = (M.glogg2 > 0.0 && fg2 > 0.0 && f2 > 0.0) ? log10(M.glogg2 * fg2 / f2) : 0.0; break;
+        case 96: res[5] = pow(aux[AUX_VOL1] / aux[AUX_SA1], 1.0 / 3.0); break;
+        case 128: res[6] = pow(aux[AUX_VOL2] / aux[AUX_SA2], 1.0 / 3.0); break;
+        default: break;
     }
 }
 
@@ -2207,7 +2307,12 @@ cudaError_t launch_flux(const FluxArgs& a, int grid, cudaStream_t s) {
 
 cudaError_t launch_epilogue(const EpiArgs& a, cudaStream_t s) {
     if (a.nmodels <= 0) return cudaSuccess;
-    k_epilogue<<<(unsigned)a.nmodels, kEpiThreads, 0, s>>>(a);
+    const dim3 grid((unsigned)a.nmodels, (unsigned)a.curve_blocks);
+    if (a.curve_share) k_curve<kEpiThreads / 32><<<grid, kEpiThreads, 0, s>>>(a);
+    else k_curve<1><<<grid, kEpiThreads, 0, s>>>(a);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    k_results<<<dim3((unsigned)a.nmodels, (unsigned)(a.scale ? a.result_blocks : 1)), kEpiThreads, 0, s>>>(a);
     return cudaGetLastError();
 }
 

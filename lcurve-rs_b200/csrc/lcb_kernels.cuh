@@ -75,14 +75,18 @@ struct EpiArgs {
     const double* sp_w;
     const double* d_slfac;
     const double* partial;
-    const double* aux;
+    double* aux;         // sums (k_aux) and the count of finished k_results blocks (AUX_DONE)
     const int* status;
     int scale, rdata;
     double* calc;        // per datum
     double* results;     // 12 per model
     double* fcomp;       // iscale: 5 component fluxes per datum
     double* svda;        // iscale: 5 per datum, the weighted design matrix of the scale fit
+    double* episum;      // k_curve: 4 sums per (model, block)
+    double* chipart;     // k_results: one chi-squared part per (model, block)
     int64_t nmodels;
+    int curve_blocks, result_blocks;  // blocks per model of the two kernels
+    int curve_share;                  // k_curve: a block's warps share one tile's slots
     Sizes sz;
     int* bad;            // LCURVE_DEBUG_BOUNDS: per-model status words the epilogue may set
 };

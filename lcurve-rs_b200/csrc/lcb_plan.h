@@ -41,6 +41,8 @@ struct Plan {
     int roche_split = 1;      // threads per Roche-eclipsed element in the phase scan
     int flux_chunks = 1;      // elements per flux work unit / kFluxChunk
     int flux_blocks_per_sm = 0;  // persistent flux blocks per SM; 0 = the occupancy limit
+    int curve_blocks = 1, result_blocks = 1;  // blocks per model of k_curve and (scaled) k_results
+    int curve_share = 0;  // k_curve: 1 = a block's eight warps share one tile of data, 0 = a tile each
 
     // Empties the plan but keeps every buffer's capacity, so re-planning a
     // batch of the same size touches no fresh memory.
@@ -54,6 +56,8 @@ struct Plan {
         roche_split = 1;
         flux_chunks = 1;
         flux_blocks_per_sm = 0;
+        curve_blocks = result_blocks = 1;
+        curve_share = 0;
     }
 };
 
