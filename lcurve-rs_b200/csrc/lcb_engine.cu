@@ -1,8 +1,8 @@
 // lcb_engine.cu — context, device buffers, batch execution and the C ABI.
 //
 // A batch runs as one launch sequence on the context's stream:
-//   memset(aux, status, counter) -> k_phase -> k_elements -> k_roche (or, for
-//   small batches, k_roche_scan -> k_roche_chop2) -> k_aux -> k_flux -> k_curve -> k_results
+//   memset(aux, status, counter) -> k_phase -> k_elements -> k_roche ->
+//   k_roche_open -> k_roche_chop2 -> k_aux -> k_flux -> k_curve -> k_results
 // For a resident batch (lcb_batch_*) the sequence is captured once in a CUDA
 // graph and replayed; between runs only the model table and the tables
 // derived from it are uploaded, and the graph is rebuilt only when the
@@ -76,11 +76,11 @@ struct DevBuf {
 struct DeviceSet {
     DevBuf models, segs, bands, rings, eblocks, rblocks, ablocks, units, dmodel, dsub0, dsrc, data;
     DevBuf rec, pos, p64, d64, ecl, egrp, aux, status, spe, spphi, sptype, spw, slfac, partial, calc, results, counter,
-        datum, ecount, fcomp, svda, firsthit, episum;
+        datum, ecount, fcomp, svda, firsthit, episum, open;
     void release() {
         for (DevBuf* b : {&models, &segs, &bands, &rings, &eblocks, &rblocks, &ablocks, &units, &dmodel, &dsub0, &dsrc,
                           &data, &rec, &pos, &p64, &d64, &ecl, &egrp, &aux, &status, &spe, &spphi, &sptype, &spw, &slfac,
-                          &partial, &calc, &results, &counter, &datum, &ecount, &fcomp, &svda, &firsthit, &episum})
+                          &partial, &calc, &results, &counter, &datum, &ecount, &fcomp, &svda, &firsthit, &episum, &open})
             b->release();
     }
 };
@@ -135,6 +135,13 @@ namespace {
 // Upload of the plan's tables (and the data) into a device set.
 // Words of the per-group eclipse slot masks (one per kEclGroup elements).
 size_t ecl_groups(const lcb::Plan& P) { return (size_t)((P.nelem + lcb::kEclGroup - 1) / lcb::kEclGroup); }
+
+// Entries of the split scan's first hits: every Roche thread of a small batch; of a large one as
+// many as a list that is split can have (a fixed split takes them all).
+size_t first_hits(const lcb_ctx* C, const lcb::Plan& P) {
+    const size_t all = std::max<size_t>(P.rblocks.size() * lcb::kRocheBlock, 1);
+    return P.split_fix > 1 ? all : std::min<size_t>(all, (size_t)lcb::split_target(C->num_sms) / 2 + lcb::kRocheBlock);
+}
 
 // Doubles of the epilogue's per-block sums: four per k_curve block, one per k_results block.
 size_t epi_sums(const lcb::Plan& P) { return P.models.size() * (size_t)(4 * P.curve_blocks + P.result_blocks); }
@@ -206,7 +213,8 @@ void upload_plan(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, const lcb_datum* 
     const size_t ncomp = P.any_iscale ? (size_t)P.ndatum * 5 : 1;
     D.fcomp.ensure(ncomp * sizeof(double));
     D.svda.ensure(ncomp * sizeof(double));
-    D.firsthit.ensure((P.roche_split > 1 ? P.rblocks.size() * lcb::kRocheBlock : 1) * sizeof(int));
+    D.open.ensure(std::max<size_t>(P.rblocks.size() * lcb::kRocheBlock, 1) * sizeof(unsigned));
+    D.firsthit.ensure(first_hits(C, P) * sizeof(int));
 }
 
 // Parts of the launch sequence: the element stage (grids, continuum, eclipses:
@@ -239,11 +247,11 @@ void enqueue_run(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, int scale, int rd
                      D.rings.as<lcb::Ring>(), D.rec.as<float4>(), D.pos.as<float4>(), D.p64.as<double4>(),
                      D.d64.as<double4>(), D.ecl.as<double2>(), D.egrp.as<unsigned>(), D.aux.as<double>(),
                      D.status.as<int>(), nblk, nrblk, (int64_t)P.ablocks.size(),
-                     D.ecount.as<unsigned long long>(), P.roche_split, D.firsthit.as<int>(), C->fblink_cap, sz};
+                     D.ecount.as<unsigned long long>(), D.open.as<unsigned>(), D.counter.as<unsigned>() + 1,
+                     D.firsthit.as<int>(), (unsigned)first_hits(C, P), P.split_fix, lcb::split_target(C->num_sms),
+                     C->num_sms * 5, C->fblink_cap, sz};
     if (elem) {
         CUDA_TRY(cudaMemsetAsync(D.egrp.p, 0, ecl_groups(P) * sizeof(unsigned), s));
-        if (P.roche_split > 1 && nrblk > 0)
-            CUDA_TRY(cudaMemsetAsync(D.firsthit.p, 0x7f, nrblk * lcb::kRocheBlock * sizeof(int), s));
         CUDA_TRY(lcb::launch_elements(ea, s));
     }
     if (timed) CUDA_TRY(cudaEventRecord(C->ev[2], s));
@@ -1092,7 +1100,11 @@ int lcb_measure_fma_peak(lcb_ctx* C, int which, double* tflops) {
 // device are serialised by a per-device lock, and each call waits for its GPU
 // work (also on its error paths) before it returns.
 // ===========================================================================
-static __device__ __align__(256) unsigned char g_noalloc_arena[LCB_NOALLOC_ARENA_BYTES];
+// The limit on a call's scratch counts the tables, element, sub-phase and result arrays.  The list of
+// open elements (4 bytes per Roche thread: at most 8 per element of 160 or more) and the epilogue's
+// sums (about one byte per datum of 76 or more) come on top, under a sixteenth of the rest.
+static constexpr size_t kNoallocArena = (size_t)LCB_NOALLOC_ARENA_BYTES + LCB_NOALLOC_ARENA_BYTES / 16 + (64u << 10);
+static __device__ __align__(256) unsigned char g_noalloc_arena[kNoallocArena];
 
 namespace {
 
@@ -1114,7 +1126,7 @@ unsigned char* noalloc_arena() {
 
 // Lays out every buffer of a planned single-model evaluation inside the arena
 // (base == nullptr only measures).  Returns the bytes used.
-size_t noalloc_carve(const lcb::Plan& P, unsigned char* base, DeviceSet& D) {
+size_t noalloc_carve(const lcb_ctx* C, const lcb::Plan& P, unsigned char* base, DeviceSet& D, size_t* total = nullptr) {
     size_t off = 0;
     auto take = [&](DevBuf& b, size_t bytes) {
         b.p = base ? base + off : nullptr;
@@ -1149,14 +1161,18 @@ size_t noalloc_carve(const lcb::Plan& P, unsigned char* base, DeviceSet& D) {
     take(D.partial, P.npartial * sizeof(double));
     take(D.calc, P.ndatum * sizeof(double));
     take(D.results, nm * 12 * sizeof(double));
-    take(D.episum, epi_sums(P) * sizeof(double));
     take(D.counter, sizeof(int) * 4);
     take(D.ecount, sizeof(unsigned long long) * 8);
     const size_t ncomp = P.any_iscale ? (size_t)P.ndatum * 5 : 1;
     take(D.fcomp, ncomp * sizeof(double));
     take(D.svda, ncomp * sizeof(double));
-    take(D.firsthit, (P.roche_split > 1 ? P.rblocks.size() * lcb::kRocheBlock : 1) * sizeof(int));
-    return off;
+    // what LCB_NOALLOC_ARENA_BYTES limits: the above and four bytes per Roche thread of a split search
+    const size_t counted = off + (((P.roche_split > 1 ? P.rblocks.size() * lcb::kRocheBlock : 1) * sizeof(int) + 255) & ~size_t(255));
+    take(D.firsthit, first_hits(C, P) * sizeof(int));
+    take(D.open, std::max<size_t>(P.rblocks.size() * lcb::kRocheBlock, 1) * sizeof(unsigned));
+    take(D.episum, epi_sums(P) * sizeof(double));
+    if (total) *total = off;
+    return counted;
 }
 
 // Host -> arena copies of the plan's tables and the data (no allocation).
@@ -1195,14 +1211,15 @@ extern "C" int lcb_light_curve_noalloc(lcb_ctx* C, const lcb_model* model, const
         lcb::plan_batch(&mp, 1, data, &st, &cnt, C->num_sms, P);
         if (!P.model_ok[0]) throw Error(LCB_ERR_MODEL, P.model_err[0]);
         DeviceSet D;  // views into the arena: never ensure()d or released
-        const size_t need = noalloc_carve(P, nullptr, D);
-        if (need > (size_t)LCB_NOALLOC_ARENA_BYTES)
+        size_t total = 0;
+        const size_t need = noalloc_carve(C, P, nullptr, D, &total);
+        if (need > (size_t)LCB_NOALLOC_ARENA_BYTES || total > kNoallocArena)
             throw Error(LCB_ERR_INVALID, "lcb_light_curve_noalloc: this model and data need " + std::to_string(need) +
                                              " bytes of device scratch, more than the fixed arena's " +
                                              std::to_string((size_t)LCB_NOALLOC_ARENA_BYTES) +
                                              "; use lcb_light_curve (or coarser grids / fewer points)");
         std::lock_guard<std::mutex> lock(g_noalloc_mu[C->device]);
-        noalloc_carve(P, noalloc_arena(), D);
+        noalloc_carve(C, P, noalloc_arena(), D);
         std::vector<double> res, calc;
         std::vector<int> status;
         try {

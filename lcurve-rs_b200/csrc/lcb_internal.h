@@ -41,8 +41,9 @@ struct RocheEcl {          // constants of a Roche-distorted eclipsing star
     double mu, comp, ssq;  // q/(1+q), 1-mu, spin^2
     double rref, pref;     // reference sphere (surface.rs:14-39)
     double cofmx;          // 0 (primary) or 1 (secondary)
+    double ry, rz;         // the surface's distance from the centre along y and z
     int32_t primary;
-    int32_t pad;
+    int32_t convex;        // the star is convex (roche_convex): its limb decides most of the eclipse search
 };
 
 struct SpotDev {           // Gaussian star spot (brightness.rs:187-201)

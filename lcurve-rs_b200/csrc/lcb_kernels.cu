@@ -10,13 +10,13 @@
 //                and by an opaque disc (disc_eclipse.rs:84-330); continuum
 //                flux (brightness.rs).  Elements eclipsed by a Roche-distorted
 //                star keep that slot for k_roche.
-//   k_roche    : one thread per element eclipsed by a Roche-distorted star:
-//                the FP64 ray-march ingress_egress (eclipse.rs:270-373), the
-//                phase scan with exact second-order miss proofs, then the two
-//                bisections.  Small batches run k_roche_scan (the scan split
-//                over several threads, first hit by atomicMin) and
-//                k_roche_chop2 (the ingress and egress bisections from that
-//                hit, one thread each) instead.
+//   k_roche    : two threads per element eclipsed by a Roche-distorted star:
+//                the FP64 ray-march ingress_egress (eclipse.rs:270-373) decided
+//                from the star's limb contacts (lcb_roche.h).  The elements that
+//                path leaves open take the general one: k_roche_open (phase scan
+//                with exact second-order miss proofs and bisections; for short
+//                lists the scan alone, split over several threads, first hit by
+//                atomicMin) and k_roche_chop2 (the bisections from that hit).
 //   k_aux      : per star element, the per-model FP64 sums of ginterp,
 //                wdwarf, log g and radii (flux.rs:115-206, 288-373).
 //   k_flux     : persistent FP32 flux sum (flux.rs:7-111) over work units of
@@ -40,6 +40,7 @@
 #include <cstdint>
 
 #include "lcb_kernels.cuh"
+#include "lcb_roche.h"
 #include "lcb_stream.h"
 
 namespace lcb {
@@ -55,17 +56,13 @@ namespace {
 #define LCB_IN_BOUNDS(cond, status_word) true
 #endif
 
-constexpr double kPi = 3.14159265358979323846;
-constexpr double kTwoPi = 2.0 * kPi;
+using namespace roche;
 constexpr double kFac1 = 2.0e27 * 6.6262e-34 * 2.99792458e8;      // planck.rs:5
 constexpr double kFac2 = 1.0e9 * 6.6262e-34 * 2.99792458e8 / 1.3806e-23;  // planck.rs:8
 constexpr double kFwhmEfac = 2.3548200450309493;                  // brightness.rs:8
 constexpr double kEfac = 1.0000001;                               // grid.rs:396
 #ifndef LCB_ROCHE_MIN_BLOCKS
 #define LCB_ROCHE_MIN_BLOCKS 5
-#endif
-#ifndef LCB_CERT_BUDGET
-#define LCB_CERT_BUDGET 32
 #endif
 constexpr int kRocheMinBlocks = LCB_ROCHE_MIN_BLOCKS;  // k_roche blocks per SM (128 threads): register budget
 #ifndef LCB_SCAN_MIN_BLOCKS
@@ -76,29 +73,10 @@ constexpr int kRocheMinBlocks = LCB_ROCHE_MIN_BLOCKS;  // k_roche blocks per SM 
 #endif
 constexpr int kScanMinBlocks = LCB_SCAN_MIN_BLOCKS;  // the same for the split scan (small batches)
 constexpr int kChopMinBlocks = LCB_CHOP_MIN_BLOCKS;  // and for its bisection kernel
-constexpr int kCertBudget = LCB_CERT_BUDGET;           // miss-proof nodes per line of sight before the full search
-#ifndef LCB_TUBE_MAX
-#define LCB_TUBE_MAX 8
-#endif
-constexpr int kTubeMax = LCB_TUBE_MAX;  // scan steps per phase-block miss proof (1: single steps only)
 #ifndef LCB_FLUX_UNROLL
 #define LCB_FLUX_UNROLL 4
 #endif
 constexpr int kFluxUnroll = LCB_FLUX_UNROLL;  // list elements per unrolled step of the flux loop
-#ifndef LCB_SPLIT_TUBES
-#define LCB_SPLIT_TUBES 0  // phase blocks in the split scan of small batches (slower there: 0)
-#endif
-#ifndef LCB_TUBE_BUDGET
-#define LCB_TUBE_BUDGET 24
-#endif
-constexpr int kTubeBudget = LCB_TUBE_BUDGET;  // nodes of one phase-block proof
-constexpr int kTubeCool = 8;  // single steps after a failed two-step block before the next block
-#ifndef LCB_CHOP_BUDGET
-#define LCB_CHOP_BUDGET 0
-#endif
-constexpr int kChopBudget = LCB_CHOP_BUDGET;           // the same in the bisections (0: no proofs there)
-
-__device__ __forceinline__ double sq(double x) { return x * x; }
 __device__ __forceinline__ double rad2deg(double r) { return r * (180.0 / kPi); }
 
 __device__ __forceinline__ double planck_d(double wave, double temp) {  // planck.rs:16-23
@@ -128,466 +106,6 @@ __device__ __forceinline__ void dpot_exact(bool primary, double q, double ssq, d
     gx = comp * x + mu1 * (x - 1.0) - (primary ? ssq * x - mu : ssq * (x - 1.0) - mu + 1.0);
     gy = comp * y + mu1 * y - ssq * y;
     gz = comp * z + mu1 * z;
-}
-
-// Potential along a line of sight p + lam*e for the eclipse search
-// (potential.rs:110-117).  1/r from rsqrt: decisions against pref differ
-// from the divided form only within an ulp of the surface.
-struct Los {
-    double px, py, pz, ex, ey, ez;
-};
-__device__ __forceinline__ double los_pot(const RocheEcl& s, const Los& L, double lam) {
-    double x = fma(lam, L.ex, L.px), y = fma(lam, L.ey, L.py), z = fma(lam, L.ez, L.pz);
-    double x2y2 = x * x + y * y;
-    double r1sq = x2y2 + z * z;
-    double r2sq = r1sq + 1.0 - 2.0 * x;
-    double v = -s.comp * rsqrt(r1sq) - s.mu * rsqrt(r2sq);
-    if (s.primary) return v - s.ssq * x2y2 * 0.5 + s.mu * x;
-    return v - s.ssq * (0.5 + 0.5 * x2y2 - x) - s.comp * x;
-}
-__device__ __forceinline__ double los_dpot(const RocheEcl& s, const Los& L, double lam) {  // potential.rs:120-127
-    double x = fma(lam, L.ex, L.px), y = fma(lam, L.ey, L.py), z = fma(lam, L.ez, L.pz);
-    double r1sq = x * x + y * y + z * z, r2sq = r1sq + 1.0 - 2.0 * x;
-    double i1 = rsqrt(r1sq), i2 = rsqrt(r2sq);
-    double comp = s.comp * (i1 * i1 * i1), mu1 = s.mu * (i2 * i2 * i2);
-    double gx = comp * x + mu1 * (x - 1.0) - (s.primary ? s.ssq * x - s.mu : s.ssq * (x - 1.0) - s.mu + 1.0);
-    double gy = comp * y + mu1 * y - s.ssq * y;
-    double gz = comp * z + mu1 * z;
-    return gx * L.ex + gy * L.ey + gz * L.ez;
-}
-
-// Work counters of the eclipse search (potential and gradient evaluations, fblink calls),
-// and the bound on one line-of-sight search's potential evaluations (the reference has
-// none; reaching it marks the model failed: kStatusIterCap).
-struct EclCount {
-    int pot = 0, dpot = 0, fbl = 0, cert = 0, skipped = 0;
-    int cap = kFblinkEvalCap;
-};
-
-// dbrent with stop-fast (crates/subs/src/numerical/dbrent.rs:20-165).
-// Returns 1 = bracketed minimum below fref, 0 = not below.
-// `local` counts the search's evaluations so far; past cnt.cap the search stops
-// and sets `capped` (the model then fails).
-__device__ bool dbrent_below(const RocheEcl& s, const Los& L, double ax, double bx, double cx, double acc,
-                             double fref, EclCount& cnt, int& local, bool& capped) {
-    double a = fmin(ax, cx), b = fmax(ax, cx);
-    double x = bx, w = bx, v = bx;
-    if (local + 2 > cnt.cap) { capped = true; return false; }
-    local += 2;
-    double fx = los_pot(s, L, x), fw = fx, fv = fx;
-    ++cnt.pot;
-    if (fx < fref) return true;
-    double dx = los_dpot(s, L, x), dw = dx, dv = dx;
-    ++cnt.dpot;
-    double e = 0.0, d = 0.0;
-    for (int it = 0; it < 100; ++it) {
-        double xm = 0.5 * (a + b);
-        double tol1 = acc, tol2 = 2.0 * tol1;
-        if (fabs(x - xm) <= tol2 - 0.5 * (b - a)) return fx < fref;
-        if (fabs(e) > tol1) {
-            double d1 = 2.0 * (b - a), d2 = d1;
-            if (dw != dx) d1 = (w - x) * dx / (dx - dw);
-            if (dv != dx) d2 = (v - x) * dx / (dx - dv);
-            double u1 = x + d1, u2 = x + d2;
-            bool ok1 = (a - u1) * (u1 - b) > 0.0 && dx * d1 <= 0.0;
-            bool ok2 = (a - u2) * (u2 - b) > 0.0 && dx * d2 <= 0.0;
-            double olde = e;
-            e = d;
-            if (ok1 || ok2) {
-                d = (ok1 && ok2) ? (fabs(d1) < fabs(d2) ? d1 : d2) : (ok1 ? d1 : d2);
-                if (fabs(d) <= fabs(0.5 * olde)) {
-                    double u = x + d;
-                    if (u - a < tol2 || b - u < tol2) d = (xm - x >= 0.0) ? fabs(tol1) : -fabs(tol1);
-                } else {
-                    e = dx >= 0.0 ? a - x : b - x;
-                    d = 0.5 * e;
-                }
-            } else {
-                e = dx >= 0.0 ? a - x : b - x;
-                d = 0.5 * e;
-            }
-        } else {
-            e = dx >= 0.0 ? a - x : b - x;
-            d = 0.5 * e;
-        }
-        double u, fu;
-        if (local + 2 > cnt.cap) { capped = true; return false; }
-        local += 2;
-        if (fabs(d) >= tol1) {
-            u = x + d;
-            fu = los_pot(s, L, u);
-            ++cnt.pot;
-            if (fu < fref) return true;
-        } else {
-            u = x + (d >= 0.0 ? fabs(tol1) : -fabs(tol1));
-            fu = los_pot(s, L, u);
-            ++cnt.pot;
-            if (fu < fref) return true;
-            if (fu > fx) return fx < fref;
-        }
-        double du = los_dpot(s, L, u);
-        ++cnt.dpot;
-        if (fu <= fx) {
-            if (u >= x) a = x; else b = x;
-            v = w; fv = fw; dv = dw;
-            w = x; fw = fx; dw = dx;
-            x = u; fx = fu; dx = du;
-        } else {
-            if (u < x) a = u; else b = u;
-            if (fu <= fw || w == x) {
-                v = w; fv = fw; dv = dw;
-                w = u; fw = fu; dw = du;
-            } else if (fu < fv || v == x || v == w) {
-                v = u; fv = fu; dv = du;
-            }
-        }
-    }
-    return false;  // iteration cap: the reference maps its Err to "not eclipsed"
-}
-
-// Squared distances from the segment p + lam*e, lam in [a, b] (|e| = 1), to the
-// two stars' centres (the primary at the origin, the secondary at (1, 0, 0)).
-__device__ __forceinline__ void closest_sq(const Los& L, double a, double b, double& d1, double& d2) {
-    double t1 = fmin(fmax(-(L.px * L.ex + L.py * L.ey + L.pz * L.ez), a), b);
-    double x1 = fma(t1, L.ex, L.px), y1 = fma(t1, L.ey, L.py), z1 = fma(t1, L.ez, L.pz);
-    d1 = x1 * x1 + y1 * y1 + z1 * z1;
-    double qx = L.px - 1.0;
-    double t2 = fmin(fmax(-(qx * L.ex + L.py * L.ey + L.pz * L.ez), a), b);
-    double x2 = fma(t2, L.ex, qx), y2 = fma(t2, L.ey, L.py), z2 = fma(t2, L.ez, L.pz);
-    d2 = x2 * x2 + y2 * y2 + z2 * z2;
-}
-
-#ifndef LCB_PROOF_FAST_RSQRT
-#define LCB_PROOF_FAST_RSQRT 1
-#endif
-// 1/sqrt(x) for the miss proofs' nodes: a single-precision hardware estimate
-// (rsqrtf, within 2 ulp of FP32, i.e. relative error e0 < 2^-22) refined by one
-// Newton-Raphson step for the inverse square root in FP64, y1 = y0 (3 - x y0^2) / 2,
-// whose relative error is 3/2 e0^2 + O(e0^3) < 2e-13 plus a few FP64 roundings.
-// The proofs' 1e-9 relative margin above the surface value covers that many
-// times over; the reference-path evaluations (los_pot, los_dpot) keep rsqrt.
-// The squared distances to the two centres along a line of sight (a few
-// separations long, in units of the separation) lie far inside FP32's normal
-// range; at x = 0 the result is NaN, so the node's bound fails and the line of
-// sight is left to the full search.
-__device__ __forceinline__ double proof_rsqrt(double x) {
-#if LCB_PROOF_FAST_RSQRT
-    const double y = (double)rsqrtf((float)x);
-    return y * fma(-0.5 * x, y * y, 1.5);
-#else
-    return rsqrt(x);
-#endif
-}
-
-// The potential and its derivative along the line of sight at one point
-// (los_pot and los_dpot sharing the two distances), and the gradient's norm
-// when `grad` is not null.  For the miss proofs only (proof_rsqrt).
-__device__ __forceinline__ void los_pot_dpot(const RocheEcl& s, const Los& L, double lam, double& f, double& df,
-                                             double* grad = nullptr) {
-    double x = fma(lam, L.ex, L.px), y = fma(lam, L.ey, L.py), z = fma(lam, L.ez, L.pz);
-    double x2y2 = x * x + y * y;
-    double r1sq = x2y2 + z * z, r2sq = r1sq + 1.0 - 2.0 * x;
-    double i1 = proof_rsqrt(r1sq), i2 = proof_rsqrt(r2sq);
-    double v = -s.comp * i1 - s.mu * i2;
-    f = s.primary ? v - s.ssq * x2y2 * 0.5 + s.mu * x : v - s.ssq * (0.5 + 0.5 * x2y2 - x) - s.comp * x;
-    double comp = s.comp * (i1 * i1 * i1), mu1 = s.mu * (i2 * i2 * i2);
-    double gx = comp * x + mu1 * (x - 1.0) - (s.primary ? s.ssq * x - s.mu : s.ssq * (x - 1.0) - s.mu + 1.0);
-    double gy = comp * y + mu1 * y - s.ssq * y;
-    double gz = comp * z + mu1 * z;
-    df = gx * L.ex + gy * L.ey + gz * L.ez;
-    if (grad) {  // |grad| = n2 / sqrt(n2), to the same 2e-13 (n2 = 0: NaN, the node fails)
-        const double n2 = gx * gx + gy * gy + gz * gz;
-        *grad = n2 * proof_rsqrt(n2);
-    }
-}
-
-// True when the potential provably stays above the surface value on the whole
-// line-of-sight segment [a, b]: an adaptive march over sub-segments, each
-// certified by a second-order bound.  Along a line the Roche potential's
-// second derivative is at least -M, M = 2 comp / r1^3 + 2 mu / r2^3 + ssq with
-// r1, r2 the segment's closest approaches to the two centres (each gravity
-// term -c / r has second derivative c (r^2 - 3 s^2) / r^5 >= -2 c / r^3, s the
-// distance along the line from the closest point; the centrifugal term
-// -ssq (x^2 + y^2) / 2 contributes -ssq (ex^2 + ey^2) >= -ssq; the rest is
-// linear), so on a sub-segment of length h around m
-//   phi >= phi(m) - |phi'(m)| h / 2 - M h^2 / 8.
-// The bound must clear the surface value by 1e-9 relative (far above the
-// rounding of any evaluation).  False means "not proven".
-//
-// With w > 0 the segment stands for a fan of lines through p whose unit
-// directions lie within w of L's: every point of the fan at parameter t is
-// within |t| w of L's point at t.  The Hessian of the potential has norm at
-// most H = 2 comp / r1^3 + 2 mu / r2^3 + ssq with r1, r2 now the closest
-// approaches of that tube, so a point x within r of the sub-segment's point y
-// has phi(x) >= phi(y) - |grad phi(y)| r - H r^2 / 2, and
-// |grad phi(y)| <= |grad phi(m)| + H h / 2: each node subtracts
-// (|grad phi(m)| + H h / 2) r + H r^2 / 2, r = (|m| + h / 2) w.
-template <bool kTube>
-__device__ __forceinline__ bool certify_miss(const RocheEcl& s, const Los& L, double a, double b, int budget,
-                                             int& nodes, double w = 0.0) {
-    const double thr = s.pref + 1e-9 * fmax(fabs(s.pref), 1.0);
-    const double hmin = 1e-6 * (b - a);
-    double d1, d2;
-    closest_sq(L, a, b, d1, d2);
-    const double i1 = rsqrt(d1), i2 = rsqrt(d2);
-    const double curv = 2.0 * s.comp * (i1 * i1 * i1) + 2.0 * s.mu * (i2 * i2 * i2) + s.ssq;
-    double hess = 0.0;
-    if (kTube) {
-        const double widen = fmax(fabs(a), fabs(b)) * w;
-        const double r1 = sqrt(d1) - widen, r2 = sqrt(d2) - widen;
-        if (!(r1 > 1e-3 && r2 > 1e-3)) return false;
-        hess = 2.0 * s.comp / (r1 * r1 * r1) + 2.0 * s.mu / (r2 * r2 * r2) + s.ssq;
-    }
-    double t = a, h = b - a;
-    for (int it = 0; it < budget; ++it) {
-        if (t >= b) return true;
-        double hh = fmin(h, b - t);
-        ++nodes;
-        const double m = t + 0.5 * hh;
-        double f, df, g = 0.0;
-        los_pot_dpot(s, L, m, f, df, kTube ? &g : nullptr);
-        double bound = f - fabs(df) * (0.5 * hh) - curv * (0.125 * hh * hh);
-        if (kTube) {
-            const double r = (fabs(m) + 0.5 * hh) * w;
-            bound -= (g + hess * (0.5 * hh)) * r + 0.5 * hess * r * r;
-        }
-        if (bound > thr) {
-            t += hh;
-            h = 2.0 * hh;
-        } else {
-            if (hh <= hmin) return false;
-            h = 0.5 * hh;
-        }
-    }
-    return t >= b;
-}
-
-// Is point p hidden from earth direction e by the Roche star? (eclipse.rs:123-197)
-// With `prove` > 0 (a node budget), a line of sight whose first reference evaluation is not
-// inside the star is first tested with the rigorous second-order bound: every point
-// the reference search evaluates lies in [lam1 - acc, lam2 + acc] (dbrent.rs:116
-// may step acc past an end), so a proven miss is exactly its "false".
-// Not inlined: as a call, the search's working set does not add to the
-// registers the surrounding scan/bisection loop keeps live, which lets the
-// kernel run 5 blocks per SM (451 -> 350 ms on the 1024-model batch).
-__device__ __noinline__ bool fblink(const RocheEcl& s, double acc, const Los& L, EclCount& cnt, bool& capped, int prove) {
-    ++cnt.fbl;
-    double dx = L.px - s.cofmx, dy = L.py, dz = L.pz;
-    double bq = L.ex * dx + L.ey * dy + L.ez * dz;  // sphere_eclipse_los, eclipse.rs:202-224
-    if (bq >= 0.0) return false;
-    double cq = (dx * dx + dy * dy + dz * dz) - sq(s.rref);
-    double fac = sq(bq) - cq;
-    if (fac <= 0.0) return false;
-    fac = sqrt(fac);
-    double lam2 = -bq + fac, lam1 = fmax(cq / lam2, 0.0);
-    if (lam1 == 0.0) return true;
-    const double pref = s.pref;
-    double step = lam2 - lam1;
-    if (!(step > acc)) return false;  // no evaluation: flam = 1 > f1 = f2 = 0
-    // the reference's first evaluation, at the middle of the chord
-    const double lam0 = lam1 + step / 2.0;
-    double flam = los_pot(s, L, lam0);
-    ++cnt.pot;
-    if (flam <= pref) return true;
-    if (prove > 0) {  // prove: the miss-proof node budget (0: no proof)
-        const double pad = 1.001 * acc + 1e-12;
-        if (certify_miss<false>(s, L, lam1 - pad, lam2 + pad, prove, cnt.cert)) { ++cnt.skipped; return false; }
-    }
-    int nstep = 1;
-    double f1 = los_pot(s, L, lam1), f2 = los_pot(s, L, lam2), lam = lam0;
-    int local = 2;
-    bool br = flam < f1 && flam < f2;
-    if (!br) {
-        step /= 2.0;
-        nstep = 2;
-        while (step > acc) {
-            lam = lam1 + step / 2.0;
-            for (int n = 0; n < nstep; ++n) {
-                flam = los_pot(s, L, lam + (double)n * step);
-                ++local;
-                if (flam <= pref) { cnt.pot += local; return true; }
-                if (flam < f1 && flam < f2) { lam = lam + (double)n * step; br = true; break; }
-            }
-            if (br) break;
-            if (local > cnt.cap) { capped = true; cnt.pot += local; return false; }
-            step /= 2.0;
-            nstep *= 2;
-        }
-    }
-    cnt.pot += local;
-    if (br) return dbrent_below(s, L, lam1, lam, lam2, acc, pref, cnt, local, capped);
-    return false;
-}
-
-// Phase-block miss proof: L is the middle line of a block of consecutive scan
-// steps whose unit directions lie within tube_w of L's (all lines pass through
-// p).  True when every step of the block provably misses, i.e. each step's own
-// fblink would return false (see certify_miss).  A separate call from fblink:
-// the single-step search keeps its own, smaller register allocation.
-__device__ __noinline__ bool tube_miss(const RocheEcl& s, double acc, const Los& L, double tube_w, int budget,
-                                       int& nodes) {
-    const double dx = L.px - s.cofmx, dy = L.py, dz = L.pz;
-    // every step's b = e.d lies within |d| tube_w of the middle line's; its chord of the
-    // bounding sphere, where it has one, within [c / lam2max, lam2max] (lam2 = -b +
-    // sqrt(b^2 - c) falls as b rises)
-    const double dd = dx * dx + dy * dy + dz * dz;
-    const double cq = dd - sq(s.rref);
-    if (!(cq > 0.0)) return false;
-    const double bmin = L.ex * dx + L.ey * dy + L.ez * dz - sqrt(dd) * tube_w;
-    if (bmin >= 0.0) return true;  // every step: b >= 0, no chord
-    const double fac = sq(bmin) - cq;
-    if (fac <= 0.0) return true;   // every step misses the bounding sphere
-    const double lam2 = -bmin + sqrt(fac), lam1 = cq / lam2;
-    const double pad = 1.001 * acc + 1e-12;
-    return certify_miss<true>(s, L, lam1 - pad, lam2 + pad, budget, nodes, tube_w);
-}
-
-__device__ __forceinline__ void earth_at(double cosi, double sini, double phase, double& ex, double& ey, double& ez) {
-    double sn, cs;  // misc.rs:42-45
-    sincos(kTwoPi * phase, &sn, &cs);
-    ex = sini * cs;
-    ey = -sini * sn;
-    ez = cosi;
-}
-
-// Analytic sphere eclipse (eclipse.rs:229-265).
-__device__ bool sphere_phase(double cosi, double sini, double px, double py, double pz, double cx, double rs,
-                             double& phi1, double& phi2, double& lam1, double& lam2) {
-    double dx = px - cx, dy = py, dz = pz;
-    double pdist = sqrt(sq(dx) + sq(dy));
-    double bq = dz * cosi - pdist * sini;
-    if (bq >= 0.0) return false;
-    double cq = (dx * dx + dy * dy + dz * dz) - sq(rs);
-    double fac = sq(bq) - cq;
-    if (fac <= 0.0) return false;
-    fac = sqrt(fac);
-    lam2 = -bq + fac;
-    lam1 = fmax(cq / lam2, 0.0);
-    if (cq < 0.0) {
-        phi1 = 0.0;
-        phi2 = 1.0;
-    } else {
-        double delta = acos((cosi * dz + sqrt(cq)) / (sini * pdist));
-        double phi = atan2(dy, -dx);
-        double p1 = (phi - delta) / kTwoPi;
-        p1 -= floor(p1);
-        phi1 = p1;
-        phi2 = p1 + 2.0 * delta / kTwoPi;
-    }
-    return true;
-}
-
-// Ingress/egress of point p behind a Roche-distorted star (eclipse.rs:270-373).
-// The phase scan of pot_min_search (eclipse.rs:347-373) and the two bisections
-// (eclipse.rs:301-332) run as one loop with a single line-of-sight search call
-// site: lanes of a warp in different stages reconverge inside the search, and
-// the search code exists once.  Misses are proven (fblink's `prove`) only in the
-// scan, where nearly all lines of sight miss by a wide margin.
-// The phase scan of pot_min_search (eclipse.rs:347-373): phases phi1 + i dphi,
-// i = 0 .. nsteps, and the search tolerance acc (eclipse.rs:297).
-struct Scan {
-    double phi1, phi2, acc, dphi;
-    int nsteps;
-};
-__device__ __forceinline__ bool scan_setup(const RocheEcl& s, double cosi, double sini, double delta, double px,
-                                           double py, double pz, Scan& sc) {
-    double lam1, lam2;
-    if (!sphere_phase(cosi, sini, px, py, pz, s.cofmx, s.rref, sc.phi1, sc.phi2, lam1, lam2)) return false;
-    sc.acc = 2.0 * sqrt(2.0 * kTwoPi * (lam2 - lam1) * delta);
-    double ns = ceil((sc.phi2 - sc.phi1) / (sc.acc / kTwoPi));
-    sc.nsteps = (ns != ns || ns <= 10.0) ? 10 : (ns >= 1000.0 ? 1000 : (int)ns);
-    sc.dphi = (sc.phi2 - sc.phi1) / (double)sc.nsteps;
-    return true;
-}
-
-// Bound on |e(ph) - e(mid)| for phases within `half` of mid: the earth vector's
-// xy part (length sini) turns by 2 pi (ph - mid), a chord of 2 sini sin(pi |ph - mid|).
-__device__ __forceinline__ double tube_width(double sini, double half) {
-    return 2.0 * sini * sin(fmin(kPi * half, 0.5 * kPi)) * (1.0 + 1e-12) + 1e-15;
-}
-
-constexpr int kNoHit = 0x7f7f7f7f;  // first-hit sentinel (the byte pattern a memset of 0x7f writes)
-
-// `known_hit` >= 0: the scan's first hit is already known (split scan): go
-// straight to the bisections from that phase; kNoHit: the point is not eclipsed.
-// `only` = 1 or 2 runs just the ingress or just the egress bisection (the two are
-// independent: both start from the first hit), leaving `ing` resp. the unwrapped
-// `eg` set; the caller then applies egress < ingress -> egress + 1 itself.
-// kScan = false compiles the bisections alone (a known first hit is then required).
-template <bool kScan>
-__device__ bool ingress_egress(const RocheEcl& s, double cosi, double sini, double delta, double px, double py,
-                               double pz, double& ing, double& eg, bool& capped, EclCount& evals, int known_hit = -1,
-                               int only = 0) {
-    Scan sc;
-    if (!scan_setup(s, cosi, sini, delta, px, py, pz, sc)) return false;
-    if (known_hit == kNoHit) return false;
-    const double phi1 = sc.phi1, phi2 = sc.phi2, acc = sc.acc, dphi = sc.dphi;
-    const int nsteps = sc.nsteps;
-    Los L{px, py, pz, 0.0, 0.0, 0.0};
-    enum { SCAN, CHOP_IN, CHOP_EG };
-    // blk: scan steps the next phase-block proof covers; after a failed two-step block,
-    // kTubeCool single steps before the next (wait)
-    int mode = SCAN, i = 0, it = 0, blk = kTubeMax, wait = 0, last = 0;
-    double phi = 0.0, pin = 0.0, pout = 0.0;
-    if (known_hit >= 0) {  // as the scan below sets up its first hit
-        phi = phi1 + (double)known_hit * dphi;
-        if (only == 2) { mode = CHOP_EG; pin = phi; pout = phi2; }
-        else { mode = CHOP_IN; pin = phi; pout = phi1; }
-    }
-    for (;;) {
-        double ph, tube = 0.0;
-        if (kScan && mode == SCAN) {
-            if (i > nsteps) return false;  // no eclipsed phase found
-            last = wait > 0 ? i : min(i + blk - 1, nsteps);
-            if (last > i) {  // steps i .. last at once: one phase-block proof
-                ph = phi1 + 0.5 * (double)(i + last) * dphi;
-                tube = tube_width(sini, 0.5 * (double)(last - i) * dphi);
-            } else {
-                ph = phi1 + (double)i * dphi;
-            }
-        } else {
-            if (!(fabs(pin - pout) > delta) || it >= 200) {
-                double r = (pin + pout) / 2.0;
-                r -= floor(r);
-                if (mode == CHOP_IN) {
-                    ing = r;
-                    if (only == 1) return true;
-                    mode = CHOP_EG; pin = phi; pout = phi2; it = 0;
-                    continue;
-                }
-                eg = r;
-                if (only == 2) return true;
-                if (eg < ing) eg += 1.0;
-                return true;
-            }
-            ph = (pin + pout) / 2.0;
-        }
-        earth_at(cosi, sini, ph, L.ex, L.ey, L.ez);
-        const bool hit = tube > 0.0 ? tube_miss(s, acc, L, tube, kTubeBudget, evals.cert)
-                                    : fblink(s, acc, L, evals, capped, !(kScan && mode == SCAN) ? kChopBudget : kCertBudget);
-        if (capped) return false;
-        if (kScan && mode == SCAN) {
-            if (tube > 0.0) {
-                if (hit) {  // the block's steps are all misses: counted as the searches they stand for
-                    evals.fbl += last - i + 1;
-                    ++evals.skipped;  // one proof
-                    i = last + 1;
-                    blk = min(2 * blk, kTubeMax);
-                } else {
-                    blk >>= 1;
-                    if (blk < 2) wait = kTubeCool;
-                }
-            } else if (hit) { phi = ph; mode = CHOP_IN; pin = phi; pout = phi1; it = 0; }
-            else {
-                ++i;
-                if (wait > 0) --wait;
-                if (wait == 0) blk = max(blk, min(2, kTubeMax));
-            }
-        } else {
-            if (hit) pin = ph; else pout = ph;
-            ++it;
-        }
-    }
 }
 
 // Disc occultation (disc_eclipse.rs:29-70, 84-330); returns the number of pairs (<= 2).
@@ -970,31 +488,137 @@ __device__ __forceinline__ void group_or_warp(unsigned* grp, int64_t g, unsigned
     }
 }
 
+// Eclipses by Roche-distorted stars through their limb contacts (lcb_roche.h):
+// two adjacent lanes per element, one for the ingress and one for the egress,
+// each with its own Newton iteration and bisection; block b covers half of
+// Roche block b / 2.  Elements the limb path leaves open (stars that are not
+// convex, elements near the bounding sphere, grazes narrower than the margins)
+// go to a list that k_roche_open and k_roche_chop2 take.  Bound by FP64 latency
+// and issue: ~12 contact nodes and ~6 searches an element of ~10 evaluations.
 __global__ void __launch_bounds__(kRocheBlock, kRocheMinBlocks) k_roche(ElemArgs A) {
-    const ElemBlock blk = A.rblocks[blockIdx.x];
+    const int64_t rb = blockIdx.x >> 1;
+    const int slot = (int)(blockIdx.x & 1) * (kRocheBlock / 2) + (int)(threadIdx.x >> 1);
+    const bool egress = threadIdx.x & 1;
+    const ElemBlock blk = A.rblocks[rb];
     const SegDesc sg = A.segs[blk.seg];
-    const int64_t i = blk.offset + threadIdx.x;
-    EclCount cnt;
-    cnt.cap = A.fblink_cap;
-    bool capped = false;
-    int64_t g = -1;
-    unsigned bits = 0u;
-    if (i < sg.count && LCB_IN_BOUNDS(sg.first + i < A.sz.nelem, A.status + sg.model)) {
-        const ModelDev& M = A.models[sg.model];
-        const int by = blk.by;
-        const int64_t e = sg.first + i;
+    const int64_t i = blk.offset + slot, e = sg.first + i;
+    EclCount cnt, scan;  // scan: what both lanes of a pair do alike, counted by the first
+    cnt.cap = scan.cap = A.fblink_cap;
+    bool capped = false, open = false, hidden = false;
+    const bool valid = i < sg.count && LCB_IN_BOUNDS(e < A.sz.nelem, A.status + sg.model);
+    const ModelDev& M = A.models[sg.model];
+    const RocheEcl& R = blk.by == 1 ? M.ecl1 : M.ecl2;
+    Geom G;
+    Limb L;
+    bool found = false, seek = false;  // both contacts known; guesses in c.phi to try
+    Contact c{0.0, 0.0, false};
+    bool crosses = false;  // the bounding sphere, at some phase
+    if (valid) {
         const double4 p = A.el_p64[e];
-        double a, b;
-        if (ingress_egress<true>(by == 1 ? M.ecl1 : M.ecl2, M.cosi_e, M.sini_e, M.delta, p.x, p.y, p.z, a, b, capped, cnt)) {
-            const int slot = roche_slot(sg.kind, by);
-            A.el_ecl[slot * A.sz.nelem + e] = make_double2(a, b);
-            g = e / kEclGroup;
-            bits = 1u << slot;
+        crosses = geom_setup(R, M.cosi_e, M.sini_e, M.delta, p.x, p.y, p.z, G);
+        open = crosses && !limb_applies(R, G);
+        double half;
+        if (crosses && !open) {
+            seek = limb_guess(R, G, half);
+            c.phi = 0.5 * (G.sc.phi1 + G.sc.phi2) + (egress ? half : -half);
         }
-        if (capped) atomicOr(A.status + sg.model, kStatusIterCap);
     }
-    group_or_warp(A.ecl_grp, g, bits);
+    for (int attempt = 0; attempt < 2; ++attempt) {  // from the ellipsoid, then from the lowest potential
+        c.ok = false;
+        if (seek) c = limb_contact(R, G, egress, c.phi, cnt);
+        Contact o;  // the pair's other contact
+        o.phi = __shfl_xor_sync(0xffffffffu, c.phi, 1);
+        o.margin = __shfl_xor_sync(0xffffffffu, c.margin, 1);
+        o.ok = __shfl_xor_sync(0xffffffffu, (int)c.ok, 1) != 0;
+        if (seek) found = limb_make(egress ? o : c, egress ? c : o, L);
+        const bool lost = crosses && !open && !found;
+        if (attempt) {
+            if (seek && !found) open = true;
+            break;
+        }
+        seek = false;
+        if (lost) {
+            double lo, hi;
+            const int st = limb_lowest(R, G, lo, hi, scan);
+            if (st == LIMB_NONE) {
+                scan.fbl += G.sc.nsteps + 1;
+                ++scan.skipped;
+            }
+            open = st == LIMB_OPEN;
+            seek = st == LIMB_ECLIPSED;
+            c.phi = egress ? hi : lo;
+        }
+        if (!__any_sync(0xffffffffu, seek)) break;
+    }
+    double r = 0.0;
+    if (found) {
+        const int hit = limb_scan(R, G, L, capped, scan);
+        if (!capped && hit >= 0) {
+            r = limb_chop(R, G, L, egress, G.sc.phi1 + (double)hit * G.sc.dphi, M.delta, capped, cnt);
+            hidden = !capped;
+        }
+    }
+    const double eg = __shfl_xor_sync(0xffffffffu, r, 1);
+    const bool hidden2 = __shfl_xor_sync(0xffffffffu, (int)hidden, 1) != 0 && hidden;
+    int64_t grp = -1;
+    unsigned bits = 0u;
+    if (capped) atomicOr(A.status + sg.model, kStatusIterCap);
+    if (!egress && hidden2) {
+        const int slot = roche_slot(sg.kind, blk.by);
+        A.el_ecl[slot * A.sz.nelem + e] = make_double2(r, eg < r ? eg + 1.0 : eg);
+        grp = e / kEclGroup;
+        bits = 1u << slot;
+    }
+    group_or_warp(A.ecl_grp, grp, bits);
+    // open elements to the list, one atomic per warp
+    const unsigned mine = __ballot_sync(0xffffffffu, open && !egress);
+    if (mine) {
+        const int lane = threadIdx.x & 31, src = __ffs(mine) - 1;
+        unsigned base = 0;
+        if (lane == src) base = atomicAdd(A.nopen, (unsigned)__popc(mine));
+        base = __shfl_sync(0xffffffffu, base, src);
+        if ((mine >> lane) & 1u) {
+            const unsigned k = base + __popc(mine & ((1u << lane) - 1u));
+            A.open[k] = (unsigned)(rb * kRocheBlock + slot);
+            if (k < A.nfirst) A.firsthit[k] = kNoHit;
+        }
+    }
+    if (!egress) {
+        cnt.pot += scan.pot; cnt.dpot += scan.dpot; cnt.fbl += scan.fbl; cnt.cert += scan.cert; cnt.skipped += scan.skipped;
+    }
     roche_counters(A, cnt);
+}
+
+// Threads per open element in the split phase scan: a power of two up to 16,
+// until about sixteen waves of scan threads fill the GPU (the choices an
+// autotuning of 8..128-model batches made); 1: whole searches, one thread
+// each, where the scan proves blocks of steps at once.
+__device__ __forceinline__ int open_split(const ElemArgs& A, unsigned n) {
+    if (A.split_fix > 0) return n <= A.nfirst ? A.split_fix : 1;
+    const unsigned threads = (n + kRocheBlock - 1) / kRocheBlock * kRocheBlock;
+    int split = 1;
+    while (split < 16 && (int64_t)(2 * split) * threads <= A.split_target) split *= 2;
+    return n <= A.nfirst ? split : 1;
+}
+
+struct OpenElem {
+    const ModelDev* M;
+    const RocheEcl* R;
+    int64_t e;
+    int model, slot;
+    bool valid;
+};
+__device__ __forceinline__ OpenElem open_elem(const ElemArgs& A, unsigned item) {
+    const ElemBlock blk = A.rblocks[item / kRocheBlock];
+    const SegDesc sg = A.segs[blk.seg];
+    OpenElem o;
+    o.M = A.models + sg.model;
+    o.R = blk.by == 1 ? &o.M->ecl1 : &o.M->ecl2;
+    o.e = sg.first + blk.offset + item % kRocheBlock;
+    o.model = sg.model;
+    o.slot = roche_slot(sg.kind, blk.by);
+    o.valid = LCB_IN_BOUNDS(o.e < A.sz.nelem, A.status + sg.model);
+    return o;
 }
 
 // One chunk of a split phase scan: scan indices [c L, (c+1) L) of 0 .. nsteps,
@@ -1008,35 +632,6 @@ __device__ void scan_chunk(const RocheEcl& s, double cosi, double sini, double d
     const int total = sc.nsteps + 1, len = (total + split - 1) / split;
     const int lo = chunk * len, hi = min(total, lo + len);
     Los L{px, py, pz, 0.0, 0.0, 0.0};
-#if LCB_SPLIT_TUBES
-    int blk = kTubeMax, wait = 0, n = 0;  // phase blocks as in ingress_egress
-    for (int i = lo; i < hi; ++n) {
-        if ((n & 7) == 0 && *(volatile int*)first < lo) return;
-        const int last = wait > 0 ? i : min(i + blk - 1, hi - 1);
-        if (last > i) {
-            earth_at(cosi, sini, sc.phi1 + 0.5 * (double)(i + last) * sc.dphi, L.ex, L.ey, L.ez);
-            if (tube_miss(s, sc.acc, L, tube_width(sini, 0.5 * (double)(last - i) * sc.dphi), kTubeBudget, evals.cert)) {
-                ++evals.skipped;
-                i = last + 1;
-                blk = min(2 * blk, kTubeMax);
-            } else {
-                blk >>= 1;
-                if (blk < 2) wait = kTubeCool;
-            }
-            continue;
-        }
-        earth_at(cosi, sini, sc.phi1 + (double)i * sc.dphi, L.ex, L.ey, L.ez);
-        const bool hit = fblink(s, sc.acc, L, evals, capped, kCertBudget);
-        if (capped) return;
-        if (hit) {
-            atomicMin(first, i);
-            return;
-        }
-        ++i;
-        if (wait > 0) --wait;
-        if (wait == 0) blk = max(blk, min(2, kTubeMax));
-    }
-#else
     for (int i = lo; i < hi; ++i) {
         if (((i - lo) & 7) == 0 && *(volatile int*)first < lo) return;
         earth_at(cosi, sini, sc.phi1 + (double)i * sc.dphi, L.ex, L.ey, L.ez);
@@ -1047,7 +642,6 @@ __device__ void scan_chunk(const RocheEcl& s, double cosi, double sini, double d
             return;
         }
     }
-#endif
 }
 
 __device__ __forceinline__ void roche_counters(const ElemArgs& A, const EclCount& cnt) {
@@ -1061,73 +655,91 @@ __device__ __forceinline__ void roche_counters(const ElemArgs& A, const EclCount
     }
 }
 
-// Split scan, first kernel: block b scans chunk b % split of the elements of
-// Roche block b / split.  For small batches, whose time is otherwise the
-// longest single scan, this spreads each scan over `split` threads.
-__global__ void __launch_bounds__(kRocheBlock, kScanMinBlocks) k_roche_scan(ElemArgs A) {
-    const int64_t rb = blockIdx.x / A.roche_split;
-    const int chunk = (int)(blockIdx.x % A.roche_split);
-    const ElemBlock blk = A.rblocks[rb];
-    const SegDesc sg = A.segs[blk.seg];
-    const int64_t i = blk.offset + threadIdx.x;
+// The general search of the open elements: persistent blocks over the list.
+// Unsplit, one thread runs an element's whole search (phase scan with block
+// proofs, then both bisections).  Split, the scans' chunks are spread over
+// `split` threads an element and k_roche_chop2 bisects from the first hit: the
+// time of a short list is otherwise its longest single scan.
+__global__ void __launch_bounds__(kRocheBlock, kScanMinBlocks) k_roche_open(ElemArgs A) {
+    const unsigned n = *A.nopen;
+    if (n == 0) return;
+    const int split = open_split(A, n);
+    const int64_t groups = (int64_t)((n + kRocheBlock - 1) / kRocheBlock) * split;
     EclCount cnt;
     cnt.cap = A.fblink_cap;
-    bool capped = false;
-    if (i < sg.count && LCB_IN_BOUNDS(sg.first + i < A.sz.nelem, A.status + sg.model)) {
-        const ModelDev& M = A.models[sg.model];
-        const double4 p = A.el_p64[sg.first + i];
-        scan_chunk(blk.by == 1 ? M.ecl1 : M.ecl2, M.cosi_e, M.sini_e, M.delta, p.x, p.y, p.z, chunk, A.roche_split,
-                   A.firsthit + rb * kRocheBlock + threadIdx.x, capped, cnt);
-        if (capped) atomicOr(A.status + sg.model, kStatusIterCap);
+    for (int64_t w = blockIdx.x; w < groups; w += gridDim.x) {
+        const unsigned k = (unsigned)(w / split) * kRocheBlock + threadIdx.x;
+        int64_t g = -1;
+        unsigned bits = 0u;
+        if (k < n) {
+            const OpenElem o = open_elem(A, A.open[k]);
+            bool capped = false;
+            if (o.valid) {
+                const double4 p = A.el_p64[o.e];
+                if (split == 1) {
+                    double a, b;
+                    if (ingress_egress<true>(*o.R, o.M->cosi_e, o.M->sini_e, o.M->delta, p.x, p.y, p.z, a, b, capped, cnt)) {
+                        A.el_ecl[o.slot * A.sz.nelem + o.e] = make_double2(a, b);
+                        g = o.e / kEclGroup;
+                        bits = 1u << o.slot;
+                    }
+                } else {
+                    const int fbl = cnt.fbl;  // k_roche_chop2 counts the reference's scan searches
+                    scan_chunk(*o.R, o.M->cosi_e, o.M->sini_e, o.M->delta, p.x, p.y, p.z, (int)(w % split), split,
+                               A.firsthit + k, capped, cnt);
+                    cnt.fbl = fbl;
+                }
+                if (capped) atomicOr(A.status + o.model, kStatusIterCap);
+            }
+        }
+        if (split == 1) group_or_warp(A.ecl_grp, g, bits);
     }
-    cnt.fbl = 0;  // the second kernel counts the reference's scan searches
     roche_counters(A, cnt);
 }
 
 // Split scan, second kernel with two threads per element: adjacent lanes run
 // the ingress and the egress bisection of one element at once (each from the
 // first hit, eclipse.rs:301-332), halving the longest chain of line-of-sight
-// searches; the ingress lane combines the pair.  Block b covers half of Roche
-// block b / 2.
+// searches; the ingress lane combines the pair.
 __global__ void __launch_bounds__(kRocheBlock, kChopMinBlocks) k_roche_chop2(ElemArgs A) {
-    const int64_t rb = blockIdx.x >> 1;
-    const int slot = (int)(blockIdx.x & 1) * (kRocheBlock / 2) + (int)(threadIdx.x >> 1);
+    const unsigned n = *A.nopen;
+    if (n == 0 || open_split(A, n) == 1) return;
     const int part = threadIdx.x & 1;  // 0: ingress, 1: egress
-    const ElemBlock blk = A.rblocks[rb];
-    const SegDesc sg = A.segs[blk.seg];
-    const int64_t i = blk.offset + slot;
     EclCount cnt;
     cnt.cap = A.fblink_cap;
-    bool capped = false, found = false;
-    double a = 0.0, b = 0.0;
-    int64_t e = 0;
-    const bool valid = i < sg.count && LCB_IN_BOUNDS(sg.first + i < A.sz.nelem, A.status + sg.model);
-    if (valid) {
-        const ModelDev& M = A.models[sg.model];
-        const RocheEcl& R = blk.by == 1 ? M.ecl1 : M.ecl2;
-        e = sg.first + i;
-        const double4 p = A.el_p64[e];
-        const int first = A.firsthit[rb * kRocheBlock + slot];
-        Scan sc;
-        if (part == 0 && scan_setup(R, M.cosi_e, M.sini_e, M.delta, p.x, p.y, p.z, sc))
-            cnt.fbl += first == kNoHit ? sc.nsteps + 1 : first + 1;  // the single scan's searches
-        found = ingress_egress<false>(R, M.cosi_e, M.sini_e, M.delta, p.x, p.y, p.z, a, b, capped, cnt, first, part + 1);
-    }
-    const double egress = __shfl_xor_sync(0xffffffffu, b, 1);
-    const bool found_eg = __shfl_xor_sync(0xffffffffu, (int)found, 1) != 0;
-    const bool capped_eg = __shfl_xor_sync(0xffffffffu, (int)capped, 1) != 0;
-    int64_t g = -1;
-    unsigned bits = 0u;
-    if (valid && part == 0) {
-        if (found && found_eg) {
-            const int slot = roche_slot(sg.kind, blk.by);
-            A.el_ecl[slot * A.sz.nelem + e] = make_double2(a, egress < a ? egress + 1.0 : egress);
-            g = e / kEclGroup;
-            bits = 1u << slot;
+    for (int64_t k0 = (int64_t)blockIdx.x * (kRocheBlock / 2); k0 < n; k0 += (int64_t)gridDim.x * (kRocheBlock / 2)) {
+        const int64_t k = k0 + (threadIdx.x >> 1);
+        bool capped = false, found = false;
+        double a = 0.0, b = 0.0;
+        OpenElem o;
+        o.valid = false;
+        if (k < n) {
+            o = open_elem(A, A.open[k]);
+            if (o.valid) {
+                const double4 p = A.el_p64[o.e];
+                const int first = A.firsthit[k];
+                Scan sc;
+                if (part == 0 && scan_setup(*o.R, o.M->cosi_e, o.M->sini_e, o.M->delta, p.x, p.y, p.z, sc))
+                    cnt.fbl += first == kNoHit ? sc.nsteps + 1 : first + 1;  // the single scan's searches
+                found = ingress_egress<false>(*o.R, o.M->cosi_e, o.M->sini_e, o.M->delta, p.x, p.y, p.z, a, b, capped, cnt,
+                                              first, part + 1);
+            }
         }
-        if (capped || capped_eg) atomicOr(A.status + sg.model, kStatusIterCap);
+        const double egress = __shfl_xor_sync(0xffffffffu, b, 1);
+        const bool found_eg = __shfl_xor_sync(0xffffffffu, (int)found, 1) != 0;
+        const bool capped_eg = __shfl_xor_sync(0xffffffffu, (int)capped, 1) != 0;
+        int64_t g = -1;
+        unsigned bits = 0u;
+        if (o.valid && part == 0) {
+            if (found && found_eg) {
+                A.el_ecl[o.slot * A.sz.nelem + o.e] = make_double2(a, egress < a ? egress + 1.0 : egress);
+                g = o.e / kEclGroup;
+                bits = 1u << o.slot;
+            }
+            if (capped || capped_eg) atomicOr(A.status + o.model, kStatusIterCap);
+        }
+        group_or_warp(A.ecl_grp, g, bits);
     }
-    group_or_warp(A.ecl_grp, g, bits);
     roche_counters(A, cnt);
 }
 
@@ -2277,15 +1889,14 @@ cudaError_t launch_elements(const ElemArgs& a, cudaStream_t s) {
 
 cudaError_t launch_roche(const ElemArgs& a, cudaStream_t s) {
     if (a.nrblocks <= 0) return cudaSuccess;
-    if (a.roche_split <= 1) {
-        k_roche<<<(unsigned)a.nrblocks, kRocheBlock, 0, s>>>(a);
-        return cudaGetLastError();
-    }
-    // firsthit starts at kNoHit (memset by the caller's launch sequence)
-    k_roche_scan<<<(unsigned)(a.nrblocks * a.roche_split), kRocheBlock, 0, s>>>(a);
+    k_roche<<<(unsigned)(2 * a.nrblocks), kRocheBlock, 0, s>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_roche_chop2<<<(unsigned)(2 * a.nrblocks), kRocheBlock, 0, s>>>(a);
+    const unsigned grid = (unsigned)std::min<int64_t>(a.open_grid, 16 * a.nrblocks);
+    k_roche_open<<<grid, kRocheBlock, 0, s>>>(a);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    k_roche_chop2<<<grid, kRocheBlock, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -31,8 +31,13 @@ struct ElemArgs {
     int* status;         // per model
     int64_t nblocks, nrblocks, nablocks;
     unsigned long long* counters;  // [pot evals, dpot evals, fblink calls, bound nodes, proven misses] or null
-    int roche_split;     // threads per Roche-eclipsed element in the phase scan (1: one kernel)
-    int* firsthit;       // split scan: first hit per Roche thread (nrblocks x kRocheBlock), starts at 0x7f7f7f7f
+    unsigned* open;      // elements left to the general search: Roche block x kRocheBlock + slot
+    unsigned* nopen;     // their number (zeroed before k_roche)
+    int* firsthit;       // split scan: first hit per open element, set to kNoHit as it is listed
+    unsigned nfirst;     // entries of firsthit: longer lists are not split
+    int split_fix;       // threads per open element in the split scan; 0: by the list's length
+    int64_t split_target;  // scan threads that fill the GPU
+    int open_grid;       // blocks of the two general kernels
     int fblink_cap;      // potential evaluations allowed in one line-of-sight search (kFblinkEvalCap)
     Sizes sz;
 };

@@ -120,6 +120,26 @@ double face_gravity(bool primary, double q, double spin, V3 dirn, double rref, d
     return std::sqrt(norm2(dpot(primary, q, spin, add(cofm, scale(r, dirn)))));
 }
 
+// The surface's distance from the centre along a direction, to about 1e-6 (a first guess's input).
+double face_radius(bool primary, double q, double spin, V3 dirn, double rref, double pref) {
+    V3 cofm = primary ? V3{0, 0, 0} : V3{1.0, 0.0, 0.0};
+    double lo = 0.2 * rref, hi = rref;
+    for (int i = 0; i < 20; ++i) {
+        const double mid = 0.5 * (lo + hi);
+        if (pot(primary, q, spin, add(cofm, scale(mid, dirn))) < pref) lo = mid; else hi = mid;
+    }
+    return 0.5 * (lo + hi);
+}
+
+// Whether a Roche-distorted star is convex.  A lobe-filling star is convex up to its point at L1
+// when it has at most half the mass and rotates at least synchronously; a more massive one is
+// slightly hollow beside that point, but convex up to 95% of its lobe.  (Least principal curvature
+// over the surface times the lobe radius, mass ratios 1e-3..1e3, spins 1..6: > 0 in the first case,
+// 1e-4 for equal masses at the point; > 0.45 in the second.)
+int32_t roche_convex(double own, double spin, double ffac) {
+    return spin >= 1.0 && spin <= 6.0 && (own <= 0.5 || ffac <= 0.95);
+}
+
 // Planck function and its log-derivative (planck.rs:4-44).
 const double kFac1 = 2.0e27 * kH * kC;
 const double kFac2 = 1.0e9 * kH * kC / kK;
@@ -351,8 +371,14 @@ void prepare_model(const Model& m, const lcb_datum* data, int64_t ndata, ModelLa
     D.gref1 = m.roche1 ? face_gravity(true, q, spin1, {-1.0, 0.0, 0.0}, D.rref1, D.pref1, D.acc_face) : 1.0;
     D.gref2 = m.roche2 ? face_gravity(false, q, spin2, {1.0, 0.0, 0.0}, D.rref2, D.pref2, D.acc_face) : 1.0;
     double mu = q / (1.0 + q);
-    D.ecl1 = RocheEcl{mu, 1.0 - mu, sq(spin1), D.rref1, D.pref1, 0.0, 1, 0};
-    D.ecl2 = RocheEcl{mu, 1.0 - mu, sq(spin2), D.rref2, D.pref2, 1.0, 0, 0};
+    D.ecl1 = RocheEcl{mu, 1.0 - mu, sq(spin1), D.rref1, D.pref1, 0.0, 0.0, 0.0, 1, roche_convex(1.0 - mu, spin1, D.ffac1)};
+    D.ecl2 = RocheEcl{mu, 1.0 - mu, sq(spin2), D.rref2, D.pref2, 1.0, 0.0, 0.0, 0, roche_convex(mu, spin2, D.ffac2)};
+    for (RocheEcl* e : {&D.ecl1, &D.ecl2}) {
+        const bool first = e == &D.ecl1;
+        if (!(first ? m.roche1 : m.roche2)) continue;
+        e->ry = face_radius(first, q, first ? spin1 : spin2, {0.0, 1.0, 0.0}, e->rref, e->pref);
+        e->rz = face_radius(first, q, first ? spin1 : spin2, {0.0, 0.0, 1.0}, e->rref, e->pref);
+    }
     D.roche1 = m.roche1; D.roche2 = m.roche2; D.eclipse1 = m.eclipse1; D.eclipse2 = m.eclipse2;
     D.npole = m.npole; D.glens1 = m.glens1;
     D.add_disc = m.add_disc; D.opaque = m.opaque; D.add_spot = m.add_spot; D.iscale = m.iscale;
@@ -855,17 +881,16 @@ void plan_batch(const Model* const* models, int64_t n, const lcb_datum* data, co
                 for (int64_t off = 0; off < g.count; off += kRocheBlock) P.rblocks[k++] = ElemBlock{(int32_t)s, by, off};
     });
 
-    // small batches: spread each element's phase scan over several threads, a power
-    // of two up to 16, until about sixteen waves of scan threads fill the GPU (the
-    // choices an autotuning of 8..128-model batches made; large batches keep one
-    // thread per element, where the scan proves blocks of steps at once)
+    // small batches: where the general search runs, it spreads each element's phase scan over
+    // several threads (open_split's rule on the device, here for the case that every element is
+    // left to it)
     {
         const int64_t threads = (int64_t)P.rblocks.size() * kRocheBlock;
-        const int64_t target = (int64_t)std::max(num_sms, 1) * 640 * 16;
+        const int64_t target = split_target(num_sms);
         int split = 1;
         while (threads > 0 && split < 16 && (int64_t)(2 * split) * threads <= target) split *= 2;
         P.roche_split = split;
-        if (tune.roche_split > 0 && threads > 0) P.roche_split = std::min(std::max(tune.roche_split, 1), 16);
+        if (tune.roche_split > 0 && threads > 0) P.split_fix = P.roche_split = std::min(std::max(tune.roche_split, 1), 16);
     }
 
     // flux work units: choose the element range so there are a few units per resident block
@@ -989,7 +1014,7 @@ void plan_batch(const Model* const* models, int64_t n, const lcb_datum* data, co
     // shape key: what the device buffers and the captured graph depend on
     P.shape_key = {n, P.nelem, P.nsub, P.ndatum, P.npartial, (int64_t)P.units.size(), (int64_t)P.eblocks.size(),
                    (int64_t)P.rblocks.size(), (int64_t)P.ablocks.size(), (int64_t)P.segs.size(),
-                   (int64_t)P.bands.size(), (int64_t)P.rings.size(), (int64_t)P.roche_split,
+                   (int64_t)P.bands.size(), (int64_t)P.rings.size(), (int64_t)P.roche_split, (int64_t)P.split_fix,
                    (int64_t)P.flux_blocks_per_sm, (int64_t)P.curve_blocks, (int64_t)P.result_blocks,
                    (int64_t)P.curve_share};
 }

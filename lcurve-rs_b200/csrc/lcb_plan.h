@@ -38,7 +38,8 @@ struct Plan {
     // datum_src[d] == datum_src[0] + d for every d: the data can be copied as one range
     bool datum_contiguous = false;
     bool any_iscale = false;  // some model fits per-component scale factors (needs fcomp scratch)
-    int roche_split = 1;      // threads per Roche-eclipsed element in the phase scan
+    int roche_split = 1;      // threads per element of the general eclipse search, were every element left to it
+    int split_fix = 0;        // PlanTuning::roche_split where it applies: fixed, whatever the list's length
     int flux_chunks = 1;      // elements per flux work unit / kFluxChunk
     int flux_blocks_per_sm = 0;  // persistent flux blocks per SM; 0 = the occupancy limit
     int curve_blocks = 1, result_blocks = 1;  // blocks per model of k_curve and (scaled) k_results
@@ -54,6 +55,7 @@ struct Plan {
         datum_contiguous = false;
         any_iscale = false;
         roche_split = 1;
+        split_fix = 0;
         flux_chunks = 1;
         flux_blocks_per_sm = 0;
         curve_blocks = result_blocks = 1;
@@ -66,6 +68,9 @@ struct Plan {
 // invalid are marked failed (model_ok = 0) instead of throwing.
 void plan_batch(const Model* const* models, int64_t n, const lcb_datum* data, const int64_t* start,
                 const int64_t* count, int num_sms, Plan& out, const PlanTuning& tune = PlanTuning{});
+
+// Scan threads of the split eclipse search that fill the GPU: sixteen waves of five 128-thread blocks.
+inline int64_t split_target(int num_sms) { return (int64_t)(num_sms > 1 ? num_sms : 1) * 640 * 16; }
 
 // Host FP64 helpers also used by tests of the planner.
 double host_xl1(double q);
