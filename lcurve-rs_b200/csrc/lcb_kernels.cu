@@ -206,6 +206,37 @@ __device__ int disc_eclipse(const ModelDev& M, double rdisc1, double px, double 
     return 0;
 }
 
+// Where the ray from a Roche star's centre along (ux, uy, uz) meets its surface
+// (potential = pref): Newton's method from the ellipsoid of half widths ry and
+// rz.  The bisection of surface.rs:54-121 needs only the side of the surface a
+// radius lies on; away from the root by more than `tol` (the rounding of its
+// own potential evaluation, thousands of times over) the root tells, so the ~25
+// evaluations of two square roots and divisions each become ~5 of two
+// reciprocal square roots, and the radii keep their bits.  Not converged, or
+// too flat to trust (near L1): tol is infinite and every step evaluates.
+struct FaceRoot {
+    double r, tol;
+};
+__device__ __forceinline__ FaceRoot face_root(const RocheEcl& s, double ux, double uy, double uz) {
+    double r = inv_sqrt((ux * ux + uy * uy) / (s.ry * s.ry) + uz * uz / (s.rz * s.rz)), dr = 1.0, slope = 0.0;
+    for (int it = 0; it < 8 && fabs(dr) > 1e-9; ++it) {
+        const double x = fma(r, ux, s.cofmx), y = r * uy, z = r * uz;
+        const double x2y2 = x * x + y * y, r1sq = x2y2 + z * z, r2sq = r1sq + 1.0 - 2.0 * x;
+        const double i1 = inv_sqrt(r1sq), i2 = inv_sqrt(r2sq);
+        const double v = -s.comp * i1 - s.mu * i2;
+        const double f = s.primary ? v - s.ssq * x2y2 * 0.5 + s.mu * x : v - s.ssq * (0.5 + 0.5 * x2y2 - x) - s.comp * x;
+        const double a = s.comp * (i1 * i1 * i1), b = s.mu * (i2 * i2 * i2), w = x - 1.0;
+        const double gx = a * x + b * w - (s.primary ? s.ssq * x - s.mu : s.ssq * w - s.mu + 1.0);
+        slope = gx * ux + (a + b - s.ssq) * y * uy + (a + b) * z * uz;
+        dr = (f - s.pref) / slope;
+        r = fmin(fmax(r - dr, 0.2 * s.rref), s.rref);
+    }
+    // quadratic: a last step below 1e-9 leaves far less than tol; the potential's rounding is ~1e-15
+    // of its size (1/r of either star), in radius that over the slope
+    const bool ok = fabs(dr) <= 1e-9 && slope > 1e-2;
+    return FaceRoot{r, ok ? 1e-12 + 1e-13 * fmax(1.0, fabs(s.pref)) / slope : (double)INFINITY};
+}
+
 // Irradiated temperature (brightness.rs:150-174) -> temp, geom.
 __device__ __forceinline__ double irradiate(double tbase, double gravity, double gdcbol, double absorb, double tirr,
                                             double mu, double r, double rirr, double& geom) {
@@ -314,15 +345,23 @@ __global__ void __launch_bounds__(kElemThreads) k_elements(ElemArgs A) {
         if (roche) {  // face (surface.rs:54-121)
             const double ssq = primary ? sq(M.spin1) : sq(M.spin2);
             const double rref = primary ? M.rref1 : M.rref2, pref = primary ? M.pref1 : M.pref2;
-            double rlo = rref / 2.0, rhi = rref, t = pref + 1.0;
-            for (int k = 0; k < 30 && t > pref; ++k) {
+            const FaceRoot root = face_root(primary ? M.ecl1 : M.ecl2, ux, uy, uz);
+            // 1 below the surface, 0 on or above it (potential > pref), -1 equal
+            auto side = [&](double r) {
+                if (fabs(r - root.r) > root.tol) return r < root.r ? 1 : 0;
+                const double t = pot_exact(primary, M.q, ssq, cofm + r * ux, r * uy, r * uz);
+                return t < pref ? 1 : t > pref ? 0 : -1;
+            };
+            double rlo = rref / 2.0, rhi = rref;
+            bool above = true;
+            for (int k = 0; k < 30 && above; ++k) {
                 rlo = rhi / 2.0;
-                t = pot_exact(primary, M.q, ssq, cofm + rlo * ux, rlo * uy, rlo * uz);
-                if (t > pref) rhi = rlo;
+                above = side(rlo) == 0;
+                if (above) rhi = rlo;
             }
             for (int k = 0; k < 100 && rhi - rlo > M.acc_face; ++k) {
                 double mid = (rlo + rhi) / 2.0;
-                if (pot_exact(primary, M.q, ssq, cofm + mid * ux, mid * uy, mid * uz) < pref) rlo = mid;
+                if (side(mid) == 1) rlo = mid;
                 else rhi = mid;
             }
             rad = (rlo + rhi) / 2.0;
