@@ -261,7 +261,7 @@ void enqueue_run(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, int scale, int rd
     CUDA_TRY(lcb::launch_aux(ea, s));
     if (timed) CUDA_TRY(cudaEventRecord(C->ev[4], s));
     lcb::FluxArgs fa{D.models.as<lcb::ModelDev>(), D.units.as<lcb::FluxUnit>(), (int64_t)P.units.size(),
-                     D.counter.as<int>(), D.rec.as<float4>(), D.pos.as<float4>(), D.ecl.as<double2>(),
+                     P.flux_share, D.counter.as<int>(), D.rec.as<float4>(), D.pos.as<float4>(), D.ecl.as<double2>(),
                      D.egrp.as<unsigned>(), D.spe.as<float4>(), D.spphi.as<double>(), D.sptype.as<int8_t>(), D.partial.as<double>(),
                      D.status.as<int>(), sz};
     const int bps_max = lcb::flux_blocks_per_sm();

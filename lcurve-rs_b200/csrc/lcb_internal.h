@@ -145,7 +145,8 @@ struct ElemBlock {          // one block of an element kernel
 enum UnitKind : int32_t {
     UK_STAR_POLY1 = 0, UK_STAR_POLY2, UK_STAR_POLY3, UK_STAR_POLY4, UK_STAR_CLARET,
     UK_STAR_GENERIC,        // beaming and/or lensing
-    UK_DISC, UK_SPOT, UK_COUNT
+    UK_DISC, UK_DISC_LIN,   // disc and rim: quadratic or linear limb darkening
+    UK_SPOT, UK_COUNT
 };
 
 struct FluxUnit {

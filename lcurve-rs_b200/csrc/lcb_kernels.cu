@@ -74,9 +74,21 @@ constexpr int kRocheMinBlocks = LCB_ROCHE_MIN_BLOCKS;  // k_roche blocks per SM 
 constexpr int kScanMinBlocks = LCB_SCAN_MIN_BLOCKS;  // the same for the split scan (small batches)
 constexpr int kChopMinBlocks = LCB_CHOP_MIN_BLOCKS;  // and for its bisection kernel
 #ifndef LCB_FLUX_UNROLL
-#define LCB_FLUX_UNROLL 4
+#define LCB_FLUX_UNROLL 2
 #endif
-constexpr int kFluxUnroll = LCB_FLUX_UNROLL;  // list elements per unrolled step of the flux loop
+#ifndef LCB_DISC_UNROLL
+#define LCB_DISC_UNROLL 4
+#endif
+#ifndef LCB_LIMB_UNROLL
+#define LCB_LIMB_UNROLL 2
+#endif
+#ifndef LCB_GENERIC_UNROLL
+#define LCB_GENERIC_UNROLL 2
+#endif
+#ifndef LCB_FLUX_MIN_BLOCKS
+#define LCB_FLUX_MIN_BLOCKS 4
+#endif
+constexpr int kFluxMinBlocks = LCB_FLUX_MIN_BLOCKS;  // k_flux blocks per SM (128 threads): register budget
 __device__ __forceinline__ double rad2deg(double r) { return r * (180.0 / kPi); }
 
 __device__ __forceinline__ double planck_d(double wave, double temp) {  // planck.rs:16-23
@@ -912,15 +924,6 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)_
 __device__ __forceinline__ void mbar_init(uint64_t* bar) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)));
 }
-__device__ __forceinline__ void mbar_expect(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -961,23 +964,9 @@ __global__ void k_wait_probe(long long limit, int* status, long long* waited) {
 }
 
 enum { CLS_VIS = 0, CLS_MIX = 1, CLS_HID = 2 };
+constexpr int kFluxWarps = kFluxThreads / 32;
 // used-slot words a flux unit spans (units hold at most 16 chunks of elements)
 constexpr int kUnitGroups = 16 * kFluxChunk / kEclGroup + 2;
-
-struct FluxSmem {
-    float4 rec[2][kFluxChunk];
-    double2 ecl[2][kMaxEcl][kFluxChunk];  // the slots the chunk uses, slot-major
-    unsigned cmask[2];                    // which slots were staged
-    unsigned gw[kUnitGroups];             // the unit's words of used-slot masks (ecl_grp)
-    uint16_t list[kFluxChunk];   // contributing elements: index | pairs << 8 | (partly eclipsed << 15)
-    int wtot[2][kFluxThreads / 32];
-    uint64_t bar[2];
-    int unit;
-};
-static_assert(kFluxChunk == 2 * kFluxThreads, "the classification pass gives each thread two elements");
-static_assert(kFluxChunk <= 256 && kMaxEcl < 8, "list entries hold the element in 8 bits and its pairs in 3");
-
-size_t flux_smem_bytes_impl() { return sizeof(FluxSmem); }
 
 // Range classification of one eclipse pair against [lo, hi] (exact in FP64).
 __device__ __forceinline__ int pair_cls(double ing, double eg, double lo, double hi) {
@@ -986,36 +975,67 @@ __device__ __forceinline__ int pair_cls(double ing, double eg, double lo, double
     return CLS_MIX;
 }
 
-// Classifies element e of a staged chunk against the tile's phase range from
-// the chunk's staged slots `cm` (an unused slot, (inf, -inf), is neutral).
-__device__ __forceinline__ int classify(const double2 (*ecl)[kFluxChunk], unsigned cm, int e, const double* rlo,
-                                        const double* rhi) {
-    int res = -1;
-    for (int h = 0; h < 2; ++h) {
-        if (!(rlo[h] <= rhi[h])) continue;  // empty half
-        int c = CLS_VIS;
-        for (unsigned m = cm; m; m &= m - 1u) {
-            const double2 p = ecl[__ffs(m) - 1][e];
-            const int pc = pair_cls(p.x, p.y, rlo[h], rhi[h]);
-            if (pc == CLS_HID) { c = CLS_HID; break; }
-            if (pc == CLS_MIX) c = CLS_MIX;
+// The phases of some sub-phases: their range in each half of [0, 1).
+struct PhaseRange {
+    double lo[2], hi[2];
+    __device__ __forceinline__ void clear() {
+        lo[0] = lo[1] = 2.0;
+        hi[0] = hi[1] = -1.0;
+    }
+    // class of an element from its pairs' classes in the two halves (an empty half says nothing)
+    __device__ __forceinline__ int join(const int* cls) const {
+        const bool a = lo[0] <= hi[0], b = lo[1] <= hi[1];
+        if (a && b) return cls[0] == cls[1] ? cls[0] : CLS_MIX;
+        return a ? cls[0] : b ? cls[1] : CLS_HID;
+    }
+    __device__ __forceinline__ void add(int* cls, double2 p) const {
+        for (int h = 0; h < 2; ++h) cls[h] = max(cls[h], pair_cls(p.x, p.y, lo[h], hi[h]));
+    }
+    __device__ __forceinline__ void put(double p) {
+        const int h = p >= 0.5 ? 1 : 0;
+        lo[h] = fmin(lo[h], p);
+        hi[h] = fmax(hi[h], p);
+    }
+    __device__ __forceinline__ void join_range(const PhaseRange& r) {
+        for (int h = 0; h < 2; ++h) {
+            lo[h] = fmin(lo[h], r.lo[h]);
+            hi[h] = fmax(hi[h], r.hi[h]);
         }
-        if (res < 0) res = c;
-        else if (res != c) res = CLS_MIX;
     }
-    return res < 0 ? CLS_HID : res;
-}
+    // over the warp: doubles >= 0 are ordered as their bits, reduced a word at a time
+    __device__ __forceinline__ void warp_all() {
+        for (int h = 0; h < 2; ++h) {
+            const unsigned lh = __double2hiint(lo[h]), ll = __double2loint(lo[h]);
+            const unsigned mh = __reduce_min_sync(0xffffffffu, lh);
+            const unsigned ml = __reduce_min_sync(0xffffffffu, lh == mh ? ll : ~0u);
+            const bool none = hi[h] < 0.0;
+            const unsigned hh = none ? 0u : (unsigned)__double2hiint(hi[h]), hl = none ? 0u : (unsigned)__double2loint(hi[h]);
+            const unsigned xh = __reduce_max_sync(0xffffffffu, hh);
+            const unsigned xl = __reduce_max_sync(0xffffffffu, hh == xh ? hl : 0u);
+            lo[h] = __hiloint2double((int)mh, (int)ml);
+            hi[h] = lo[h] > 1.0 ? -1.0 : __hiloint2double((int)xh, (int)xl);
+        }
+    }
+};
 
-// Moves element e's used pairs among the staged slots `cm` to slots 0, 1, ..
-// (in place: a pair only moves to a lower slot); returns their number.
-__device__ __forceinline__ int compact_pairs(double2 (*ecl)[kFluxChunk], unsigned cm, int e) {
-    int n = 0;
-    for (unsigned m = cm; m; m &= m - 1u) {
-        const double2 p = ecl[__ffs(m) - 1][e];
-        if (p.x <= 2.0) ecl[n++][e] = p;
-    }
-    return n;
-}
+constexpr int kUnitLists = 16 * kFluxChunk / 32;  // groups of 32 elements of a unit
+constexpr int kQuarters = kFluxThreads / 32;      // a tile's sub-phases, a warp's worth each
+
+struct FluxWarpSmem {
+    float4 rec[32];               // the warp's current 32 elements
+    double2 pair[kMaxEcl][32];    // and the pairs of the mixed ones
+    double ph[32 * kFluxR];       // the phases of its current quarter
+};
+struct FluxUnitSmem {             // a unit, sorted (flux_sort)
+    PhaseRange own[kQuarters];    // of each quarter's sub-phases
+    float2 trig[4 + 2 * kQuarters];  // (sin, cos) of the ends of the tile's and the quarters' arcs
+    unsigned gw[kUnitGroups];     // the unit's words of used-slot masks (ecl_grp)
+    unsigned list[kUnitLists];    // per 32 elements: those on the tile's list
+    unsigned used[kUnitLists][kQuarters], plain[kUnitLists][kQuarters], mixed[kUnitLists][kQuarters];
+    int unit;
+};
+static_assert(kFluxChunk % 32 == 0, "a chunk is whole groups of 32 elements");
+
 
 // The earth vector of phase theta/2pi is (sini cos t, -sini sin t, cosi), so an
 // element's mu over a phase arc is A cos t + B sin t + C.  The tile's active
@@ -1024,88 +1044,119 @@ struct Arcs {
     float ca[2], sa[2], cb[2], sb[2];
     bool on[2];
 };
-// Largest mu of direction (dx, dy, dz) over the arcs (FP32; the caller keeps a margin).
-__device__ __forceinline__ float max_mu(const Arcs& a, float si, float ci, float dx, float dy, float dz) {
-    const float A = si * dx, B = -si * dy, C = ci * dz;
+// An element's mu over phases: A cos t + B sin t + C, amplitude R (a few ulp are
+// far inside the margins).
+struct MuCurve {
+    float A, B, C, R;
+    __device__ __forceinline__ MuCurve(float si, float ci, const float4& d) : A(si * d.x), B(-si * d.y), C(ci * d.z) {
+        asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(R) : "f"(A * A + B * B));
+    }
+};
+// Largest mu over the arcs (FP32; the caller keeps a margin).
+__device__ __forceinline__ float max_mu(const Arcs& a, const MuCurve& u) {
     float m = -2.f;
     for (int h = 0; h < 2; ++h) {
         if (!a.on[h]) continue;
-        float in1 = a.ca[h] * B - a.sa[h] * A, in2 = A * a.sb[h] - B * a.cb[h];
-        float v = (in1 >= 0.f && in2 >= 0.f) ? sqrtf(A * A + B * B)
-                                              : fmaxf(A * a.ca[h] + B * a.sa[h], A * a.cb[h] + B * a.sb[h]);
-        m = fmaxf(m, v + C);
+        float in1 = a.ca[h] * u.B - a.sa[h] * u.A, in2 = u.A * a.sb[h] - u.B * a.cb[h];
+        float v = (in1 >= 0.f && in2 >= 0.f) ? u.R : fmaxf(u.A * a.ca[h] + u.B * a.sa[h], u.A * a.cb[h] + u.B * a.sb[h]);
+        m = fmaxf(m, v + u.C);
     }
     return m;
 }
 constexpr float kFacingMargin = 2e-5f;  // far above the FP32 rounding of mu
 
-// The thread's sub-phases (bit k: phase ph[k]) at which element e is behind one
-// of its npair pairs (moved to slots 0 .. npair-1 by compact_pairs).
-__device__ __forceinline__ unsigned hidden_mask(const double2 (*ecl)[kFluxChunk], int npair, int e,
-                                                const double* ph) {
-    unsigned h = 0u;
-#pragma unroll 1
-    for (int j = 0; j < npair; ++j) {
-        const double2 p = ecl[j][e];
-#pragma unroll
-        for (int k = 0; k < kFluxR; ++k)
-            h |= (((ph[k] >= p.x && ph[k] <= p.y) || ph[k] <= p.y - 1.0) ? 1u : 0u) << k;
+// The single arc (shorter than pi) that a quarter's sub-phases lie on, and an
+// element's extreme mu over it.
+struct WarpArc {
+    float ca, sa, cb, sb;
+    // from the ranges in the two halves of [0, 1): the arc's ends; false: none such
+    static __device__ __forceinline__ bool ends(const PhaseRange& r, double& from, double& to) {
+        const bool a = r.lo[0] <= r.hi[0], b = r.lo[1] <= r.hi[1];
+        from = a ? r.lo[0] : r.lo[1];
+        to = b ? r.hi[1] : r.hi[0];
+        if (a && b && to - from > 0.5) {  // through 0 instead of 0.5
+            from = r.lo[1];
+            to = r.hi[0] + 1.0;
+        }
+        return (a || b) && to - from < 0.49;
     }
+    __device__ __forceinline__ void range(const MuCurve& u, float& mn, float& mx) const {
+        const float va = u.A * ca + u.B * sa, vb = u.A * cb + u.B * sb;
+        const float up = u.B * ca - u.A * sa, down = u.A * sb - u.B * cb;  // slope at the start, fall at the end
+        mx = (up >= 0.f && down >= 0.f ? u.R : fmaxf(va, vb)) + u.C;
+        mn = (up <= 0.f && down <= 0.f ? -u.R : fminf(va, vb)) + u.C;
+    }
+};
+
+// The thread's sub-phases (bit k: phase ph[32 k]) at which element e is behind
+// one of its npair >= 1 pairs.
+__device__ __forceinline__ unsigned hidden_mask(const double2 (*ecl)[32], int npair, int e, const double* ph) {
+    unsigned h = 0u;
+    auto test = [&](double2 p) {
+#pragma unroll
+        for (int k = 0; k < kFluxR; ++k) {
+            const double x = ph[32 * k];
+            h |= (((x >= p.x && x <= p.y) || x <= p.y - 1.0) ? 1u : 0u) << k;
+        }
+    };
+    test(ecl[0][e]);
+#pragma unroll 1
+    for (int j = 1; j < npair; ++j) test(ecl[j][e]);
     return h;
+}
+
+// 1/sqrt(x) of a normal positive x, by the hardware estimate that rsqrtf rounds to as well.
+__device__ __forceinline__ float rsqrt_normal(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// The mu above which an element of a unit's kind is seen.
+__device__ __forceinline__ float mu_threshold(const ModelDev& M, int kind, int star) {
+    if (kind == UK_DISC || kind == UK_DISC_LIN || kind == UK_SPOT) return 0.f;
+    const float mc = star == 1 ? M.mucrit1f : M.mucrit2f;
+    return kind == UK_STAR_GENERIC ? mc : fmaxf(mc, 0.f);  // see(mu) alone for the generic one
 }
 
 // Per-kind contribution of one element at one sub-phase (FP32).
 template <int KIND>
 struct Contrib {
-    float a0, a1, a2, a3, thr, sumc;  // LD coefficients, mu threshold, sum of Claret coefficients
+    float a0, a1, a2, a3, thr, sumc, minus0;  // LD coefficients, mu threshold, sum of Claret coefficients
     __device__ void setup(const ModelDev& M, int star) {
+        minus0 = __int_as_float(M.nslots >= 0 ? (int)0x80000000 : 0);
         const float* l = star == 1 ? M.ld1f : M.ld2f;
         a0 = l[0]; a1 = l[1]; a2 = l[2]; a3 = l[3];
-        float mc = star == 1 ? M.mucrit1f : M.mucrit2f;
-        thr = fmaxf(mc, 0.f);
+        thr = mu_threshold(M, KIND, star);
         sumc = a0 + a1 + a2 + a3;
-        if (KIND == UK_DISC) { a0 = M.lin_ldf; a1 = M.quad_ldf; thr = 0.f; }
-        if (KIND == UK_SPOT) thr = 0.f;
+        if (KIND == UK_DISC || KIND == UK_DISC_LIN) { a0 = M.lin_ldf; a1 = M.quad_ldf; }
     }
-    __device__ __forceinline__ float operator()(float mu, float fl) const {
-        if (KIND == UK_SPOT) return mu * fl;
-        if (KIND == UK_DISC) {
-            float om = 1.f - mu;
-            return mu * fl * (1.f - om * (a0 + a1 * om));
-        }
-        if (KIND == UK_STAR_CLARET) {
-            float m = fminf(mu, 1.f);
-            float ms = m * rsqrtf(m);
-            float im = (1.f - sumc) + ms * (a0 + ms * (a1 + ms * (a2 + ms * a3)));
-            return mu * fl * im;
-        }
-        float om = 1.f - fminf(mu, 1.f);
-        float p;
-        if (KIND == UK_STAR_POLY1) p = a0;
-        else if (KIND == UK_STAR_POLY2) p = a0 + om * a1;
-        else if (KIND == UK_STAR_POLY3) p = a0 + om * (a1 + om * a2);
-        else p = a0 + om * (a1 + om * (a2 + om * a3));
-        return mu * fl * (1.f - om * p);
-    }
-    // Two sub-phases at once with the packed FP32x2 pipe (sm_100): the same
-    // operations as operator(), each lane rounded as its scalar counterpart.
+    // Two sub-phases at once with the packed FP32x2 pipe (sm_100): each lane
+    // rounded as a scalar operation is.
+    // kInside: mu < 1 is known, so the clamp to 1 is left out (same bits), and
+    // the product is an FMA with -0 (the same rounding; a value the compiler does
+    // not know): it would fuse a plain packed product with the packed sum after it.
+    template <bool kInside>
     __device__ __forceinline__ float2 pair(float2 mu, float fl) const {
         const float2 one = make_float2(1.f, 1.f), f2 = make_float2(fl, fl);
+        const float2 nz = make_float2(minus0, minus0);
+        auto product = [&](float2 x, float2 y) { return kInside ? __ffma2_rn(x, y, nz) : __fmul2_rn(x, y); };
+        if (KIND == UK_SPOT) return product(mu, f2);
         const float2 mf = __fmul2_rn(mu, f2);
-        if (KIND == UK_SPOT) return mf;
-        if (KIND == UK_DISC) {
-            const float2 om = __fadd2_rn(one, make_float2(-mu.x, -mu.y));
-            const float2 q = __ffma2_rn(make_float2(a1, a1), om, make_float2(a0, a0));
-            return __fmul2_rn(mf, __ffma2_rn(make_float2(-om.x, -om.y), q, one));
+        if (KIND == UK_DISC || KIND == UK_DISC_LIN) {  // linear law: a1 om + a0 is a0
+            const float2 om = __fadd2_rn(one, make_float2(-mu.x, -mu.y)), c0 = make_float2(a0, a0);
+            const float2 q = KIND == UK_DISC ? __ffma2_rn(make_float2(a1, a1), om, c0) : c0;
+            return product(mf, __ffma2_rn(make_float2(-om.x, -om.y), q, one));
         }
-        const float2 m = make_float2(fminf(mu.x, 1.f), fminf(mu.y, 1.f));
+        const float2 m = kInside ? mu : make_float2(fminf(mu.x, 1.f), fminf(mu.y, 1.f));
         if (KIND == UK_STAR_CLARET) {
-            const float2 ms = __fmul2_rn(m, make_float2(rsqrtf(m.x), rsqrtf(m.y)));
+            const float2 ms = __fmul2_rn(m, kInside ? make_float2(rsqrt_normal(m.x), rsqrt_normal(m.y))
+                                                               : make_float2(rsqrtf(m.x), rsqrtf(m.y)));
             float2 h = __ffma2_rn(ms, make_float2(a3, a3), make_float2(a2, a2));
             h = __ffma2_rn(ms, h, make_float2(a1, a1));
             h = __ffma2_rn(ms, h, make_float2(a0, a0));
             const float2 im = __ffma2_rn(ms, h, make_float2(1.f - sumc, 1.f - sumc));
-            return __fmul2_rn(mf, im);
+            return product(mf, im);
         }
         const float2 om = __fadd2_rn(one, make_float2(-m.x, -m.y));
         float2 p;
@@ -1119,7 +1170,7 @@ struct Contrib {
             p = __ffma2_rn(om, p, make_float2(a1, a1));
             p = __ffma2_rn(om, p, make_float2(a0, a0));
         }
-        return __fmul2_rn(mf, __ffma2_rn(make_float2(-om.x, -om.y), p, one));
+        return product(mf, __ffma2_rn(make_float2(-om.x, -om.y), p, one));
     }
 };
 
@@ -1133,251 +1184,361 @@ __device__ __forceinline__ float imu_f(const float* l, int lt, float mu) {
     return (1.f - (l[0] + l[1] + l[2] + l[3])) + ms * (l[0] + ms * (l[1] + ms * (l[2] + ms * l[3])));
 }
 
-template <int KIND>
-__device__ void flux_unit(const FluxArgs& A, const FluxUnit& U, FluxSmem& S, uint32_t* parity) {
+// A unit's sub-phases are worked on in quarters of 32 n consecutive ones, n =
+// ceil(tile / 128) to a thread, so that a quarter's lines of sight span a
+// quarter of the tile's arc.  kBlock: the block's four warps share a unit, one
+// quarter each, and sort its elements together; else each warp has a unit of its
+// own and no barrier is met anywhere.
+// flux_sort fills the unit's element masks; not a template over the kinds, so
+// that all of them share its code.  Returns the quarters that have sub-phases
+// (bit 2 q).
+__device__ __forceinline__ bool sub_active(const FluxUnit& U, int t) {
+    if (U.star == 1) return U.role == ROLE_BOTH || ((U.role == ROLE_FINE) == (t == 1));
+    if (U.star == 2) return U.role == ROLE_BOTH || ((U.role == ROLE_FINE) == (t == 3));
+    return true;
+}
+
+template <bool kBlock>
+__device__ __noinline__ unsigned flux_sort(const FluxArgs& A, const FluxUnit& U, FluxUnitSmem& S) {
     const ModelDev& M = A.models[U.model];
-    const int tid = threadIdx.x;
+    const int lane = threadIdx.x & 31;
     const int64_t sbase = M.sub_begin + U.t0;
-    // ---- the tile's sub-phases in registers
-    float ex[kFluxR], ey[kFluxR], ez[kFluxR];
-    double ph[kFluxR];
-    bool act[kFluxR];
-    double dlo[2] = {2.0, 2.0}, dhi[2] = {-1.0, -1.0};
+    const int nslot = min(kFluxR, (U.nt + kFluxThreads - 1) / kFluxThreads);
+    // ---- phase ranges of the quarters and of the tile, which decides the list of elements
+    const int first = kBlock ? threadIdx.x >> 5 : 0, step = kBlock ? kFluxWarps : 1;
+    auto sync = [] {
+        if (kBlock) __syncthreads();
+        else __syncwarp();
+    };
+    for (int q = first; q < kQuarters; q += step) {
+        PhaseRange own;
+        own.clear();
 #pragma unroll
-    for (int k = 0; k < kFluxR; ++k) {
-        int j = tid + k * kFluxThreads;
-        act[k] = false;
-        ex[k] = ey[k] = ez[k] = 0.f;
-        ph[k] = -1.0;
-        if (j < U.nt) {
-            int t = A.sp_type[sbase + j];
-            bool a = true;
-            if (U.star == 1) a = U.role == ROLE_BOTH || ((U.role == ROLE_FINE) == (t == 1));
-            else if (U.star == 2) a = U.role == ROLE_BOTH || ((U.role == ROLE_FINE) == (t == 3));
-            if (a) {
-                float4 e = A.sp_e[sbase + j];
-                ex[k] = e.x; ey[k] = e.y; ez[k] = e.z;
-                ph[k] = A.sp_phi[sbase + j];
-                act[k] = true;
-                int h = ph[k] >= 0.5 ? 1 : 0;
-                dlo[h] = fmin(dlo[h], ph[k]);
-                dhi[h] = fmax(dhi[h], ph[k]);
+        for (int k = 0; k < kFluxR; ++k) {
+            const int j = (q * nslot + k) * 32 + lane;
+            if (k < nslot && j < U.nt && sub_active(U, A.sp_type[sbase + j])) own.put(A.sp_phi[sbase + j]);
+        }
+        own.warp_all();
+        if (lane == 0) S.own[q] = own;
+    }
+    // the unit's used-slot words
+    const int64_t g0 = U.e0 / kEclGroup;
+    const int ngw = (int)((U.e0 + U.ne - 1) / kEclGroup - g0 + 1);
+    for (int t = first * 32 + lane; t < ngw && t < kUnitGroups; t += 32 * step) S.gw[t] = A.ecl_grp[g0 + t];
+    sync();
+    PhaseRange tile = S.own[0];
+    for (int q = 1; q < kQuarters; ++q) tile.join_range(S.own[q]);
+    const bool any = tile.lo[0] <= tile.hi[0] || tile.lo[1] <= tile.hi[1];
+    unsigned arc_on = 0u, arc_one = 0u;  // quarters with sub-phases; with all of them on one arc
+    if (lane < 4 + 2 * kQuarters) {  // an angle per lane
+        float x = 0.f;
+        if (lane < 4) {
+            const int h = lane >> 1;
+            if (tile.lo[h] <= tile.hi[h]) x = (float)((lane & 1) ? tile.hi[h] : tile.lo[h]);
+        } else {
+            double from, to;
+            const PhaseRange& r = S.own[(lane - 4) >> 1];
+            if (WarpArc::ends(r, from, to)) arc_one = 1u;
+            if (r.lo[0] <= r.hi[0] || r.lo[1] <= r.hi[1]) arc_on = 1u;
+            x = (float)((lane & 1) ? to : from);
+        }
+        float sn, cs;
+        sincospif(2.f * x, &sn, &cs);
+        S.trig[lane] = make_float2(sn, cs);
+    }
+    arc_on = __ballot_sync(0xffffffffu, arc_on != 0u);
+    arc_one = __ballot_sync(0xffffffffu, arc_one != 0u);
+    __syncwarp();
+    const float sif = (float)M.sini_l, cif = (float)M.cosi_l;
+    const bool generic = U.kind == UK_STAR_GENERIC;
+    const float thr = mu_threshold(M, U.kind, U.star), face_thr = thr - kFacingMargin;
+    const int ngroups = any ? (U.ne + 31) / 32 : 0;
+    const float4* recs = A.el_rec + U.e0 + lane;
+
+    // ---- sort the elements, 32 at a time, a lane each.  The tile's list: those
+    // that face the observer somewhere on the tile and are not hidden on all of it;
+    // every 32 listed elements of a chunk the FP32 sums are folded into a two-sum
+    // pair.  A quarter's arc then sorts the listed ones: those that never face it
+    // or are hidden on all of it add nothing and are left out (leaving out zeros
+    // changes neither blocks nor sums); plain ones face it throughout, unhidden and
+    // with mu < 1, and need no test per sub-phase; limb ones need the test of mu;
+    // mixed ones that of their pairs too.
+    {
+        Arcs arcs;
+        for (int h = 0; h < 2; ++h) {
+            arcs.on[h] = tile.lo[h] <= tile.hi[h];
+            arcs.sa[h] = S.trig[2 * h].x; arcs.ca[h] = S.trig[2 * h].y;
+            arcs.sb[h] = S.trig[2 * h + 1].x; arcs.cb[h] = S.trig[2 * h + 1].y;
+        }
+        float4 next = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (first * 32 + lane < U.ne) next = __ldg(recs + first * 32);
+        for (int g = first; g < ngroups; g += step) {
+            const MuCurve curve(sif, cif, next);
+            const bool in = g * 32 + lane < U.ne;
+            if ((g + step) * 32 + lane < U.ne) next = __ldg(recs + (g + step) * 32);
+            bool list = in && !(max_mu(arcs, curve) <= face_thr);
+            unsigned cls = 0u;  // per quarter two bits
+            if (list) {
+                const int64_t e = U.e0 + g * 32 + lane;
+                const unsigned cm = S.gw[e / kEclGroup - g0];
+                if (cm) {
+                    int ct[2] = {CLS_VIS, CLS_VIS};
+                    for (unsigned m = cm; m; m &= m - 1u)  // an unused slot, (inf, -inf), is neutral
+                        tile.add(ct, __ldg(A.el_ecl + (__ffs(m) - 1) * A.sz.nelem + e));
+                    const int t = tile.join(ct);
+                    list = t != CLS_HID;
+                    if (t == CLS_MIX)
+                        for (int q = 0; q < kQuarters; ++q) {
+                            int cq[2] = {CLS_VIS, CLS_VIS};
+                            for (unsigned m = cm; m; m &= m - 1u)
+                                S.own[q].add(cq, __ldg(A.el_ecl + (__ffs(m) - 1) * A.sz.nelem + e));
+                            cls |= (unsigned)S.own[q].join(cq) << (2 * q);
+                        }
+                }
+            }
+            const unsigned listed = __ballot_sync(0xffffffffu, list);
+            if (lane == 0) S.list[g] = listed;
+            if (!listed) continue;
+            for (int q = 0; q < kQuarters; ++q) {
+                const unsigned c = (cls >> (2 * q)) & 3u;
+                bool use = list && c != CLS_HID, plain = false;
+                if ((arc_one >> (4 + 2 * q)) & 1u) {
+                    const float2 a = S.trig[4 + 2 * q], b = S.trig[5 + 2 * q];
+                    float mn, mx;
+                    WarpArc{a.y, a.x, b.y, b.x}.range(curve, mn, mx);
+                    use = use && mx > face_thr;
+                    plain = !generic && c == CLS_VIS && mn > thr + kFacingMargin && mx < 1.f - kFacingMargin;
+                }
+                const unsigned us = __ballot_sync(0xffffffffu, use), pl = __ballot_sync(0xffffffffu, use && plain);
+                const unsigned mi = __ballot_sync(0xffffffffu, use && c == CLS_MIX);
+                if (lane == 0) {
+                    S.used[g][q] = us;
+                    S.plain[g][q] = pl;
+                    S.mixed[g][q] = mi;
+                }
             }
         }
     }
-    // the unit's used-slot words, read once (issue() combines them per chunk)
+    sync();
+    return any ? arc_on >> 4 & 0x55u : 0u;
+}
+
+// Quarters [q0, q1) of a sorted unit, by one warp.
+template <int KIND>
+__device__ __forceinline__ void flux_unit(const FluxArgs& A, const FluxUnit& U, int q0, int q1, unsigned arc_on,
+                                          const FluxUnitSmem& T, FluxWarpSmem& S) {
+    const ModelDev& M = A.models[U.model];
+    const int lane = threadIdx.x & 31;
+    const int64_t sbase = M.sub_begin + U.t0;
+    const int nslot = min(kFluxR, (U.nt + kFluxThreads - 1) / kFluxThreads);
+    q1 = min(q1, (U.nt + 32 * nslot - 1) / (32 * nslot));
     const int64_t g0 = U.e0 / kEclGroup;
-    const int ngw = (int)((U.e0 + U.ne - 1) / kEclGroup - g0 + 1);
-    for (int t = tid; t < ngw && t < kUnitGroups; t += kFluxThreads) S.gw[t] = A.ecl_grp[g0 + t];
-    // block min/max of the two halves
-    for (int h = 0; h < 2; ++h) {
-        double a = dlo[h], b = dhi[h];
-        for (int o = 16; o > 0; o >>= 1) {
-            a = fmin(a, __shfl_xor_sync(0xffffffffu, a, o));
-            b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
-        }
-        dlo[h] = a; dhi[h] = b;
-    }
-    __shared__ double s_lo[kFluxThreads / 32][2], s_hi[kFluxThreads / 32][2];
-    if ((tid & 31) == 0) {
-        s_lo[tid >> 5][0] = dlo[0]; s_lo[tid >> 5][1] = dlo[1];
-        s_hi[tid >> 5][0] = dhi[0]; s_hi[tid >> 5][1] = dhi[1];
-    }
-    __syncthreads();
-    double rlo[2] = {2.0, 2.0}, rhi[2] = {-1.0, -1.0};
-    for (int w = 0; w < kFluxThreads / 32; ++w)
-        for (int h = 0; h < 2; ++h) { rlo[h] = fmin(rlo[h], s_lo[w][h]); rhi[h] = fmax(rhi[h], s_hi[w][h]); }
-    const bool any = rlo[0] <= rhi[0] || rlo[1] <= rhi[1];
-    Arcs arcs;
-    for (int h = 0; h < 2; ++h) {
-        arcs.on[h] = rlo[h] <= rhi[h];
-        float lo = arcs.on[h] ? (float)rlo[h] : 0.f, hi = arcs.on[h] ? (float)rhi[h] : 0.f;
-        sincospif(2.f * lo, &arcs.sa[h], &arcs.ca[h]);
-        sincospif(2.f * hi, &arcs.sb[h], &arcs.cb[h]);
-    }
-    const float sif = (float)M.sini_l, cif = (float)M.cosi_l;
-
-    static_assert(kFluxR % 2 == 0, "sub-phases are processed in pairs");
-    float2 ex2[kFluxR / 2], ey2[kFluxR / 2], ez2[kFluxR / 2];
-#pragma unroll
-    for (int k = 0; k < kFluxR; k += 2) {
-        ex2[k / 2] = make_float2(ex[k], ex[k + 1]);
-        ey2[k / 2] = make_float2(ey[k], ey[k + 1]);
-        ez2[k / 2] = make_float2(ez[k], ez[k + 1]);
-    }
-    float acc_hi[kFluxR], acc_lo[kFluxR];
-#pragma unroll
-    for (int k = 0; k < kFluxR; ++k) acc_hi[k] = acc_lo[k] = 0.f;
-
+    const int ngroups = (U.ne + 31) / 32;
+    const float4* recs = A.el_rec + U.e0 + lane;
     Contrib<KIND> C;
     C.setup(M, U.star);
-    const float face_thr = (KIND == UK_STAR_GENERIC ? (U.star == 1 ? M.mucrit1f : M.mucrit2f) : C.thr) - kFacingMargin;
+    // elements per unrolled step: more hides latency in long runs (a disc's), more code costs
+    // instruction fetches where stars of two laws share an SM
+    constexpr int kPlainUnroll = KIND == UK_DISC || KIND == UK_DISC_LIN ? LCB_DISC_UNROLL : LCB_FLUX_UNROLL;
+    constexpr int kTestUnroll = KIND == UK_STAR_GENERIC ? LCB_GENERIC_UNROLL : LCB_LIMB_UNROLL;
     // generic-path constants
     const float* ldg = U.star == 1 ? M.ld1f : M.ld2f;
     const int ltg = U.star == 1 ? M.ltype1 : M.ltype2;
     const float beam = U.star == 1 ? M.beam1f : M.beam2f;
     const float spin = U.star == 1 ? M.spin1f : M.spin2f;
-    const float thrg = U.star == 1 ? M.mucrit1f : M.mucrit2f;  // see(mu) without the mu > 0 shortcut
     const bool lens = U.star == 2 && M.glens1;
+    double* out = A.partial + M.pbase + (int64_t)U.slot * M.nsub + U.t0;
+    static_assert(kFluxR % 2 == 0, "sub-phases are processed in pairs");
 
-    const int nchunks = any ? (U.ne + kFluxChunk - 1) / kFluxChunk : 0;
-    auto issue = [&](int c) {
-        int b = c & 1;
-        int64_t e0 = U.e0 + (int64_t)c * kFluxChunk;
-        int n = min(kFluxChunk, U.ne - c * kFluxChunk);
-        // only the eclipse slots some element of the chunk uses
-        unsigned cm = 0;
-        for (int64_t g = e0 / kEclGroup; g <= (e0 + n - 1) / kEclGroup; ++g)
-            cm |= g - g0 < kUnitGroups ? S.gw[g - g0] : A.ecl_grp[g];
-        S.cmask[b] = cm;  // published to the waiting threads by the arrive below
-        uint32_t bytes = (uint32_t)n * 16u * (1u + (uint32_t)__popc(cm));
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_expect(&S.bar[b], bytes);
-        bulk_load(S.rec[b], A.el_rec + e0, (uint32_t)n * 16u, &S.bar[b]);
-        for (int k = 0; k < kMaxEcl; ++k)
-            if ((cm >> k) & 1u) bulk_load(S.ecl[b][k], A.el_ecl + k * A.sz.nelem + e0, (uint32_t)n * 16u, &S.bar[b]);
-    };
-    if (tid == 0) {
-        if (nchunks > 0) issue(0);
-        if (nchunks > 1) issue(1);
-    }
-    for (int c = 0; c < nchunks; ++c) {
-        const int b = c & 1;
-        const int n = min(kFluxChunk, U.ne - c * kFluxChunk);
-        if (!mbar_wait(&S.bar[b], parity[b])) atomicOr(A.status + U.model, kStatusTmaTimeout);
-        parity[b] ^= 1u;
-        const unsigned cm = S.cmask[b];
-        // classify every element of the chunk and list the contributing ones in
-        // ascending order (ballot prefix sums): the loop below then runs over a
-        // dense list without per-element branches
-        const int lane = tid & 31, warp = tid >> 5;
-        uint16_t ent[2];
-        unsigned keep[2];
+    // ---- the sums, a quarter at a time
+    for (int quarter = q0; quarter < q1; ++quarter) {
+        const int j0 = quarter * 32 * nslot + lane;  // the thread's sub-phases: j0 + 32 k, k < nslot
+        float ex[kFluxR], ey[kFluxR], ez[kFluxR];
+        float2 ex2[kFluxR / 2], ey2[kFluxR / 2], ez2[kFluxR / 2], part[kFluxR / 2];
+        float acc_hi[kFluxR], acc_lo[kFluxR];
+        unsigned act = 0u;
 #pragma unroll
-        for (int rr = 0; rr < 2; ++rr) {
-            const int e = tid + rr * kFluxThreads;
-            int cl = CLS_HID;
-            if (e < n) {
-                cl = classify(S.ecl[b], cm, e, rlo, rhi);
-                if (cl != CLS_HID) {  // never facing the observer on this tile: contributes exactly 0
-                    const float4 r = S.rec[b][e];
-                    if (max_mu(arcs, sif, cif, r.x, r.y, r.z) <= face_thr) cl = CLS_HID;
-                }
+        for (int k = 0; k < kFluxR; ++k) {
+            const int j = j0 + 32 * k;
+            float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
+            double ph = -1.0;
+            if (k < nslot && j < U.nt && sub_active(U, A.sp_type[sbase + j])) {
+                e = A.sp_e[sbase + j];
+                ph = A.sp_phi[sbase + j];
+                act |= 1u << k;
             }
-            // list entry: element | pairs << 8 | partly eclipsed << 15 (the pairs of a
-            // partly eclipsed element are moved to the front for hidden_at)
-            ent[rr] = (uint16_t)(cl == CLS_MIX ? (e | compact_pairs(S.ecl[b], cm, e) << 8 | 0x8000) : e);
-            keep[rr] = __ballot_sync(0xffffffffu, cl != CLS_HID);
-            if (lane == 0) S.wtot[rr][warp] = __popc(keep[rr]);
+            S.ph[32 * k + lane] = ph;
+            ex[k] = e.x; ey[k] = e.y; ez[k] = e.z;
+            acc_hi[k] = acc_lo[k] = 0.f;
         }
-        __syncthreads();
-        int nlist = 0;
-        {
-            const unsigned below = (1u << lane) - 1u;
-            int base = 0;
 #pragma unroll
-            for (int rr = 0; rr < 2; ++rr) {
-                int off = base;
-                for (int w = 0; w < kFluxThreads / 32; ++w) {
-                    if (w == warp) off = base;
-                    base += S.wtot[rr][w];
-                }
-                if ((keep[rr] >> lane) & 1u) S.list[off + __popc(keep[rr] & below)] = ent[rr];
-            }
-            nlist = base;
+        for (int k = 0; k < kFluxR; k += 2) {
+            ex2[k / 2] = make_float2(ex[k], ex[k + 1]);
+            ey2[k / 2] = make_float2(ey[k], ey[k + 1]);
+            ez2[k / 2] = make_float2(ez[k], ez[k + 1]);
+            part[k / 2] = make_float2(0.f, 0.f);
         }
-        __syncthreads();
-        for (int s0 = 0; s0 < nlist; s0 += 32) {
-            float part[kFluxR];
+        auto fold = [&] {
 #pragma unroll
-            for (int k = 0; k < kFluxR; ++k) part[k] = 0.f;
-            const int s1 = min(s0 + 32, nlist);
-#pragma unroll kFluxUnroll
-            for (int q = s0; q < s1; ++q) {
-                const int ev = S.list[q];
-                const int e = ev & 0xff;
-                const float4 r = S.rec[b][e];
-                // sub-phases behind one of a partly eclipsed element's pairs (bit k: sub-phase k)
-                const unsigned hid = (ev & 0x8000) ? hidden_mask(S.ecl[b], (ev >> 8) & 7, e, ph) : 0u;
-                if (KIND == UK_STAR_GENERIC) {
-                    const float4 p = __ldg(A.el_pos + U.e0 + (int64_t)c * kFluxChunk + e);
-                    float vx, vy;
-                    if (U.star == 1) { vx = -M.vfacf * spin * p.y; vy = M.vfacf * (spin * p.x - M.xcofmf); }
-                    else { vx = -M.vfacf * spin * p.y; vy = M.vfacf * (spin * (p.x - 1.f) + 1.f - M.xcofmf); }
-                    const float vn = r.x * vx + r.y * vy;
-#pragma unroll
-                    for (int k = 0; k < kFluxR; ++k) {
-                        float mu = ex[k] * r.x + ey[k] * r.y + ez[k] * r.z;
-                        bool v = mu > thrg && !((hid >> k) & 1u);
-                        if (v) {
-                            float mag = 1.f;
-                            if (lens) {
-                                float d = -(p.x * ex[k] + p.y * ey[k] + p.z * ez[k]);
-                                if (d > 0.f) {
-                                    float ax = p.x + d * ex[k], ay = p.y + d * ey[k], az = p.z + d * ez[k];
-                                    float pp = sqrtf(ax * ax + ay * ay + az * az), phh = pp * 0.5f, phsq = phh * phh;
-                                    float rd = M.rlens1f * d;
-                                    float pd = phsq > 25.f * rd ? pp + rd / pp : phh + sqrtf(phsq + rd);
-                                    mag = pd * pd / (pd - phh) / phh * 0.25f;
-                                }
-                            }
-                            if (beam != 0.f) {
-                                float vr = -(ex[k] * vx + ey[k] * vy);
-                                float mud = mu - mu * vr - vn;
-                                part[k] += mu * mag * r.w * (1.f - beam * vr) * imu_f(ldg, ltg, mud);
-                            } else {
-                                part[k] += mu * mag * r.w * imu_f(ldg, ltg, mu);
-                            }
-                        }
-                    }
-                } else {
-                    // sub-phases in pairs on the packed FP32x2 pipe
-                    const float2 rx = make_float2(r.x, r.x), ry = make_float2(r.y, r.y), rz = make_float2(r.z, r.z);
-#pragma unroll
-                    for (int k = 0; k < kFluxR; k += 2) {
-                        const float2 mu = __ffma2_rn(ez2[k / 2], rz, __ffma2_rn(ey2[k / 2], ry, __fmul2_rn(ex2[k / 2], rx)));
-                        const float2 c = C.pair(mu, r.w);
-                        if (mu.x > C.thr && !((hid >> k) & 1u)) part[k] += c.x;
-                        if (mu.y > C.thr && !((hid >> (k + 1)) & 1u)) part[k + 1] += c.y;
-                    }
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < kFluxR; ++k) {  // two-sum fold of the 32-element block
-                float s = acc_hi[k] + part[k];
-                float bb = s - acc_hi[k];
-                float err = (acc_hi[k] - (s - bb)) + (part[k] - bb);
+            for (int k = 0; k < kFluxR; ++k) {
+                float& x = (k & 1) ? part[k / 2].y : part[k / 2].x;
+                const float s = acc_hi[k] + x;
+                const float bb = s - acc_hi[k];
+                const float err = (acc_hi[k] - (s - bb)) + (x - bb);
                 acc_hi[k] = s;
                 acc_lo[k] += err;
+                x = 0.f;
+            }
+        };
+        auto mu_pair = [&](int k, const float4& r) {
+            const float2 rx = make_float2(r.x, r.x), ry = make_float2(r.y, r.y), rz = make_float2(r.z, r.z);
+            return __ffma2_rn(ez2[k], rz, __ffma2_rn(ey2[k], ry, __fmul2_rn(ex2[k], rx)));
+        };
+        const int ng = (arc_on >> (2 * quarter)) & 1u ? ngroups : 0;
+        float4 next = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ng > 0 && lane < U.ne) next = __ldg(recs);
+        int pos = 0;  // listed elements of the chunk so far
+        for (int g = 0; g < ng; ++g) {
+            const float4 mine = next;
+            if ((g + 1) * 32 + lane < U.ne) next = __ldg(recs + (g + 1) * 32);
+            const unsigned listed = T.list[g];
+            if (listed) {
+                const unsigned used = T.used[g][quarter], plains = T.plain[g][quarter], mixed = T.mixed[g][quarter];
+                const int total = __popc(listed), room = 32 - (pos & 31);  // to the end of the FP32 block
+                int npair = 0;
+                if (used) {
+                    S.rec[lane] = mine;
+                    if ((mixed >> lane) & 1u) {
+                        const int64_t e = U.e0 + g * 32 + lane;
+                        for (unsigned m = T.gw[e / kEclGroup - g0]; m; m &= m - 1u) {
+                            const double2 p = __ldg(A.el_ecl + (__ffs(m) - 1) * A.sz.nelem + e);
+                            if (p.x <= 2.0) S.pair[npair++][lane] = p;
+                        }
+                    }
+                    __syncwarp();
+                }
+                bool more = total >= room;  // the block ends in this group
+                unsigned low = ~0u;
+                if (more) low = __ballot_sync(0xffffffffu, __popc(listed & ((1u << lane) - 1u)) < room);
+                unsigned m = used & low;
+                for (;;) {
+                    while (m) {
+                        const int i = __ffs(m) - 1;
+                        const float4* q = S.rec + i;
+                        // a run of elements of one kind: plain, limb or mixed
+                        const bool pl = (plains >> i) & 1u, mi = (mixed >> i) & 1u;
+                        const unsigned rest = ~((m & (pl ? plains : mi ? mixed : ~(plains | mixed))) >> i);
+                        const int len = rest ? __ffs(rest) - 1 : 32;
+                        m &= ~((len < 32 ? (1u << len) - 1u : ~0u) << i);
+                        if (KIND != UK_STAR_GENERIC && pl) {
+#pragma unroll kPlainUnroll
+                            for (int n = 0; n < len; ++n) {
+                                const float4 r = q[n];
+#pragma unroll
+                                for (int k = 0; k < kFluxR / 2; ++k)
+                                    part[k] = __fadd2_rn(part[k], C.template pair<true>(mu_pair(k, r), r.w));
+                            }
+                        } else if (KIND != UK_STAR_GENERIC && !mi) {
+#pragma unroll kTestUnroll
+                            for (int n = 0; n < len; ++n) {
+                                const float4 r = q[n];
+#pragma unroll
+                                for (int k = 0; k < kFluxR / 2; ++k) {
+                                    const float2 mu = mu_pair(k, r), c = C.template pair<false>(mu, r.w);
+                                    if (mu.x > C.thr) part[k].x += c.x;
+                                    if (mu.y > C.thr) part[k].y += c.y;
+                                }
+                            }
+                        } else
+#pragma unroll kTestUnroll
+                        for (int n = 0; n < len; ++n) {
+                        const float4 r = q[n];
+                        // sub-phases behind one of the pairs (bit k: sub-phase k)
+                        const int np = __shfl_sync(0xffffffffu, npair, i + n);
+                        const unsigned hid = mi ? hidden_mask(S.pair, np, i + n, S.ph + lane) : 0u;
+                        if (KIND == UK_STAR_GENERIC) {
+                            const float4 p = __ldg(A.el_pos + U.e0 + g * 32 + i + n);
+                            float vx, vy;
+                            if (U.star == 1) { vx = -M.vfacf * spin * p.y; vy = M.vfacf * (spin * p.x - M.xcofmf); }
+                            else { vx = -M.vfacf * spin * p.y; vy = M.vfacf * (spin * (p.x - 1.f) + 1.f - M.xcofmf); }
+                            const float vn = r.x * vx + r.y * vy;
+#pragma unroll
+                            for (int k = 0; k < kFluxR; ++k) {
+                                float& sum = (k & 1) ? part[k / 2].y : part[k / 2].x;
+                                float mu = ex[k] * r.x + ey[k] * r.y + ez[k] * r.z;
+                                bool v = mu > C.thr && !((hid >> k) & 1u);
+                                if (v) {
+                                    float mag = 1.f;
+                                    if (lens) {
+                                        float d = -(p.x * ex[k] + p.y * ey[k] + p.z * ez[k]);
+                                        if (d > 0.f) {
+                                            float ax = p.x + d * ex[k], ay = p.y + d * ey[k], az = p.z + d * ez[k];
+                                            float pp = sqrtf(ax * ax + ay * ay + az * az), phh = pp * 0.5f, phsq = phh * phh;
+                                            float rd = M.rlens1f * d;
+                                            float pd = phsq > 25.f * rd ? pp + rd / pp : phh + sqrtf(phsq + rd);
+                                            mag = pd * pd / (pd - phh) / phh * 0.25f;
+                                        }
+                                    }
+                                    if (beam != 0.f) {
+                                        float vr = -(ex[k] * vx + ey[k] * vy);
+                                        float mud = mu - mu * vr - vn;
+                                        sum += mu * mag * r.w * (1.f - beam * vr) * imu_f(ldg, ltg, mud);
+                                    } else {
+                                        sum += mu * mag * r.w * imu_f(ldg, ltg, mu);
+                                    }
+                                }
+                            }
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < kFluxR; k += 2) {
+                                const float2 mu = mu_pair(k / 2, r), c = C.template pair<false>(mu, r.w);
+                                if (mu.x > C.thr && !((hid >> k) & 1u)) part[k / 2].x += c.x;
+                                if (mu.y > C.thr && !((hid >> (k + 1)) & 1u)) part[k / 2].y += c.y;
+                            }
+                        }
+                        }
+                    }
+                    if (!more) break;
+                    fold();
+                    more = false;
+                    m = used & ~low;
+                }
+                pos += total;
+                __syncwarp();  // the next group rewrites rec and pair
+            }
+            if (((g + 1) & (kFluxChunk / 32 - 1)) == 0 || g + 1 == ng) {  // the chunk's last block
+                fold();
+                pos = 0;
             }
         }
-        __syncthreads();  // everyone is done with buffer b
-        if (tid == 0 && c + 2 < nchunks) issue(c + 2);
-    }
-    // ---- write the partial sums of this (slot, tile)
-    double* out = A.partial + M.pbase + (int64_t)U.slot * M.nsub + U.t0;
 #pragma unroll
-    for (int k = 0; k < kFluxR; ++k) {
-        int j = tid + k * kFluxThreads;
-        if (j < U.nt) out[j] = act[k] ? (double)acc_hi[k] + (double)acc_lo[k] : 0.0;
+        for (int k = 0; k < kFluxR; ++k) {
+            const int j = j0 + 32 * k;
+            if (k < nslot && j < U.nt) out[j] = (act >> k) & 1u ? (double)acc_hi[k] + (double)acc_lo[k] : 0.0;
+        }
+        __syncwarp();  // the next quarter rewrites ph
     }
 }
 
-__global__ void __launch_bounds__(kFluxThreads, 5) k_flux(FluxArgs A) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    FluxSmem& S = *reinterpret_cast<FluxSmem*>(smem_raw);
-    if (threadIdx.x == 0) {
-        mbar_init(&S.bar[0]);
-        mbar_init(&S.bar[1]);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    uint32_t parity[2] = {0u, 0u};
+template <bool kBlock>
+__global__ void __launch_bounds__(kFluxThreads, kFluxMinBlocks) k_flux(FluxArgs A) {
+    __shared__ FluxUnitSmem units[kBlock ? 1 : kFluxWarps];
+    __shared__ FluxWarpSmem warps[kFluxWarps];
+    const int warp = threadIdx.x >> 5;
+    FluxUnitSmem& T = units[kBlock ? 0 : warp];
+    FluxWarpSmem& S = warps[warp];
+    const int q0 = kBlock ? warp : 0, q1 = kBlock ? warp + 1 : kQuarters;
     for (;;) {
-        if (threadIdx.x == 0) S.unit = atomicAdd(A.counter, 1);
-        __syncthreads();
-        const int64_t u = S.unit;
-        __syncthreads();
+        if (kBlock) {
+            __syncthreads();  // the last unit's masks are read
+            if (threadIdx.x == 0) T.unit = atomicAdd(A.counter, 1);
+            __syncthreads();
+        } else {
+            __syncwarp();
+            if ((threadIdx.x & 31) == 0) T.unit = atomicAdd(A.counter, 1);
+            __syncwarp();
+        }
+        const int64_t u = T.unit;
         if (u >= A.nunits) break;
         const FluxUnit U = A.units[u];
         if (!LCB_IN_BOUNDS(U.e0 + U.ne <= A.sz.nelem &&
@@ -1385,18 +1546,19 @@ __global__ void __launch_bounds__(kFluxThreads, 5) k_flux(FluxArgs A) {
                                A.models[U.model].pbase + (int64_t)(U.slot + 1) * A.models[U.model].nsub <=
                                    A.sz.npartial,
                            A.status + U.model))
-            continue;  // the unit is skipped by the whole block
+            continue;  // the unit is skipped by all who share it
+        const unsigned on = flux_sort<kBlock>(A, U, T);
         switch (U.kind) {
-            case UK_STAR_POLY1: flux_unit<UK_STAR_POLY1>(A, U, S, parity); break;
-            case UK_STAR_POLY2: flux_unit<UK_STAR_POLY2>(A, U, S, parity); break;
-            case UK_STAR_POLY3: flux_unit<UK_STAR_POLY3>(A, U, S, parity); break;
-            case UK_STAR_POLY4: flux_unit<UK_STAR_POLY4>(A, U, S, parity); break;
-            case UK_STAR_CLARET: flux_unit<UK_STAR_CLARET>(A, U, S, parity); break;
-            case UK_STAR_GENERIC: flux_unit<UK_STAR_GENERIC>(A, U, S, parity); break;
-            case UK_DISC: flux_unit<UK_DISC>(A, U, S, parity); break;
-            default: flux_unit<UK_SPOT>(A, U, S, parity); break;
+            case UK_STAR_POLY1: flux_unit<UK_STAR_POLY1>(A, U, q0, q1, on, T, S); break;
+            case UK_STAR_POLY2: flux_unit<UK_STAR_POLY2>(A, U, q0, q1, on, T, S); break;
+            case UK_STAR_POLY3: flux_unit<UK_STAR_POLY3>(A, U, q0, q1, on, T, S); break;
+            case UK_STAR_POLY4: flux_unit<UK_STAR_POLY4>(A, U, q0, q1, on, T, S); break;
+            case UK_STAR_CLARET: flux_unit<UK_STAR_CLARET>(A, U, q0, q1, on, T, S); break;
+            case UK_STAR_GENERIC: flux_unit<UK_STAR_GENERIC>(A, U, q0, q1, on, T, S); break;
+            case UK_DISC: flux_unit<UK_DISC>(A, U, q0, q1, on, T, S); break;
+            case UK_DISC_LIN: flux_unit<UK_DISC_LIN>(A, U, q0, q1, on, T, S); break;
+            default: flux_unit<UK_SPOT>(A, U, q0, q1, on, T, S); break;
         }
-        __syncthreads();
     }
 }
 
@@ -1892,21 +2054,11 @@ cudaError_t launch_wait_probe(long long limit, int* status, long long* waited, c
     return cudaGetLastError();
 }
 
-size_t flux_smem_bytes() { return flux_smem_bytes_impl(); }
-
-// The flux kernel's dynamic shared memory exceeds the 48 KB default; the
-// attribute is set once per process (outside any stream capture).
-cudaError_t configure_flux() {
-    static cudaError_t status = cudaFuncSetAttribute(k_flux, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)flux_smem_bytes());
-    return status;
-}
-
 int flux_blocks_per_sm() {
-    if (configure_flux() != cudaSuccess) return 0;
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_flux, kFluxThreads, flux_smem_bytes()) != cudaSuccess) return 0;
-    return n;
+    int n = 0, m = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_flux<false>, kFluxThreads, 0) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m, k_flux<true>, kFluxThreads, 0) != cudaSuccess) return 0;
+    return std::min(n, m);
 }
 
 cudaError_t launch_phase(const PhaseArgs& a, cudaStream_t s) {
@@ -1949,9 +2101,8 @@ int roche_block_size() { return kRocheBlock; }
 
 cudaError_t launch_flux(const FluxArgs& a, int grid, cudaStream_t s) {
     if (a.nunits <= 0) return cudaSuccess;
-    cudaError_t e = configure_flux();
-    if (e != cudaSuccess) return e;
-    k_flux<<<grid, kFluxThreads, flux_smem_bytes(), s>>>(a);
+    if (a.share) k_flux<true><<<grid, kFluxThreads, 0, s>>>(a);
+    else k_flux<false><<<grid, kFluxThreads, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -59,6 +59,7 @@ struct FluxArgs {
     const ModelDev* models;
     const FluxUnit* units;
     int64_t nunits;
+    int share;                 // 1: a block's four warps share a unit, 0: each has its own
     int* counter;
     const float4* el_rec;
     const float4* el_pos;
@@ -96,7 +97,6 @@ struct EpiArgs {
     int* bad;            // LCURVE_DEBUG_BOUNDS: per-model status words the epilogue may set
 };
 
-size_t flux_smem_bytes();
 cudaError_t launch_phase(const PhaseArgs& a, cudaStream_t s);
 cudaError_t launch_elements(const ElemArgs& a, cudaStream_t s);
 cudaError_t launch_roche(const ElemArgs& a, cudaStream_t s);

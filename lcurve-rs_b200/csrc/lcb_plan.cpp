@@ -897,11 +897,15 @@ void plan_batch(const Model* const* models, int64_t n, const lcb_datum* data, co
     int64_t total = 0;
     for (const SegDesc& g : P.segs) total += g.count * lay[g.model].dev.nsub;
     P.evals = total;
-    const int64_t resident = (int64_t)std::max(num_sms, 1) * 4;
-    int64_t per_unit = std::max<int64_t>(total / (resident * 8), 1);
-    int64_t erange = per_unit / kFluxTile;
-    erange = std::min<int64_t>(std::max<int64_t>(erange, kFluxChunk), 16 * kFluxChunk);
-    erange = (erange + kFluxChunk - 1) / kFluxChunk * kFluxChunk;
+    const int64_t sms = std::max(num_sms, 1);
+    auto range = [&](int64_t units) {  // elements per unit for about that many units, whole chunks
+        const int64_t e = std::max<int64_t>(total / units, 1) / kFluxTile;
+        return (std::min<int64_t>(std::max<int64_t>(e, kFluxChunk), 16 * kFluxChunk) + kFluxChunk - 1) / kFluxChunk * kFluxChunk;
+    };
+    // a warp per unit where every resident warp (20 per SM) gets several, else a block per unit
+    int64_t erange = range(sms * 20 * 6);
+    P.flux_share = total / (erange * kFluxTile) < sms * 20 * 4;
+    if (P.flux_share) erange = range(sms * 4 * 8);
     if (tune.flux_chunks > 0) erange = (int64_t)std::min(std::max(tune.flux_chunks, 1), 16) * kFluxChunk;
     P.flux_chunks = (int)(erange / kFluxChunk);
     P.flux_blocks_per_sm = std::max(tune.flux_blocks_per_sm, 0);
@@ -915,7 +919,7 @@ void plan_batch(const Model* const* models, int64_t n, const lcb_datum* data, co
         if (!P.model_ok[i] || D.nsub == 0) { D.nslots = D.g1_end = D.g2_end = D.gd_end = D.ge_end = 0; continue; }
         int32_t slot = 0;
         auto kind_of = [&](const SegDesc& g) {
-            if (g.kind == SEG_DISC || g.kind == SEG_EDGE) return (int32_t)UK_DISC;
+            if (g.kind == SEG_DISC || g.kind == SEG_EDGE) return (int32_t)(D.quad_ldf == 0.f ? UK_DISC_LIN : UK_DISC);
             if (g.kind == SEG_SPOT) return (int32_t)UK_SPOT;
             bool s1 = g.kind == SEG_STAR1;
             bool generic = s1 ? D.beam1 != 0.0 : (D.beam2 != 0.0 || D.glens1);
@@ -1016,7 +1020,7 @@ void plan_batch(const Model* const* models, int64_t n, const lcb_datum* data, co
                    (int64_t)P.rblocks.size(), (int64_t)P.ablocks.size(), (int64_t)P.segs.size(),
                    (int64_t)P.bands.size(), (int64_t)P.rings.size(), (int64_t)P.roche_split, (int64_t)P.split_fix,
                    (int64_t)P.flux_blocks_per_sm, (int64_t)P.curve_blocks, (int64_t)P.result_blocks,
-                   (int64_t)P.curve_share};
+                   (int64_t)P.curve_share, (int64_t)P.flux_share};
 }
 
 }  // namespace lcb

@@ -42,6 +42,7 @@ struct Plan {
     int split_fix = 0;        // PlanTuning::roche_split where it applies: fixed, whatever the list's length
     int flux_chunks = 1;      // elements per flux work unit / kFluxChunk
     int flux_blocks_per_sm = 0;  // persistent flux blocks per SM; 0 = the occupancy limit
+    int flux_share = 1;          // 1: a block's four warps share a flux unit, 0: each warp has its own
     int curve_blocks = 1, result_blocks = 1;  // blocks per model of k_curve and (scaled) k_results
     int curve_share = 0;  // k_curve: 1 = a block's eight warps share one tile of data, 0 = a tile each
 
@@ -60,6 +61,7 @@ struct Plan {
         flux_blocks_per_sm = 0;
         curve_blocks = result_blocks = 1;
         curve_share = 0;
+        flux_share = 1;
     }
 };
 
