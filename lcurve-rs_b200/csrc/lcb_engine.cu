@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -55,11 +56,11 @@ struct DevBuf {
     void* p = nullptr;
     size_t cap = 0;
     void ensure(size_t bytes) {
-        if (bytes <= cap && p) return;
+        if (((bytes + 255) & ~size_t(255)) <= cap && p) return;
         if (p) cudaFree(p);
         p = nullptr;
         cap = 0;
-        size_t want = std::max<size_t>(bytes, 256);
+        const size_t want = (std::max<size_t>(bytes, 1) + 255) & ~size_t(255);  // push() copies whole 256 bytes
         CUDA_TRY(cudaMalloc(&p, want));
         cap = want;
     }
@@ -72,16 +73,61 @@ struct DevBuf {
     T* as() const { return static_cast<T*>(p); }
 };
 
-// All device storage of one planned batch.
+struct View {  // a part of another buffer
+    void* p = nullptr;
+    template <class T>
+    T* as() const { return static_cast<T*>(p); }
+};
+
+// All device storage of one planned batch, parts of one allocation (carve).
 struct DeviceSet {
-    DevBuf models, segs, bands, rings, eblocks, rblocks, ablocks, units, dmodel, dsub0, dsrc, data;
-    DevBuf rec, pos, p64, d64, ecl, egrp, aux, status, spe, spphi, sptype, spw, slfac, partial, calc, results, counter,
-        datum, ecount, fcomp, svda, firsthit, episum, open;
+    DevBuf arena;
+    // the plan's tables, uploaded as one piece
+    View tables, models, segs, bands, rings, eblocks, rblocks, ablocks, units, dsub0;
+    // what a run clears and what it returns, so that one memset and one copy do: [egrp | aux | counter |
+    // status | ecount | results | calc]
+    View work, egrp, aux, counter, status, ecount, results, calc;
+    View datum, rec, pos, p64, d64, ecl, spe, spphi, sptype, spw, slfac, partial, fcomp, svda, firsthit, episum, open;
+    void release() { arena.release(); }
+};
+
+// Page-locked staging of host arrays: two slots used in turn, so that one fills while the other's copy
+// runs.  A slot grows with the transfers that use it, up to kSlotMax.
+struct Staging {
+    static constexpr size_t kSlotMax = 8u << 20;
+    struct Slot {
+        char* p = nullptr;
+        size_t cap = 0;
+        cudaEvent_t done = nullptr;  // its last copy
+        bool busy = false;
+    } slot[2];
+    int next = 0;
+    // a slot of at least `bytes` (<= kSlotMax), its last copy finished
+    Slot& take(size_t bytes) {
+        Slot& s = slot[next];
+        next ^= 1;
+        if (!s.done) CUDA_TRY(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
+        if (s.busy) CUDA_TRY(cudaEventSynchronize(s.done));
+        s.busy = false;
+        if (s.cap < bytes) {
+            const size_t want = std::min(std::max<size_t>(2 * bytes, 64u << 10), kSlotMax);
+            if (s.p) CUDA_TRY(cudaFreeHost(s.p));
+            s.p = nullptr;
+            s.cap = 0;
+            CUDA_TRY(cudaMallocHost((void**)&s.p, want));
+            s.cap = want;
+        }
+        return s;
+    }
     void release() {
-        for (DevBuf* b : {&models, &segs, &bands, &rings, &eblocks, &rblocks, &ablocks, &units, &dmodel, &dsub0, &dsrc,
-                          &data, &rec, &pos, &p64, &d64, &ecl, &egrp, &aux, &status, &spe, &spphi, &sptype, &spw, &slfac,
-                          &partial, &calc, &results, &counter, &datum, &ecount, &fcomp, &svda, &firsthit, &episum, &open})
-            b->release();
+        for (Slot& s : slot) {
+            if (s.done) {
+                if (s.busy) cudaEventSynchronize(s.done);
+                cudaEventDestroy(s.done);
+            }
+            if (s.p) cudaFreeHost(s.p);
+            s = Slot();
+        }
     }
 };
 
@@ -102,7 +148,11 @@ struct lcb_ctx {
     std::string last_error;
     DeviceSet scratch;  // buffers of transient (non-resident) calls
     lcb::Plan plan;     // plan of the last transient call (its buffers are reused)
-    std::vector<lcb_datum> stage;  // host staging of gathered data
+    Staging up, down;              // host -> device and device -> host
+    std::vector<char> fetched;     // the last fetched results
+    int flux_bps = 0;              // k_flux blocks that fit an SM
+    cudaStream_t copy = nullptr;   // large data uploads, beside the kernels that do not need them
+    cudaEvent_t entered = nullptr, copied = nullptr;  // the call's start on `stream`; the copy stream's end
     cudaEvent_t ev[kStages + 1] = {};
     int64_t h2d = 0, d2h = 0;  // bytes moved by the current / last call
     int fblink_cap = lcb::kFblinkEvalCap;  // lcb_ctx_set_search_cap
@@ -132,7 +182,6 @@ struct lcb_batch {
 
 namespace {
 
-// Upload of the plan's tables (and the data) into a device set.
 // Words of the per-group eclipse slot masks (one per kEclGroup elements).
 size_t ecl_groups(const lcb::Plan& P) { return (size_t)((P.nelem + lcb::kEclGroup - 1) / lcb::kEclGroup); }
 
@@ -146,75 +195,155 @@ size_t first_hits(const lcb_ctx* C, const lcb::Plan& P) {
 // Doubles of the epilogue's per-block sums: four per k_curve block, one per k_results block.
 size_t epi_sums(const lcb::Plan& P) { return P.models.size() * (size_t)(4 * P.curve_blocks + P.result_blocks); }
 
-// `prev` (a resident batch's previous plan, its tables already on the device):
-// tables equal to prev's are not uploaded again (a re-parameterised batch of
-// unchanged shape usually changes only the model table and the grid bands).
-void upload_plan(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, const lcb_datum* data, int64_t ndata_src,
-                 bool upload_data, const lcb::Plan* prev = nullptr) {
-    cudaStream_t s = C->stream;
-    auto put = [&](DevBuf& b, const void* src, size_t bytes) {
-        b.ensure(bytes);
-        if (bytes) CUDA_TRY(cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, s));
-        C->h2d += (int64_t)bytes;
-    };
-    // a table equal to the previous plan's is already on the device
-    auto put_new = [&](DevBuf& b, const auto& now, const auto& before) {
-        const size_t bytes = now.size() * sizeof(now[0]);
-        if (prev && b.p && b.cap >= bytes && before.size() == now.size() &&
-            (bytes == 0 || std::memcmp(now.data(), before.data(), bytes) == 0))
-            return;
-        put(b, now.data(), bytes);
-    };
-    const int64_t nm = (int64_t)P.models.size();
-    put(D.models, P.models.data(), nm * sizeof(lcb::ModelDev));
-    const lcb::Plan& Q = prev ? *prev : P;
-    put_new(D.segs, P.segs, Q.segs);
-    put_new(D.bands, P.bands, Q.bands);
-    put_new(D.rings, P.rings, Q.rings);
-    put_new(D.eblocks, P.eblocks, Q.eblocks);
-    put_new(D.rblocks, P.rblocks, Q.rblocks);
-    put_new(D.ablocks, P.ablocks, Q.ablocks);
-    put_new(D.units, P.units, Q.units);
-    put_new(D.dmodel, P.datum_model, Q.datum_model);
-    put_new(D.dsub0, P.datum_sub0, Q.datum_sub0);
-    if (upload_data) {
-        (void)ndata_src;
-        if (P.datum_contiguous && P.ndatum > 0) {
-            // ragged data laid out model after model: one copy straight from the caller's buffer
-            put(D.datum, data + P.datum_src[0], P.ndatum * sizeof(lcb_datum));
-        } else {
-            // expanded (model, datum) records; shared data is gathered on the host once
-            std::vector<lcb_datum>& ex = C->stage;
-            ex.resize(P.ndatum);
-            for (int64_t d = 0; d < P.ndatum; ++d) ex[d] = data[P.datum_src[d]];
-            put(D.datum, ex.data(), ex.size() * sizeof(lcb_datum));
-            // the copy is from pageable memory: it is staged before cudaMemcpyAsync returns
-        }
+size_t pad256(size_t b) { return (b + 255) & ~size_t(255); }
+
+// Host pieces that follow one another in a device range (each padded to 256 bytes).
+struct Piece {
+    const void* src;
+    size_t bytes;
+};
+
+// Copies pieces to dst through the page-locked slots; returns once the host memory has been read.
+void push(lcb_ctx* C, cudaStream_t s, void* dst, const std::vector<Piece>& pieces) {
+    size_t total = 0;
+    for (const Piece& p : pieces) {
+        total += pad256(p.bytes);
+        C->h2d += (int64_t)p.bytes;
     }
-    D.rec.ensure(P.nelem * sizeof(float4));
-    D.pos.ensure(P.nelem * sizeof(float4));
-    D.p64.ensure(P.nelem * sizeof(double4));
-    D.d64.ensure(P.nelem * sizeof(double4));
-    D.ecl.ensure(P.nelem * lcb::kMaxEcl * sizeof(double2));
-    D.egrp.ensure(ecl_groups(P) * sizeof(unsigned));
-    D.aux.ensure(nm * lcb::kNumAux * sizeof(double));
-    D.status.ensure(nm * sizeof(int));
-    D.spe.ensure(P.nsub * sizeof(float4));
-    D.spphi.ensure(P.nsub * sizeof(double));
-    D.sptype.ensure(P.nsub * sizeof(int8_t));
-    D.spw.ensure(P.nsub * sizeof(double));
-    D.slfac.ensure(P.ndatum * sizeof(double));
-    D.partial.ensure(P.npartial * sizeof(double));
-    D.calc.ensure(P.ndatum * sizeof(double));
-    D.results.ensure(nm * 12 * sizeof(double));
-    D.episum.ensure(epi_sums(P) * sizeof(double));
-    D.counter.ensure(sizeof(int) * 4);
-    D.ecount.ensure(sizeof(unsigned long long) * 8);
+    size_t k = 0, in = 0;  // piece, and how much of it is done
+    for (size_t at = 0; at < total;) {
+        const size_t len = std::min(total - at, Staging::kSlotMax);
+        Staging::Slot& slot = C->up.take(len);
+        for (size_t o = 0; o < len;) {
+            const Piece& p = pieces[k];
+            const size_t n = std::min(pad256(p.bytes) - in, len - o);
+            if (in < p.bytes) lcb::host_copy(slot.p + o, (const char*)p.src + in, std::min(n, p.bytes - in));
+            o += n;
+            in += n;
+            if (in == pad256(p.bytes)) {
+                ++k;
+                in = 0;
+            }
+        }
+        CUDA_TRY(cudaMemcpyAsync((char*)dst + at, slot.p, len, cudaMemcpyHostToDevice, s));
+        slot.busy = true;
+        CUDA_TRY(cudaEventRecord(slot.done, s));
+        at += len;
+    }
+}
+
+// The plan's tables in upload order, and their device views.
+std::vector<Piece> plan_tables(const lcb::Plan& P, DeviceSet& D, void* base) {
+    std::vector<Piece> pieces;
+    size_t off = 0;
+    auto add = [&](View& v, const auto& t) {
+        v.p = base ? (char*)base + off : nullptr;
+        pieces.push_back({t.data(), t.size() * sizeof(t[0])});
+        off += pad256(pieces.back().bytes);
+    };
+    add(D.models, P.models);
+    add(D.segs, P.segs);
+    add(D.bands, P.bands);
+    add(D.rings, P.rings);
+    add(D.eblocks, P.eblocks);
+    add(D.rblocks, P.rblocks);
+    add(D.ablocks, P.ablocks);
+    add(D.units, P.units);
+    add(D.dsub0, P.datum_sub0);
+    return pieces;
+}
+
+// Sizes of the work buffer's parts, in its order.
+std::vector<size_t> work_sizes(const lcb::Plan& P) {
+    const size_t nm = P.models.size();
+    return {ecl_groups(P) * sizeof(unsigned), nm * lcb::kNumAux * sizeof(double), sizeof(int) * 4, nm * sizeof(int),
+            sizeof(unsigned long long) * 8, nm * 12 * sizeof(double), P.ndatum * sizeof(double)};
+}
+void work_views(const lcb::Plan& P, DeviceSet& D, void* base) {
+    View* v[7] = {&D.egrp, &D.aux, &D.counter, &D.status, &D.ecount, &D.results, &D.calc};
+    size_t off = 0, k = 0;
+    for (size_t b : work_sizes(P)) {
+        v[k++]->p = base ? (char*)base + off : nullptr;
+        off += pad256(b);
+    }
+}
+size_t total_of(const std::vector<size_t>& v) {
+    size_t t = 0;
+    for (size_t b : v) t += pad256(b);
+    return t;
+}
+
+// Lays out every buffer of a planned batch from `base` on (nullptr only measures).  Returns the bytes
+// used; `counted`, if given, those that lcb_light_curve_noalloc's limit counts.
+size_t carve(const lcb_ctx* C, const lcb::Plan& P, void* base, DeviceSet& D, size_t* counted = nullptr) {
+    size_t off = 0;
+    auto take = [&](View& v, size_t bytes) {
+        v.p = base ? (char*)base + off : nullptr;
+        off += pad256(bytes);
+    };
+    size_t tables = 0;
+    for (const Piece& p : plan_tables(P, D, nullptr)) tables += pad256(p.bytes);
+    take(D.tables, tables);
+    plan_tables(P, D, D.tables.p);
+    take(D.work, total_of(work_sizes(P)));
+    work_views(P, D, D.work.p);
+    take(D.datum, P.data_count * sizeof(lcb_datum));
+    take(D.rec, P.nelem * sizeof(float4));
+    take(D.pos, P.nelem * sizeof(float4));
+    take(D.p64, P.nelem * sizeof(double4));
+    take(D.d64, P.nelem * sizeof(double4));
+    take(D.ecl, P.nelem * lcb::kMaxEcl * sizeof(double2));
+    take(D.spe, P.nsub * sizeof(float4));
+    take(D.spphi, P.nsub * sizeof(double));
+    take(D.sptype, P.nsub * sizeof(int8_t));
+    take(D.spw, P.nsub * sizeof(double));
+    take(D.slfac, P.ndatum * sizeof(double));
+    take(D.partial, P.npartial * sizeof(double));
     const size_t ncomp = P.any_iscale ? (size_t)P.ndatum * 5 : 1;
-    D.fcomp.ensure(ncomp * sizeof(double));
-    D.svda.ensure(ncomp * sizeof(double));
-    D.open.ensure(std::max<size_t>(P.rblocks.size() * lcb::kRocheBlock, 1) * sizeof(unsigned));
-    D.firsthit.ensure(first_hits(C, P) * sizeof(int));
+    take(D.fcomp, ncomp * sizeof(double));
+    take(D.svda, ncomp * sizeof(double));
+    // the above and four bytes per Roche thread of a split search
+    if (counted) *counted = off + pad256((P.roche_split > 1 ? P.rblocks.size() * lcb::kRocheBlock : 1) * sizeof(int));
+    take(D.firsthit, first_hits(C, P) * sizeof(int));
+    take(D.open, std::max<size_t>(P.rblocks.size() * lcb::kRocheBlock, 1) * sizeof(unsigned));
+    take(D.episum, epi_sums(P) * sizeof(double));
+    return off;
+}
+
+// Device arrays and tables of a plan (not the data).
+void upload_plan(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P) {
+    D.arena.ensure(carve(C, P, nullptr, D));
+    carve(C, P, D.arena.p, D);
+    push(C, C->stream, D.tables.p, plan_tables(P, D, D.tables.p));
+}
+
+// The data of a plan, on the context's stream; large ones on the copy stream, which `joined` (the
+// caller, before the first kernel that reads them) makes the context's stream wait for.
+constexpr size_t kCopyBeside = 1u << 20;
+void upload_data(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, const lcb_datum* data, bool beside = false) {
+    const lcb_datum* src = data + P.data_first;
+    const size_t bytes = P.data_count * sizeof(lcb_datum);
+    if (!bytes) return;
+    const bool other = beside && bytes >= kCopyBeside;
+    cudaStream_t s = C->stream;
+    if (other) {
+        if (!C->copy) CUDA_TRY(cudaStreamCreateWithFlags(&C->copy, cudaStreamNonBlocking));
+        if (!C->copied) CUDA_TRY(cudaEventCreateWithFlags(&C->copied, cudaEventDisableTiming));
+        s = C->copy;
+        CUDA_TRY(cudaStreamWaitEvent(s, C->entered, 0));  // whatever an earlier call left on the stream is done
+    }
+    cudaPointerAttributes at{};
+    if (bytes >= kCopyBeside && cudaPointerGetAttributes(&at, src) == cudaSuccess && at.type == cudaMemoryTypeHost) {
+        CUDA_TRY(cudaMemcpyAsync(D.datum.p, src, bytes, cudaMemcpyHostToDevice, s));  // page-locked already
+        C->h2d += (int64_t)bytes;
+    } else {
+        (void)cudaGetLastError();
+        push(C, s, D.datum.p, {{src, bytes}});
+    }
+    if (other) {
+        CUDA_TRY(cudaEventRecord(C->copied, s));
+        CUDA_TRY(cudaStreamWaitEvent(C->stream, C->copied, 0));
+    }
 }
 
 // Parts of the launch sequence: the element stage (grids, continuum, eclipses:
@@ -223,25 +352,22 @@ constexpr int kStageElements = 1, kStageRest = 2, kStagesAll = 3;
 
 // The device launch sequence of one batch evaluation.  nblk / nrblk (>= 0)
 // launch only the first nblk element blocks and nrblk Roche blocks of the
-// uploaded block lists (an element slab, lcb_model_elements).
+// uploaded block lists (an element slab, lcb_model_elements).  `data` runs
+// before the first kernel that reads the data (k_phase).
 void enqueue_run(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, int scale, int rdata, bool timed,
-                 int stages = kStagesAll, int64_t nblk = -1, int64_t nrblk = -1) {
+                 int stages = kStagesAll, int64_t nblk = -1, int64_t nrblk = -1,
+                 const std::function<void()>& data = nullptr) {
     cudaStream_t s = C->stream;
     const int64_t nm = (int64_t)P.models.size();
     if (nblk < 0) nblk = (int64_t)P.eblocks.size();
     if (nrblk < 0) nrblk = (int64_t)P.rblocks.size();
-    CUDA_TRY(cudaMemsetAsync(D.aux.p, 0, nm * lcb::kNumAux * sizeof(double), s));
-    CUDA_TRY(cudaMemsetAsync(D.status.p, 0, nm * sizeof(int), s));
-    CUDA_TRY(cudaMemsetAsync(D.counter.p, 0, sizeof(int) * 4, s));
-    CUDA_TRY(cudaMemsetAsync(D.ecount.p, 0, sizeof(unsigned long long) * 8, s));
-    if (timed) CUDA_TRY(cudaEventRecord(C->ev[0], s));
     const bool rest = stages & kStageRest, elem = stages & kStageElements;
-    const lcb::Sizes sz{P.nelem, P.nsub, P.npartial, P.ndatum, (int64_t)P.bands.size(), (int64_t)P.rings.size()};
-    lcb::PhaseArgs pa{D.models.as<lcb::ModelDev>(), D.datum.as<lcb_datum>(), D.dmodel.as<int32_t>(),
-                      D.dsub0.as<int64_t>(), P.ndatum, D.spe.as<float4>(), D.spphi.as<double>(),
-                      D.sptype.as<int8_t>(), D.spw.as<double>(), D.slfac.as<double>()};
-    if (rest) CUDA_TRY(lcb::launch_phase(pa, s));
-    if (timed) CUDA_TRY(cudaEventRecord(C->ev[1], s));
+    {   // used-slot words (element stage), sums, counters and status words
+        void* from = elem ? D.egrp.p : D.aux.p;
+        CUDA_TRY(cudaMemsetAsync(from, 0, (char*)D.results.p - (char*)from, s));
+    }
+    if (timed) CUDA_TRY(cudaEventRecord(C->ev[0], s));
+    const lcb::Sizes sz{P.nelem, P.nsub, P.npartial, P.ndatum, (int64_t)P.bands.size(), (int64_t)P.rings.size(), P.data_count};
     lcb::ElemArgs ea{D.models.as<lcb::ModelDev>(), D.segs.as<lcb::SegDesc>(), D.eblocks.as<lcb::ElemBlock>(),
                      D.rblocks.as<lcb::ElemBlock>(), D.ablocks.as<lcb::ElemBlock>(), D.bands.as<lcb::Band>(),
                      D.rings.as<lcb::Ring>(), D.rec.as<float4>(), D.pos.as<float4>(), D.p64.as<double4>(),
@@ -250,21 +376,24 @@ void enqueue_run(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, int scale, int rd
                      D.ecount.as<unsigned long long>(), D.open.as<unsigned>(), D.counter.as<unsigned>() + 1,
                      D.firsthit.as<int>(), (unsigned)first_hits(C, P), P.split_fix, lcb::split_target(C->num_sms),
                      C->num_sms * 5, C->fblink_cap, sz};
-    if (elem) {
-        CUDA_TRY(cudaMemsetAsync(D.egrp.p, 0, ecl_groups(P) * sizeof(unsigned), s));
-        CUDA_TRY(lcb::launch_elements(ea, s));
-    }
-    if (timed) CUDA_TRY(cudaEventRecord(C->ev[2], s));
+    if (elem) CUDA_TRY(lcb::launch_elements(ea, s));
+    if (timed) CUDA_TRY(cudaEventRecord(C->ev[1], s));
     if (elem) CUDA_TRY(lcb::launch_roche(ea, s));
-    if (timed) CUDA_TRY(cudaEventRecord(C->ev[3], s));
+    if (timed) CUDA_TRY(cudaEventRecord(C->ev[2], s));
     if (!rest) return;
     CUDA_TRY(lcb::launch_aux(ea, s));
+    if (timed) CUDA_TRY(cudaEventRecord(C->ev[3], s));
+    if (data) data();
+    lcb::PhaseArgs pa{D.models.as<lcb::ModelDev>(), D.datum.as<lcb_datum>(), D.dsub0.as<int64_t>(), nm, P.most_data,
+                      D.spe.as<float4>(), D.spphi.as<double>(), D.sptype.as<int8_t>(), D.spw.as<double>(),
+                      D.slfac.as<double>()};
+    CUDA_TRY(lcb::launch_phase(pa, s));
     if (timed) CUDA_TRY(cudaEventRecord(C->ev[4], s));
     lcb::FluxArgs fa{D.models.as<lcb::ModelDev>(), D.units.as<lcb::FluxUnit>(), (int64_t)P.units.size(),
                      P.flux_share, D.counter.as<int>(), D.rec.as<float4>(), D.pos.as<float4>(), D.ecl.as<double2>(),
                      D.egrp.as<unsigned>(), D.spe.as<float4>(), D.spphi.as<double>(), D.sptype.as<int8_t>(), D.partial.as<double>(),
                      D.status.as<int>(), sz};
-    const int bps_max = lcb::flux_blocks_per_sm();
+    const int bps_max = C->flux_bps;
     const int bps = P.flux_blocks_per_sm > 0 ? std::min(P.flux_blocks_per_sm, bps_max) : bps_max;
     int64_t grid = (int64_t)C->num_sms * bps;
     grid = std::min<int64_t>(grid, std::max<int64_t>((int64_t)P.units.size(), 1));
@@ -279,27 +408,59 @@ void enqueue_run(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, int scale, int rd
     CUDA_TRY(lcb::launch_epilogue(pe, s));
     if (timed) CUDA_TRY(cudaEventRecord(C->ev[6], s));
 }
+// the order of the timed stages above in the reported one (phase, elements, roche, aux, flux, epilogue)
+constexpr int kStageOrder[kStages] = {1, 2, 3, 0, 4, 5};
 
 void set_device(lcb_ctx* C) { CUDA_TRY(cudaSetDevice(C->device)); }
 
+// Copies a device range into dst through the page-locked slots (synchronises).
+void pull(lcb_ctx* C, void* dst, const void* src, size_t bytes) {
+    struct { Staging::Slot* s; size_t at, len; } open[2] = {};
+    int n = 0;
+    auto drain = [&](int k) {
+        CUDA_TRY(cudaEventSynchronize(open[k].s->done));
+        open[k].s->busy = false;
+        lcb::host_copy((char*)dst + open[k].at, open[k].s->p, open[k].len);
+        open[k].s = nullptr;
+    };
+    for (size_t at = 0; at < bytes; n ^= 1) {
+        if (open[n].s) drain(n);
+        const size_t len = std::min(bytes - at, Staging::kSlotMax);
+        Staging::Slot& s = C->down.take(len);
+        CUDA_TRY(cudaMemcpyAsync(s.p, (const char*)src + at, len, cudaMemcpyDeviceToHost, C->stream));
+        s.busy = true;
+        CUDA_TRY(cudaEventRecord(s.done, C->stream));
+        open[n] = {&s, at, len};
+        at += len;
+    }
+    for (int k = 0; k < 2; ++k, n ^= 1)
+        if (open[n].s) drain(n);
+    C->d2h += (int64_t)bytes;
+}
+
+// The status words, search counters and results of a run, and with `calc` its fluxes: one copy.
 void fetch_results(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, std::vector<double>& res, std::vector<double>* calc,
                    std::vector<int>* status, unsigned long long* ecount = nullptr) {
     const int64_t nm = (int64_t)P.models.size();
+    const char* base = (const char*)D.status.p;
+    const size_t head = (const char*)D.calc.p - base, tail = calc ? P.ndatum * sizeof(double) : 0;
+    std::vector<char>& h = C->fetched;
+    const bool one = head + tail <= Staging::kSlotMax;  // else the fluxes straight into their vector
+    h.resize(head + (one ? tail : 0));
+    pull(C, h.data(), base, h.size());
+    auto part = [&](const View& v) { return h.data() + ((const char*)v.p - base); };
     res.resize(nm * 12);
-    CUDA_TRY(cudaMemcpyAsync(res.data(), D.results.p, nm * 12 * sizeof(double), cudaMemcpyDeviceToHost, C->stream));
-    if (calc) {
-        calc->resize(P.ndatum);
-        if (P.ndatum)
-            CUDA_TRY(cudaMemcpyAsync(calc->data(), D.calc.p, P.ndatum * sizeof(double), cudaMemcpyDeviceToHost, C->stream));
-    }
+    std::memcpy(res.data(), part(D.results), nm * 12 * sizeof(double));
     if (status) {
         status->resize(nm);
-        CUDA_TRY(cudaMemcpyAsync(status->data(), D.status.p, nm * sizeof(int), cudaMemcpyDeviceToHost, C->stream));
+        std::memcpy(status->data(), part(D.status), nm * sizeof(int));
     }
-    if (ecount)  // the eclipse-search counters (5)
-        CUDA_TRY(cudaMemcpyAsync(ecount, D.ecount.p, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, C->stream));
-    C->d2h += (int64_t)(nm * 12 * sizeof(double)) + (calc ? P.ndatum * (int64_t)sizeof(double) : 0) +
-              (status ? nm * (int64_t)sizeof(int) : 0);
+    if (ecount) std::memcpy(ecount, part(D.ecount), 5 * sizeof(unsigned long long));
+    if (calc) {
+        calc->resize(P.ndatum);
+        if (one) std::memcpy(calc->data(), part(D.calc), tail);
+        else pull(C, calc->data(), D.calc.p, tail);
+    }
     CUDA_TRY(cudaStreamSynchronize(C->stream));
 }
 
@@ -317,21 +478,33 @@ void fill_result(const double* r, lcb_result* out) {
 }
 
 
+// The engine's plans carry no per-datum tables where a model's data are sub-divided alike.
+lcb::PlanTuning engine_tuning() {
+    lcb::PlanTuning t;
+    t.datum_tables = false;
+    return t;
+}
+
 // A transient evaluation on the context's scratch buffers.
 void run_transient(lcb_ctx* C, const lcb::Model* const* models, int64_t n, const lcb_datum* data,
                    const int64_t* start, const int64_t* count, int scale, int rdata, std::vector<double>& res,
                    std::vector<double>* calc, lcb::Plan& P, std::vector<int>& st) {
     {
         Range r("lcb plan");
-        lcb::plan_batch(models, n, data, start, count, C->num_sms, P);
+        lcb::plan_batch(models, n, data, start, count, C->num_sms, P, engine_tuning());
     }
     {
         Range r("lcb upload");
-        upload_plan(C, C->scratch, P, data, 0, true);
+        upload_plan(C, C->scratch, P);
+        if (P.data_count * sizeof(lcb_datum) >= kCopyBeside) {
+            if (!C->entered) CUDA_TRY(cudaEventCreateWithFlags(&C->entered, cudaEventDisableTiming));
+            CUDA_TRY(cudaEventRecord(C->entered, C->stream));
+        }
     }
     {
-        Range r("lcb launch");
-        enqueue_run(C, C->scratch, P, scale, rdata, false);
+        Range r("lcb launch");  // the data follow while the kernels that do not need them run
+        enqueue_run(C, C->scratch, P, scale, rdata, false, kStagesAll, -1, -1,
+                    [&] { upload_data(C, C->scratch, P, data, true); });
     }
     {
         Range r("lcb results");
@@ -400,7 +573,8 @@ int lcb_ctx_create(int device, lcb_ctx** out) {
         if (prop.major < 10) throw Error(LCB_ERR_NO_DEVICE, "this library is built for sm_100a (B200)");
         C->num_sms = prop.multiProcessorCount;
         // fails here, not later, if the sm_100a image cannot load on this device
-        if (lcb::flux_blocks_per_sm() <= 0) throw Error(LCB_ERR_NO_DEVICE, "kernel image not loadable");
+        C->flux_bps = lcb::flux_blocks_per_sm();
+        if (C->flux_bps <= 0) throw Error(LCB_ERR_NO_DEVICE, "kernel image not loadable");
         CUDA_TRY(cudaStreamCreateWithFlags(&C->stream, cudaStreamNonBlocking));
         C->own_stream = true;
         for (auto& e : C->ev) CUDA_TRY(cudaEventCreate(&e));
@@ -414,8 +588,14 @@ void lcb_ctx_destroy(lcb_ctx* C) {
     if (!C) return;
     cudaSetDevice(C->device);
     if (C->stream) cudaStreamSynchronize(C->stream);
+    if (C->copy) cudaStreamSynchronize(C->copy);
     C->scratch.release();
     C->probe.release();
+    C->up.release();
+    C->down.release();
+    if (C->entered) cudaEventDestroy(C->entered);
+    if (C->copied) cudaEventDestroy(C->copied);
+    if (C->copy) cudaStreamDestroy(C->copy);
     for (auto& e : C->ev)
         if (e) cudaEventDestroy(e);
     if (C->own_stream && C->stream) cudaStreamDestroy(C->stream);
@@ -565,7 +745,8 @@ int lcb_model_grid(lcb_ctx* C, const lcb_model* model, int which, int64_t* n, do
         }
         *n = g ? g->count : 0;
         if (!g || !posn) return;
-        upload_plan(C, C->scratch, P, &d, 1, true);
+        upload_plan(C, C->scratch, P);
+        upload_data(C, C->scratch, P, &d);
         enqueue_run(C, C->scratch, P, 0, 0, false);
         CUDA_TRY(cudaStreamSynchronize(C->stream));
         std::vector<double4> p64(g->count), d64(g->count);
@@ -628,7 +809,7 @@ int lcb_model_elements(lcb_ctx* C, const lcb_model* model, int64_t first, int64_
             if (touches(b, lcb::kElemThreads)) eb.push_back(b);
         for (const auto& b : P.rblocks)
             if (touches(b, lcb::kRocheBlock)) rb.push_back(b);
-        upload_plan(C, C->scratch, P, &d, 1, true);
+        upload_plan(C, C->scratch, P);
         DeviceSet& D = C->scratch;
         if (!eb.empty())
             CUDA_TRY(cudaMemcpyAsync(D.eblocks.p, eb.data(), eb.size() * sizeof(lcb::ElemBlock),
@@ -664,7 +845,8 @@ int lcb_light_curve_elements(lcb_ctx* C, const lcb_model* model, const lcb_datum
         lcb::Plan& P = C->plan;
         lcb::plan_batch(&mp, 1, data, &st, &cnt, C->num_sms, P);
         if (!P.model_ok[0]) throw Error(LCB_ERR_MODEL, P.model_err[0]);
-        upload_plan(C, C->scratch, P, data, 0, true);
+        upload_plan(C, C->scratch, P);
+        upload_data(C, C->scratch, P, data);
         DeviceSet& D = C->scratch;
         const void* src[4] = {rec_dev, pos_dev, p64_dev, d64_dev};
         void* dst[4] = {D.rec.p, D.pos.p, D.p64.p, D.d64.p};
@@ -741,7 +923,7 @@ int lcb_chisq_batch_ragged(lcb_ctx* C, const lcb_model* const* models, int64_t n
             }
         }
         if (calc_out)
-            for (int64_t d = 0; d < P.ndatum; ++d) calc_out[offsets[0] + d] = calc[d];
+            lcb::host_copy(calc_out + offsets[0], calc.data(), P.ndatum * sizeof(double));
     });
 }
 
@@ -766,9 +948,11 @@ int lcb_batch_create(lcb_ctx* C, const lcb_model* const* models, int64_t nmodels
         }
         std::vector<const lcb::Model*> mp(nmodels);
         for (int64_t i = 0; i < nmodels; ++i) mp[i] = &B->models[i];
+        B->tune = engine_tuning();
         lcb::plan_batch(mp.data(), nmodels, B->data.data(), B->start.data(), B->count.data(), C->num_sms, B->plan,
                         B->tune);
-        upload_plan(C, B->dev, B->plan, B->data.data(), (int64_t)B->data.size(), true);
+        upload_plan(C, B->dev, B->plan);
+        upload_data(C, B->dev, B->plan, B->data.data());
         CUDA_TRY(cudaStreamSynchronize(C->stream));
     });
     if (rc != LCB_OK) {
@@ -794,24 +978,30 @@ void lcb_batch_destroy(lcb_batch* B) {
 // If the uploads fail part-way (a buffer could not grow), the device buffers no longer
 // match the plan: the batch is marked broken, its graph dropped and its shape key
 // cleared, so no launch runs on it until a later re-plan uploads everything again.
-static void replan_batch(lcb_batch* B) {
+static void replan_batch(lcb_batch* B, bool params_only) {
     lcb_ctx* C = B->ctx;
     const int64_t n = (int64_t)B->models.size();
     std::vector<const lcb::Model*> mp(n);
     for (int64_t i = 0; i < n; ++i) mp[i] = &B->models[i];
-    lcb::Plan& P = B->spare;
     Range r("lcb replan");
+    // parameters that change no table (a sampler's, mostly) change the model table alone
+    if (params_only && !B->broken &&
+        lcb::replan_models(mp.data(), n, B->data.data(), B->start.data(), B->count.data(), B->plan)) {
+        push(C, C->stream, B->dev.models.p, {{B->plan.models.data(), n * sizeof(lcb::ModelDev)}});
+        return;
+    }
+    lcb::Plan& P = B->spare;
     lcb::plan_batch(mp.data(), n, B->data.data(), B->start.data(), B->count.data(), C->num_sms, P, B->tune);
     const bool same = !B->broken && P.shape_key == B->plan.shape_key;
     std::swap(B->plan, P);
     try {
-        upload_plan(C, B->dev, B->plan, B->data.data(), (int64_t)B->data.size(), !same, same ? &P : nullptr);
+        upload_plan(C, B->dev, B->plan);
+        if (!same) upload_data(C, B->dev, B->plan, B->data.data());
         if (!same && B->graph) {
             cudaGraphExecDestroy(B->graph);
             B->graph = nullptr;
         }
-        // copies from pageable host memory are staged before cudaMemcpyAsync returns, so the
-        // plan's host tables may change at once; a new shape waits for its uploads here
+        // a new shape waits for its uploads here
         if (!same) CUDA_TRY(cudaStreamSynchronize(C->stream));
     } catch (...) {
         cudaStreamSynchronize(C->stream);
@@ -839,7 +1029,7 @@ int lcb_batch_set_tuning(lcb_batch* B, int flux_chunks, int roche_split, int flu
         B->tune.flux_chunks = flux_chunks;
         B->tune.roche_split = roche_split;
         B->tune.flux_blocks_per_sm = flux_blocks_per_sm;
-        replan_batch(B);
+        replan_batch(B, false);
     });
 }
 
@@ -847,7 +1037,7 @@ int lcb_batch_get_tuning(const lcb_batch* B, int* out3) {
     if (!B || !out3) return fail(LCB_ERR_INVALID, "null pointer");
     return guarded(B->ctx, [&] {
         const lcb::Plan& P = B->plan;
-        const int bps_max = lcb::flux_blocks_per_sm();
+        const int bps_max = B->ctx->flux_bps;
         out3[0] = P.flux_chunks;
         out3[1] = P.roche_split;
         out3[2] = P.flux_blocks_per_sm > 0 ? std::min(P.flux_blocks_per_sm, bps_max) : bps_max;
@@ -866,8 +1056,8 @@ int lcb_batch_set_params(lcb_batch* B, const char* const* names, int ndim, const
         }
         // planned into the previous call's storage (kept capacity: no allocation or first-touch
         // page faults when a resident batch is re-parameterised step after step); with unchanged
-        // shapes only the model table and the tables derived from it are uploaded
-        replan_batch(B);
+        // tables only the model table is uploaded
+        replan_batch(B, true);
     });
 }
 
@@ -881,8 +1071,6 @@ int lcb_batch_run(lcb_batch* B, int scale) {
             B->graph = nullptr;
         }
         if (!B->graph) {
-            // the flux kernel's shared-memory attribute must be set outside capture
-            lcb::flux_blocks_per_sm();
             cudaGraph_t g;
             CUDA_TRY(cudaStreamBeginCapture(C->stream, cudaStreamCaptureModeThreadLocal));
             try {
@@ -914,12 +1102,11 @@ int lcb_batch_profile(lcb_batch* B, int scale) {
     return guarded(C, [&] {
         check_usable(B);
         enqueue_run(C, B->dev, B->plan, scale, 1, true);
-        fetch_results(C, B->dev, B->plan, B->h_results, nullptr, &B->h_status);
-        CUDA_TRY(cudaMemcpy(B->ecount, B->dev.ecount.p, sizeof(B->ecount), cudaMemcpyDeviceToHost));
+        fetch_results(C, B->dev, B->plan, B->h_results, nullptr, &B->h_status, B->ecount);
         for (int k = 0; k < kStages; ++k) {
             float ms = 0.f;
             CUDA_TRY(cudaEventElapsedTime(&ms, C->ev[k], C->ev[k + 1]));
-            B->stage_ms[k] = ms;
+            B->stage_ms[kStageOrder[k]] = ms;
         }
         B->ran = true;
         for (int s : B->h_status)
@@ -1124,76 +1311,18 @@ unsigned char* noalloc_arena() {
     return static_cast<unsigned char*>(p);
 }
 
-// Lays out every buffer of a planned single-model evaluation inside the arena
-// (base == nullptr only measures).  Returns the bytes used.
-size_t noalloc_carve(const lcb_ctx* C, const lcb::Plan& P, unsigned char* base, DeviceSet& D, size_t* total = nullptr) {
-    size_t off = 0;
-    auto take = [&](DevBuf& b, size_t bytes) {
-        b.p = base ? base + off : nullptr;
-        b.cap = bytes;
-        off += (bytes + 255) & ~size_t(255);
-    };
-    const size_t nm = P.models.size();
-    take(D.models, nm * sizeof(lcb::ModelDev));
-    take(D.segs, P.segs.size() * sizeof(lcb::SegDesc));
-    take(D.bands, P.bands.size() * sizeof(lcb::Band));
-    take(D.rings, P.rings.size() * sizeof(lcb::Ring));
-    take(D.eblocks, P.eblocks.size() * sizeof(lcb::ElemBlock));
-    take(D.rblocks, P.rblocks.size() * sizeof(lcb::ElemBlock));
-    take(D.ablocks, P.ablocks.size() * sizeof(lcb::ElemBlock));
-    take(D.units, P.units.size() * sizeof(lcb::FluxUnit));
-    take(D.dmodel, P.datum_model.size() * sizeof(int32_t));
-    take(D.dsub0, P.datum_sub0.size() * sizeof(int64_t));
-    take(D.datum, P.ndatum * sizeof(lcb_datum));
-    take(D.rec, P.nelem * sizeof(float4));
-    take(D.pos, P.nelem * sizeof(float4));
-    take(D.p64, P.nelem * sizeof(double4));
-    take(D.d64, P.nelem * sizeof(double4));
-    take(D.ecl, P.nelem * lcb::kMaxEcl * sizeof(double2));
-    take(D.egrp, ecl_groups(P) * sizeof(unsigned));
-    take(D.aux, nm * lcb::kNumAux * sizeof(double));
-    take(D.status, nm * sizeof(int));
-    take(D.spe, P.nsub * sizeof(float4));
-    take(D.spphi, P.nsub * sizeof(double));
-    take(D.sptype, P.nsub * sizeof(int8_t));
-    take(D.spw, P.nsub * sizeof(double));
-    take(D.slfac, P.ndatum * sizeof(double));
-    take(D.partial, P.npartial * sizeof(double));
-    take(D.calc, P.ndatum * sizeof(double));
-    take(D.results, nm * 12 * sizeof(double));
-    take(D.counter, sizeof(int) * 4);
-    take(D.ecount, sizeof(unsigned long long) * 8);
-    const size_t ncomp = P.any_iscale ? (size_t)P.ndatum * 5 : 1;
-    take(D.fcomp, ncomp * sizeof(double));
-    take(D.svda, ncomp * sizeof(double));
-    // what LCB_NOALLOC_ARENA_BYTES limits: the above and four bytes per Roche thread of a split search
-    const size_t counted = off + (((P.roche_split > 1 ? P.rblocks.size() * lcb::kRocheBlock : 1) * sizeof(int) + 255) & ~size_t(255));
-    take(D.firsthit, first_hits(C, P) * sizeof(int));
-    take(D.open, std::max<size_t>(P.rblocks.size() * lcb::kRocheBlock, 1) * sizeof(unsigned));
-    take(D.episum, epi_sums(P) * sizeof(double));
-    if (total) *total = off;
-    return counted;
-}
-
 // Host -> arena copies of the plan's tables and the data (no allocation).
 void noalloc_upload(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, const lcb_datum* data) {
-    auto put = [&](DevBuf& b, const void* src, size_t bytes) {
-        if (bytes) CUDA_TRY(cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, C->stream));
+    auto put = [&](void* dst, const void* src, size_t bytes) {
+        if (bytes) CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, C->stream));
         C->h2d += (int64_t)bytes;
     };
-    put(D.models, P.models.data(), P.models.size() * sizeof(lcb::ModelDev));
-    put(D.segs, P.segs.data(), P.segs.size() * sizeof(lcb::SegDesc));
-    put(D.bands, P.bands.data(), P.bands.size() * sizeof(lcb::Band));
-    put(D.rings, P.rings.data(), P.rings.size() * sizeof(lcb::Ring));
-    put(D.eblocks, P.eblocks.data(), P.eblocks.size() * sizeof(lcb::ElemBlock));
-    put(D.rblocks, P.rblocks.data(), P.rblocks.size() * sizeof(lcb::ElemBlock));
-    put(D.ablocks, P.ablocks.data(), P.ablocks.size() * sizeof(lcb::ElemBlock));
-    put(D.units, P.units.data(), P.units.size() * sizeof(lcb::FluxUnit));
-    put(D.dmodel, P.datum_model.data(), P.datum_model.size() * sizeof(int32_t));
-    put(D.dsub0, P.datum_sub0.data(), P.datum_sub0.size() * sizeof(int64_t));
-    std::vector<lcb_datum> ex(P.ndatum);
-    for (int64_t d = 0; d < P.ndatum; ++d) ex[d] = data[P.datum_src[d]];
-    put(D.datum, ex.data(), ex.size() * sizeof(lcb_datum));
+    size_t off = 0;
+    for (const Piece& p : plan_tables(P, D, D.tables.p)) {
+        put((char*)D.tables.p + off, p.src, p.bytes);
+        off += pad256(p.bytes);
+    }
+    put(D.datum.p, data + P.data_first, P.data_count * sizeof(lcb_datum));
 }
 
 }  // namespace
@@ -1210,16 +1339,16 @@ extern "C" int lcb_light_curve_noalloc(lcb_ctx* C, const lcb_model* model, const
         lcb::Plan P;
         lcb::plan_batch(&mp, 1, data, &st, &cnt, C->num_sms, P);
         if (!P.model_ok[0]) throw Error(LCB_ERR_MODEL, P.model_err[0]);
-        DeviceSet D;  // views into the arena: never ensure()d or released
-        size_t total = 0;
-        const size_t need = noalloc_carve(C, P, nullptr, D, &total);
+        DeviceSet D;  // views into the static arena: its own is never allocated
+        size_t need = 0;
+        const size_t total = carve(C, P, nullptr, D, &need);
         if (need > (size_t)LCB_NOALLOC_ARENA_BYTES || total > kNoallocArena)
             throw Error(LCB_ERR_INVALID, "lcb_light_curve_noalloc: this model and data need " + std::to_string(need) +
                                              " bytes of device scratch, more than the fixed arena's " +
                                              std::to_string((size_t)LCB_NOALLOC_ARENA_BYTES) +
                                              "; use lcb_light_curve (or coarser grids / fewer points)");
         std::lock_guard<std::mutex> lock(g_noalloc_mu[C->device]);
-        noalloc_carve(C, P, noalloc_arena(), D);
+        carve(C, P, noalloc_arena(), D);
         std::vector<double> res, calc;
         std::vector<int> status;
         try {

@@ -104,11 +104,21 @@ struct ModelDev {
     double glogg1, glogg2;      // gref * gscale terms of comp_gravity1/2
     // ---- layout
     int64_t sub_begin, nsub;        // sub-phases
-    int64_t datum_begin, ndatum;    // data
+    int64_t datum_begin, ndatum;    // per (model, datum) results
+    int64_t data_begin;             // its first record in the uploaded data (models may share records)
+    int64_t ndiv;                   // sub-divisions of every datum alike; 0: as datum_sub0 says
     int64_t pbase;                  // partial buffer offset
     int32_t nslots, g1_end, g2_end, status;  // slots: [0,g1_end) star1, [g1_end,g2_end) star2, rest
     int32_t gd_end, ge_end;                  // rest: [g2_end,gd_end) disc, [gd_end,ge_end) rim, [ge_end,nslots) spot
 };
+
+// First sub-phase of a model's datum d (sub0: the table of irregular models).
+#if defined(__CUDACC__)
+__host__ __device__
+#endif
+inline int64_t first_sub(const ModelDev& M, const int64_t* sub0, int64_t d) {
+    return M.ndiv > 0 ? M.sub_begin + d * M.ndiv : sub0[M.datum_begin + d];
+}
 
 struct SegDesc {            // a contiguous run of elements of one model and kind
     int64_t first;          // global element index

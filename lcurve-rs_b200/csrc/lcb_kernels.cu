@@ -884,11 +884,11 @@ __global__ void __launch_bounds__(kElemThreads) k_aux(ElemArgs A) {
 // k_phase
 // ---------------------------------------------------------------------------
 __global__ void k_phase(PhaseArgs A) {
-    for (int64_t d = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; d < A.ndatum;
-         d += (int64_t)gridDim.x * blockDim.x) {
-        const ModelDev& M = A.models[A.dmodel[d]];
-        if (M.status < 0) continue;
-        const lcb_datum D = A.data[d];
+    const ModelDev& M = A.models[blockIdx.x];
+    if (M.status < 0) return;
+    for (int64_t m = (int64_t)blockIdx.y * blockDim.x + threadIdx.x; m < M.ndatum; m += (int64_t)gridDim.y * blockDim.x) {
+        const int64_t d = M.datum_begin + m;
+        const lcb_datum D = A.data[M.data_begin + m];
         double phase = (D.time - M.t0) / M.period;
         for (int k = 0; k < 4; ++k)
             phase -= (M.t0 + phase * (M.period + M.pdot * phase) - D.time) / (M.period + 2.0 * M.pdot * phase);
@@ -896,7 +896,7 @@ __global__ void k_phase(PhaseArgs A) {
         double expose = D.expose / M.period;
         double frac = (D.time - M.middle) / M.range;
         A.d_slfac[d] = 1.0 + frac * (M.slope + frac * (M.quad + frac * M.cube));
-        int64_t j = A.dsub0[d];
+        int64_t j = first_sub(M, A.dsub0, m);
         for (int nd = 0; nd < D.ndiv; ++nd, ++j) {
             double phi = phase, w = 1.0;
             if (D.ndiv != 1) {
@@ -1628,8 +1628,8 @@ __device__ void epilogue_iscale(const EpiArgs& A, const ModelDev& M, const Gint&
     double* X = A.svda + M.datum_begin * 5;
     for (int64_t d = threadIdx.x; d < M.ndatum; d += blockDim.x) {
         const int64_t gd = M.datum_begin + d;
-        const lcb_datum D = A.data[gd];
-        int64_t j = A.dsub0[gd] - M.sub_begin;
+        const lcb_datum D = A.data[M.data_begin + d];
+        int64_t j = first_sub(M, A.dsub0, d) - M.sub_begin;
         const double centre = (D.ndiv > 0 ? A.sp_phi[M.sub_begin + j] : 0.0) +
                               (D.ndiv > 1 ? 0.5 * D.expose / M.period : 0.0);
         double f[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
@@ -1655,7 +1655,7 @@ __device__ void epilogue_iscale(const EpiArgs& A, const ModelDev& M, const Gint&
         // rows with weight > 0, scaled by sqrt(weight)/ferr; other rows are zero and add nothing
         double nok[1] = {0.0};
         for (int64_t d = threadIdx.x; d < M.ndatum; d += blockDim.x) {
-            const lcb_datum D = A.data[M.datum_begin + d];
+            const lcb_datum D = A.data[M.data_begin + d];
             const double w = D.weight > 0.0 ? sqrt(D.weight) / D.ferr : 0.0;
             if (D.weight > 0.0) nok[0] += 1.0;
             for (int k = 0; k < 5; ++k) X[d * 5 + k] = F[d * 5 + k] * w;
@@ -1699,7 +1699,7 @@ __device__ void epilogue_iscale(const EpiArgs& A, const ModelDev& M, const Gint&
             for (int jc = 0; jc < ncol; ++jc) {
                 double su[2] = {0.0, 0.0};
                 for (int64_t d = threadIdx.x; d < M.ndatum; d += blockDim.x) {
-                    const lcb_datum D = A.data[M.datum_begin + d];
+                    const lcb_datum D = A.data[M.data_begin + d];
                     const double b = D.weight > 0.0 ? D.flux * sqrt(D.weight) / D.ferr : 0.0;
                     su[0] += X[d * 5 + jc] * X[d * 5 + jc];
                     su[1] += X[d * 5 + jc] * b;
@@ -1721,7 +1721,7 @@ __device__ void epilogue_iscale(const EpiArgs& A, const ModelDev& M, const Gint&
     double cw[2] = {0.0, 0.0};  // chi-squared, wnok
     for (int64_t d = threadIdx.x; d < M.ndatum; d += blockDim.x) {
         const int64_t gd = M.datum_begin + d;
-        const lcb_datum D = A.data[gd];
+        const lcb_datum D = A.data[M.data_begin + d];
         double c = sf[0] * F[d * 5 + 0] + sf[1] * F[d * 5 + 1] + sf[2] * F[d * 5 + 2] + sf[3] * F[d * 5 + 3];
         if (ncol == 5) c += sf[4] * F[d * 5 + 4];
         A.calc[gd] = c;
@@ -1780,7 +1780,8 @@ __global__ void __launch_bounds__(kEpiThreads) k_curve(EpiArgs A) {
     const int64_t m = blockIdx.x;
     const ModelDev& M = A.models[m];
     const bool in_range = LCB_IN_BOUNDS(M.pbase + (int64_t)M.nslots * M.nsub <= A.sz.npartial &&
-                                            M.datum_begin + M.ndatum <= A.sz.ndatum && M.sub_begin + M.nsub <= A.sz.nsub,
+                                            M.datum_begin + M.ndatum <= A.sz.ndatum && M.data_begin + M.ndatum <= A.sz.ndata &&
+                                            M.sub_begin + M.nsub <= A.sz.nsub,
                                         A.bad + m);
     if (M.status < 0 || A.status[m] != 0 || !in_range) {
         for (int64_t d = (int64_t)blockIdx.y * kEpiThreads + threadIdx.x; d < M.ndatum; d += (int64_t)gridDim.y * kEpiThreads)
@@ -1807,8 +1808,8 @@ __global__ void __launch_bounds__(kEpiThreads) k_curve(EpiArgs A) {
     for (int64_t d0 = ((int64_t)blockIdx.y * kTiles + (kShare > 1 ? 0 : warp)) * kCurveTile; d0 < M.ndatum; d0 += step) {
         const int64_t d = d0 + lane, gd = M.datum_begin + d;
         const bool on = d < M.ndatum;
-        const int ndiv = on ? A.data[gd].ndiv : 0;
-        const int64_t j0 = on ? A.dsub0[gd] - M.sub_begin : 0;
+        const int ndiv = on ? A.data[M.data_begin + d].ndiv : 0;
+        const int64_t j0 = on ? first_sub(M, A.dsub0, d) - M.sub_begin : 0;
         const int most = __reduce_max_sync(0xffffffffu, ndiv);  // the same in every warp that shares the tile
         double sum = 0.0;
         for (int nd = 0; nd < most; ++nd, buf ^= 1) {
@@ -1842,7 +1843,7 @@ __global__ void __launch_bounds__(kEpiThreads) k_curve(EpiArgs A) {
             }
         }
         if (lead && on) {
-            const lcb_datum D = A.data[gd];
+            const lcb_datum D = A.data[M.data_begin + d];
             const double c = A.d_slfac[gd] * (sum / (double)max(1, D.ndiv - 1)) + M.third;
             A.calc[gd] = c;
             if (D.weight > 0.0) {
@@ -1873,7 +1874,8 @@ __global__ void __launch_bounds__(kEpiThreads) k_results(EpiArgs A) {
     double* res = A.results + m * 12;
     __shared__ double red[kEpiThreads / 32], red4[4][kEpiThreads / 32];
     const bool in_range = M.pbase + (int64_t)M.nslots * M.nsub <= A.sz.npartial &&
-                          M.datum_begin + M.ndatum <= A.sz.ndatum && M.sub_begin + M.nsub <= A.sz.nsub;
+                          M.datum_begin + M.ndatum <= A.sz.ndatum && M.data_begin + M.ndatum <= A.sz.ndata &&
+                                            M.sub_begin + M.nsub <= A.sz.nsub;
     if (M.status < 0 || A.status[m] != 0 || !in_range) {
         if (blockIdx.y == 0 && threadIdx.x < 12) res[threadIdx.x] = NAN;
         return;
@@ -1903,7 +1905,7 @@ __global__ void __launch_bounds__(kEpiThreads) k_results(EpiArgs A) {
             for (int64_t d = (int64_t)blockIdx.y * kEpiThreads + threadIdx.x; d < M.ndatum;
                  d += (int64_t)gridDim.y * kEpiThreads) {
                 const int64_t gd = M.datum_begin + d;
-                const lcb_datum D = A.data[gd];
+                const lcb_datum D = A.data[M.data_begin + d];
                 const double c = A.calc[gd] * sfac;
                 A.calc[gd] = c;
                 if (D.weight > 0.0) chi += D.weight * sq((D.flux - c) / D.ferr);
@@ -2062,10 +2064,9 @@ int flux_blocks_per_sm() {
 }
 
 cudaError_t launch_phase(const PhaseArgs& a, cudaStream_t s) {
-    if (a.ndatum <= 0) return cudaSuccess;
-    int64_t blocks = (a.ndatum + 255) / 256;
-    if (blocks > 65535 * 8) blocks = 65535 * 8;
-    k_phase<<<(unsigned)blocks, 256, 0, s>>>(a);
+    if (a.nmodels <= 0 || a.most <= 0) return cudaSuccess;
+    const int64_t blocks = std::min<int64_t>((a.most + 127) / 128, 65535);
+    k_phase<<<dim3((unsigned)a.nmodels, (unsigned)blocks), 128, 0, s>>>(a);
     return cudaGetLastError();
 }
 

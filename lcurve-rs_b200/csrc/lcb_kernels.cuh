@@ -10,7 +10,7 @@ namespace lcb {
 
 // Sizes of the batch's arrays, for the index checks of the LCURVE_DEBUG_BOUNDS build.
 struct Sizes {
-    int64_t nelem, nsub, npartial, ndatum, nbands, nrings;
+    int64_t nelem, nsub, npartial, ndatum, nbands, nrings, ndata;
 };
 
 struct ElemArgs {
@@ -45,9 +45,8 @@ struct ElemArgs {
 struct PhaseArgs {
     const ModelDev* models;
     const lcb_datum* data;
-    const int32_t* dmodel;
-    const int64_t* dsub0;
-    int64_t ndatum;
+    const int64_t* dsub0;   // irregular models only (first_sub)
+    int64_t nmodels, most;  // the largest model's data
     float4* sp_e;
     double* sp_phi;
     int8_t* sp_type;

@@ -324,19 +324,37 @@ int highest_nonzero(const double* c) {
     return n;
 }
 
+// Latitude bands of a grid without infill: a function of nlat alone, shared by a batch's models.
+struct BandTable {
+    int nlat = 0;
+    int64_t count = 0, table = -1;  // elements; first band in the plan's table (-1: not in it)
+    std::vector<Band> bands;
+};
+
 struct ModelLayout {
     ModelDev dev;
+    std::vector<uint64_t> key;   // what the tables below, the blocks and the flux units depend on
     std::vector<SegDesc> segs;   // first = model-relative element offset
-    std::vector<Band> bands;     // SegDesc.table model-relative
+    std::vector<Band> bands;     // infilled grids' own; SegDesc.table model-relative, or with ntable < 0
+                                 // the index of a BandTable
     std::vector<Ring> rings;
     int64_t nelem = 0;
 };
 
 // Everything orchestration.rs:36-170 computes before the time loop, reduced
-// to per-model constants and element tables.
-void prepare_model(const Model& m, const lcb_datum* data, int64_t ndata, ModelLayout& L) {
+// to per-model constants and element tables.  Without `tabs` only the constants
+// and the key, with no segments or tables (replan_models).
+void prepare_model(const Model& m, const lcb_datum* data, int64_t ndata, ModelLayout& L, const std::vector<BandTable>* tabs) {
     ModelDev& D = L.dev;
     std::memset(&D, 0, sizeof D);
+    L.key.clear();
+    L.key.reserve(24);
+    auto key = [&](auto v) {
+        uint64_t u = 0;
+        static_assert(sizeof v <= sizeof u, "");
+        std::memcpy(&u, &v, sizeof v);
+        L.key.push_back(u);
+    };
     const double q = m.v(P_Q);
     const double spin1 = m.v(P_SPIN1), spin2 = m.v(P_SPIN2);
     double r1raw, r2raw;
@@ -445,13 +463,24 @@ void prepare_model(const Model& m, const lcb_datum* data, int64_t ndata, ModelLa
         bool infill = m.npole && !primary && (nf > 0 || ng > 0) && r2 > r1;
         double thelo = 0.0, thehi = 0.0;
         if (infill && !infill_limits(m, r1, r2, thelo, thehi)) { infill = false; nf = ng = 0; }
+        key((int64_t)nlat * 16 + role * 2 + infill);
+        if (infill) { key(thelo); key(thehi); key((int64_t)nf << 32 | (uint32_t)ng); }
+        if (!tabs) return;
         SegDesc s{};
         s.first = L.nelem;
         s.kind = primary ? SEG_STAR1 : SEG_STAR2;
         s.role = role;
-        s.table = (int32_t)L.bands.size();
-        s.count = star_bands(m, primary, nlat, infill, thelo, thehi, nf, ng, L.bands);
-        s.ntable = (int32_t)L.bands.size() - s.table;
+        if (infill) {
+            s.table = (int32_t)L.bands.size();
+            s.count = star_bands(m, primary, nlat, infill, thelo, thehi, nf, ng, L.bands);
+            s.ntable = (int32_t)L.bands.size() - s.table;
+        } else {  // without infill the fill counts do not enter
+            const auto t = std::lower_bound(tabs->begin(), tabs->end(), nlat,
+                                            [](const BandTable& a, int v) { return a.nlat < v; });
+            s.table = (int32_t)(t - tabs->begin());
+            s.count = t->count;
+            s.ntable = -1;
+        }
         s.fine_star = fine;
         L.nelem += s.count;
         L.segs.push_back(s);
@@ -466,13 +495,21 @@ void prepare_model(const Model& m, const lcb_datum* data, int64_t ndata, ModelLa
     D.rdisc1_l = m.v(P_RDISC1) > 0.0 ? m.v(P_RDISC1) : r1raw;
     D.rdisc2 = m.v(P_RDISC2) > 0.0 ? m.v(P_RDISC2) : m.v(P_RADIUS_SPOT);
     D.beta = m.v(P_BETA_DISC); D.height = m.v(P_HEIGHT_DISC);
+    key((int64_t)(m.add_disc ? 1 : 0) | (m.add_spot ? 2 : 0));
+    if (m.add_disc) { key((int64_t)m.nrad); key(D.rdisc1_g); key(D.rdisc2); key(D.height); key(D.beta); }
+    if (m.add_spot) key((int64_t)m.nspot);
+    // flux unit kinds and Roche blocks
+    key((int64_t)(D.beam1 != 0.0) | (int64_t)(D.beam2 != 0.0 || D.glens1) << 1 | (int64_t)(D.quad_ldf == 0.f) << 2 |
+        (int64_t)D.ltype1 << 3 | (int64_t)D.ltype2 << 7 | (int64_t)D.npoly1 << 11 | (int64_t)D.npoly2 << 15 |
+        (int64_t)(D.roche1 != 0) << 20 | (int64_t)(D.roche2 != 0) << 21 | (int64_t)(D.eclipse1 != 0) << 22 |
+        (int64_t)(D.eclipse2 != 0) << 23 | (int64_t)(D.iscale != 0) << 24);
     if (m.add_disc) {
         // set_disc_grid (grid.rs:336-392)
         SegDesc s{};
         s.first = L.nelem; s.kind = SEG_DISC; s.table = (int32_t)L.rings.size();
         double drad = (D.rdisc2 - D.rdisc1_g) / (double)m.nrad, drrad = D.rdisc2 / (double)m.nrad;
         int64_t cnt = 0;
-        for (int i = 0; i < m.nrad; ++i) {
+        for (int i = 0; tabs && i < m.nrad; ++i) {
             Ring g;
             g.rad = D.rdisc1_g + (D.rdisc2 - D.rdisc1_g) * ((double)i + 0.5) / (double)m.nrad;
             g.ntheta = std::max<int64_t>(8, sat_i32(std::ceil(kTwoPi * g.rad / drrad)));
@@ -562,13 +599,15 @@ void prepare_model(const Model& m, const lcb_datum* data, int64_t ndata, ModelLa
     // ephemeris and polynomial fudge (orchestration.rs:173-179, 231-241)
     D.t0 = m.v(P_T0); D.period = m.v(P_PERIOD); D.pdot = m.v(P_PDOT); D.deltat = m.v(P_DELTAT);
     D.slope = m.v(P_SLOPE); D.quad = m.v(P_QUAD); D.cube = m.v(P_CUBE); D.third = m.v(P_THIRD);
-    double xmin = data[0].time, xmax = data[0].time;
-    for (int64_t i = 1; i < ndata; ++i) {
-        if (data[i].time < xmin) xmin = data[i].time;
-        if (data[i].time > xmax) xmax = data[i].time;
+    if (tabs) {
+        double xmin = data[0].time, xmax = data[0].time;
+        for (int64_t i = 1; i < ndata; ++i) {
+            if (data[i].time < xmin) xmin = data[i].time;
+            if (data[i].time > xmax) xmax = data[i].time;
+        }
+        D.middle = (xmin + xmax) / 2.0;
+        D.range = (xmax - xmin) / 2.0;
     }
-    D.middle = (xmin + xmax) / 2.0;
-    D.range = (xmax - xmin) / 2.0;
 
     // log g reference terms (flux.rs:288-322)
     {
@@ -703,26 +742,9 @@ void parallel_for(int64_t n, int64_t grain, F&& f) {
     HostPool::get().run(n, (int)nthreads - 1, fn);
 }
 
-void plan_batch(const Model* const* models, int64_t n, const lcb_datum* data, const int64_t* start,
-                const int64_t* count, int num_sms, Plan& P, const PlanTuning& tune) {
-    P.reset();
-    P.models.resize(n);
-    P.model_ok.assign(n, 0);
-    P.model_err.assign(n, std::string());
-    std::vector<ModelLayout> lay(n);
-    auto prep = [&](int64_t i) {
-        int64_t nd = count[i];
-        try {
-            if (nd <= 0) throw Error(LCB_ERR_EMPTY, "no data points");
-            prepare_model(*models[i], data + start[i], nd, lay[i]);
-            P.model_ok[i] = 1;
-        } catch (const std::exception& e) {
-            P.model_err[i] = e.what();
-            lay[i] = ModelLayout();
-            std::memset(&lay[i].dev, 0, sizeof(ModelDev));
-            lay[i].dev.status = -1;
-        }
-    };
+namespace {
+
+void integrate_spots(const Model* const* models, int64_t n, const int64_t* count) {
     // a bright spot's stream integration (~0.7 ms) outweighs the rest of a model's planning:
     // the batch's pairs (q, radius_spot) missing from the memo are integrated first, one per
     // thread, so that a small batch (an MCMC step over q) does not run them eight to a thread
@@ -769,6 +791,57 @@ void plan_batch(const Model* const* models, int64_t n, const lcb_datum* data, co
             }
         });
     }
+}
+
+}  // namespace
+
+void host_copy(void* dst, const void* src, size_t bytes) {
+    constexpr size_t kPart = 1 << 18;
+    parallel_for((int64_t)((bytes + kPart - 1) / kPart), 4, [&](int64_t i) {
+        const size_t at = (size_t)i * kPart;
+        std::memcpy((char*)dst + at, (const char*)src + at, std::min(kPart, bytes - at));
+    });
+}
+
+void plan_batch(const Model* const* models, int64_t n, const lcb_datum* data, const int64_t* start,
+                const int64_t* count, int num_sms, Plan& P, const PlanTuning& tune) {
+    P.reset();
+    P.models.resize(n);
+    P.model_ok.assign(n, 0);
+    P.model_err.assign(n, std::string());
+    std::vector<ModelLayout> lay(n);
+    // the band tables of the batch's grids, each once (a batch's models mostly have the same grids)
+    std::vector<BandTable> tabs;
+    {
+        std::vector<int> nl;
+        for (int64_t i = 0; i < n; ++i) {
+            const Model& m = *models[i];
+            for (int v : {m.nlat1f, m.nlat1c, m.nlat2f, m.nlat2c})
+                if (nl.empty() || nl.back() != v) nl.push_back(v);
+        }
+        std::sort(nl.begin(), nl.end());
+        nl.erase(std::unique(nl.begin(), nl.end()), nl.end());
+        tabs.resize(nl.size());
+        parallel_for((int64_t)nl.size(), 8, [&](int64_t k) {
+            BandTable& t = tabs[k];
+            t.nlat = nl[k];
+            t.count = star_bands(*models[0], true, t.nlat, false, 0.0, 0.0, 0, 0, t.bands);
+        });
+    }
+    auto prep = [&](int64_t i) {
+        int64_t nd = count[i];
+        try {
+            if (nd <= 0) throw Error(LCB_ERR_EMPTY, "no data points");
+            prepare_model(*models[i], data + start[i], nd, lay[i], &tabs);
+            P.model_ok[i] = 1;
+        } catch (const std::exception& e) {
+            P.model_err[i] = e.what();
+            lay[i] = ModelLayout();
+            std::memset(&lay[i].dev, 0, sizeof(ModelDev));
+            lay[i].dev.status = -1;
+        }
+    };
+    integrate_spots(models, n, count);
     // models are independent: prepare them on the host's cores, 16 at least per thread
     // (one takes ~10 us, so waking helper threads only pays off for larger batches)
     parallel_for(n, 16, prep);
@@ -777,38 +850,68 @@ void plan_batch(const Model* const* models, int64_t n, const lcb_datum* data, co
     std::vector<int64_t> dbeg(n + 1, 0), sbeg(n + 1, 0);
     for (int64_t i = 0; i < n; ++i) dbeg[i + 1] = dbeg[i] + std::max<int64_t>(count[i], 0);
     P.ndatum = dbeg[n];
+    std::vector<int64_t> uniform(n, 0);  // the sub-divisions of every datum of the model, if alike
     parallel_for(n, 64, [&](int64_t i) {
+        const int64_t nd = dbeg[i + 1] - dbeg[i];
+        if (!P.model_ok[i] || nd == 0) return;
+        const int first = data[start[i]].ndiv;
+        bool alike = first > 0;
         int64_t ns = 0;
-        if (P.model_ok[i])
-            for (int64_t k = 0; k < dbeg[i + 1] - dbeg[i]; ++k) ns += std::max(data[start[i] + k].ndiv, 0);
+        for (int64_t k = 0; k < nd; ++k) {
+            const int v = data[start[i] + k].ndiv;
+            ns += std::max(v, 0);
+            alike = alike && v == first;
+        }
         sbeg[i + 1] = ns;
+        uniform[i] = alike ? first : 0;
     });
     for (int64_t i = 0; i < n; ++i) {
         if (sbeg[i + 1] > INT32_MAX / 2) throw Error(LCB_ERR_INVALID, "too many sub-phases in one model");
         sbeg[i + 1] += sbeg[i];
     }
-    P.datum_model.resize(P.ndatum);
-    P.datum_sub0.resize(P.ndatum);
-    P.datum_src.resize(P.ndatum);
-    parallel_for(n, 64, [&](int64_t i) {
+    bool irregular = false;
+    for (int64_t i = 0; i < n; ++i) {
         ModelDev& D = lay[i].dev;
         D.datum_begin = dbeg[i];
         D.ndatum = dbeg[i + 1] - dbeg[i];
         D.sub_begin = sbeg[i];
         D.nsub = sbeg[i + 1] - sbeg[i];
-        int64_t sub = sbeg[i];
-        for (int64_t k = 0, dd = dbeg[i]; k < D.ndatum; ++k, ++dd) {
-            const int64_t src = start[i] + k;
-            P.datum_model[dd] = (int32_t)i;
-            P.datum_sub0[dd] = sub;
-            P.datum_src[dd] = src;
-            if (P.model_ok[i]) sub += std::max(data[src].ndiv, 0);
-        }
-    });
+        D.ndiv = uniform[i];
+        irregular = irregular || (P.model_ok[i] && D.nsub > 0 && !D.ndiv);
+        P.most_data = std::max(P.most_data, D.ndatum);
+    }
+    if (tune.datum_tables || irregular) P.datum_sub0.resize(P.ndatum);
+    if (tune.datum_tables) {
+        P.datum_model.resize(P.ndatum);
+        P.datum_src.resize(P.ndatum);
+    }
+    if (!P.datum_sub0.empty())
+        parallel_for(n, 64, [&](int64_t i) {
+            const ModelDev& D = lay[i].dev;
+            int64_t sub = sbeg[i];
+            for (int64_t k = 0, dd = dbeg[i]; k < D.ndatum; ++k, ++dd) {
+                const int64_t src = start[i] + k;
+                P.datum_sub0[dd] = sub;
+                if (tune.datum_tables) {
+                    P.datum_model[dd] = (int32_t)i;
+                    P.datum_src[dd] = src;
+                }
+                if (P.model_ok[i]) sub += std::max(data[src].ndiv, 0);
+            }
+        });
     P.nsub = sbeg[n];
-    P.datum_contiguous = true;
-    for (int64_t i = 1; i < n && P.datum_contiguous; ++i)
-        P.datum_contiguous = start[i] == start[i - 1] + std::max<int64_t>(count[i - 1], 0);
+    // the records to upload: the range that the models' data span
+    int64_t lo = 0, hi = 0;
+    bool some = false;
+    for (int64_t i = 0; i < n; ++i)
+        if (count[i] > 0) {
+            lo = some ? std::min(lo, start[i]) : start[i];
+            hi = some ? std::max(hi, start[i] + count[i]) : start[i] + count[i];
+            some = true;
+        }
+    P.data_first = lo;
+    P.data_count = hi - lo;
+    for (int64_t i = 0; i < n; ++i) lay[i].dev.data_begin = count[i] > 0 ? start[i] - lo : 0;
 
     // global element / table layout (a model's segments are contiguous): offsets of each model's
     // segments, bands, rings and elements, then the tables filled in parallel
@@ -820,19 +923,38 @@ void plan_batch(const Model* const* models, int64_t n, const lcb_datum* data, co
         ring_begin[i + 1] = ring_begin[i] + lay[i].rings.size();
         elem_begin[i + 1] = elem_begin[i] + lay[i].nelem;
     }
+    int64_t shared = 0;  // the shared band tables that some model uses come first
+    for (const ModelLayout& L : lay)
+        for (const SegDesc& g : L.segs)
+            if ((g.kind == SEG_STAR1 || g.kind == SEG_STAR2) && g.ntable < 0) tabs[g.table].table = 0;
+    for (BandTable& t : tabs)
+        if (t.table == 0) {
+            t.table = shared;
+            shared += (int64_t)t.bands.size();
+        }
     P.segs.resize(seg_begin[n]);
-    P.bands.resize(band_begin[n]);
+    P.bands.resize(shared + band_begin[n]);
+    for (const BandTable& t : tabs)
+        if (t.table >= 0) std::copy(t.bands.begin(), t.bands.end(), P.bands.begin() + t.table);
     P.rings.resize(ring_begin[n]);
     P.nelem = elem_begin[n];
     parallel_for(n, 64, [&](int64_t i) {
         const ModelLayout& L = lay[i];
-        std::copy(L.bands.begin(), L.bands.end(), P.bands.begin() + band_begin[i]);
+        std::copy(L.bands.begin(), L.bands.end(), P.bands.begin() + shared + band_begin[i]);
         std::copy(L.rings.begin(), L.rings.end(), P.rings.begin() + ring_begin[i]);
         size_t k = seg_begin[i];
         for (SegDesc s : L.segs) {
             s.first += elem_begin[i];
             s.model = (int32_t)i;
-            if (s.kind == SEG_STAR1 || s.kind == SEG_STAR2) s.table += (int32_t)band_begin[i];
+            if (s.kind == SEG_STAR1 || s.kind == SEG_STAR2) {
+                if (s.ntable < 0) {
+                    const BandTable& t = tabs[s.table];
+                    s.table = (int32_t)t.table;
+                    s.ntable = (int32_t)t.bands.size();
+                } else {
+                    s.table += (int32_t)(shared + band_begin[i]);
+                }
+            }
             if (s.kind == SEG_DISC) s.table += (int32_t)ring_begin[i];
             P.segs[k++] = s;
         }
@@ -994,8 +1116,10 @@ void plan_batch(const Model* const* models, int64_t n, const lcb_datum* data, co
     P.units.resize(nu);
     for (size_t k = 0; k < nu; ++k) P.units[k] = fu[idx[k]].second;
 
+    P.keys.resize(n);
     for (int64_t i = 0; i < n; ++i) {
         P.models[i] = lay[i].dev;
+        P.keys[i].swap(lay[i].key);
         P.any_iscale = P.any_iscale || (P.model_ok[i] && lay[i].dev.iscale);
     }
 
@@ -1020,7 +1144,38 @@ void plan_batch(const Model* const* models, int64_t n, const lcb_datum* data, co
                    (int64_t)P.rblocks.size(), (int64_t)P.ablocks.size(), (int64_t)P.segs.size(),
                    (int64_t)P.bands.size(), (int64_t)P.rings.size(), (int64_t)P.roche_split, (int64_t)P.split_fix,
                    (int64_t)P.flux_blocks_per_sm, (int64_t)P.curve_blocks, (int64_t)P.result_blocks,
-                   (int64_t)P.curve_share, (int64_t)P.flux_share};
+                   (int64_t)P.curve_share, (int64_t)P.flux_share, P.data_count, P.most_data,
+                   (int64_t)P.datum_sub0.size()};
+}
+
+bool replan_models(const Model* const* models, int64_t n, const lcb_datum* data, const int64_t* start,
+                   const int64_t* count, Plan& P) {
+    if ((int64_t)P.models.size() != n || (int64_t)P.keys.size() != n) return false;
+    integrate_spots(models, n, count);
+    std::vector<ModelLayout> lay(n);
+    std::atomic<bool> same{true};
+    parallel_for(n, 8, [&](int64_t i) {
+        try {
+            if (!P.model_ok[i]) throw Error(LCB_ERR_MODEL, P.model_err[i]);
+            prepare_model(*models[i], data + start[i], count[i], lay[i], nullptr);
+            if (lay[i].key != P.keys[i]) same.store(false);
+        } catch (const std::exception&) {  // a model that fails, or failed before: the whole plan again
+            same.store(false);
+        }
+    });
+    if (!same.load()) return false;
+    for (int64_t i = 0; i < n; ++i) {
+        ModelDev& D = lay[i].dev;
+        const ModelDev& O = P.models[i];
+        D.middle = O.middle; D.range = O.range;
+        D.sub_begin = O.sub_begin; D.nsub = O.nsub;
+        D.datum_begin = O.datum_begin; D.ndatum = O.ndatum;
+        D.data_begin = O.data_begin; D.ndiv = O.ndiv;
+        D.pbase = O.pbase;
+        D.nslots = O.nslots; D.g1_end = O.g1_end; D.g2_end = O.g2_end; D.gd_end = O.gd_end; D.ge_end = O.ge_end;
+        P.models[i] = D;
+    }
+    return true;
 }
 
 }  // namespace lcb

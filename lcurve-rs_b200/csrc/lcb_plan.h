@@ -15,6 +15,7 @@ struct PlanTuning {
     int flux_chunks = 0;         // elements per flux work unit, in chunks of kFluxChunk (1..16)
     int roche_split = 0;         // threads per Roche-eclipsed element in the phase scan (1..16)
     int flux_blocks_per_sm = 0;  // persistent flux blocks per SM (1..occupancy limit)
+    bool datum_tables = true;    // fill datum_model / datum_sub0 / datum_src for regular models too
 };
 
 struct Plan {
@@ -26,17 +27,20 @@ struct Plan {
     std::vector<ElemBlock> rblocks;    // k_roche
     std::vector<ElemBlock> ablocks;    // k_aux
     std::vector<FluxUnit> units;
-    std::vector<int32_t> datum_model;   // per (model, datum): model index
-    std::vector<int64_t> datum_sub0;    // per (model, datum): first global sub-phase
-    std::vector<int64_t> datum_src;     // per (model, datum): index into the caller's data array
+    // per (model, datum), with PlanTuning::datum_tables, or datum_sub0 where some model is irregular:
+    std::vector<int32_t> datum_model;   // model index
+    std::vector<int64_t> datum_sub0;    // first global sub-phase
+    std::vector<int64_t> datum_src;     // index into the caller's data array
+    // the records to upload, the caller's [data_first, data_first + data_count): the range that the
+    // models' data span (they may share records); the largest model's data
+    int64_t data_first = 0, data_count = 0, most_data = 0;
+    std::vector<std::vector<uint64_t>> keys;  // per model: what its tables and units depend on (replan_models)
     std::vector<int32_t> model_ok;      // 1 = planned, 0 = failed (NaN chisq)
     std::vector<std::string> model_err;
     int64_t nelem = 0, nsub = 0, ndatum = 0, npartial = 0;
     int64_t evals = 0, roche_elems = 0;
     // Signature of everything that fixes buffer sizes and launch shapes.
     std::vector<int64_t> shape_key;
-    // datum_src[d] == datum_src[0] + d for every d: the data can be copied as one range
-    bool datum_contiguous = false;
     bool any_iscale = false;  // some model fits per-component scale factors (needs fcomp scratch)
     int roche_split = 1;      // threads per element of the general eclipse search, were every element left to it
     int split_fix = 0;        // PlanTuning::roche_split where it applies: fixed, whatever the list's length
@@ -53,7 +57,8 @@ struct Plan {
         ablocks.clear(); units.clear(); datum_model.clear(); datum_sub0.clear(); datum_src.clear();
         model_ok.clear(); model_err.clear(); shape_key.clear();
         nelem = nsub = ndatum = npartial = evals = roche_elems = 0;
-        datum_contiguous = false;
+        data_first = data_count = most_data = 0;
+        keys.clear();
         any_iscale = false;
         roche_split = 1;
         split_fix = 0;
@@ -70,6 +75,15 @@ struct Plan {
 // invalid are marked failed (model_ok = 0) instead of throwing.
 void plan_batch(const Model* const* models, int64_t n, const lcb_datum* data, const int64_t* start,
                 const int64_t* count, int num_sms, Plan& out, const PlanTuning& tune = PlanTuning{});
+
+// New physical parameters for the models of a plan on the same data: fills in the model table alone and
+// returns true when no table, block or unit of the plan depends on what changed; false: plan again (the
+// plan is then unchanged).
+bool replan_models(const Model* const* models, int64_t n, const lcb_datum* data, const int64_t* start,
+                   const int64_t* count, Plan& P);
+
+// Copies bytes on the host's threads (large copies only; a few MB and more).
+void host_copy(void* dst, const void* src, size_t bytes);
 
 // Scan threads of the split eclipse search that fill the GPU: sixteen waves of five 128-thread blocks.
 inline int64_t split_target(int num_sms) { return (int64_t)(num_sms > 1 ? num_sms : 1) * 640 * 16; }
