@@ -9,8 +9,9 @@
 //
 // GEMM kernel (k_gemm): C[M x N] = A[M x K] . B[N x K]^T, both operands BF16
 // row-major (K contiguous), FP32 accumulation in tensor memory:
-//   - one CTA per 128 x TBN output tile (TBN = 256 when N >= 256, else 128),
-//     sixteen warps; a K-split grid (blockIdx.z) for FP32 outputs;
+//   - one CTA per 128 x TBN output tile (TBN = 256 when N >= 256, else 128; 32
+//     where those would leave most SMs idle), sixteen warps; a K-split grid
+//     (blockIdx.z) for FP32 outputs;
 //   - warp 0 lane 0 streams 64-wide K-slices of A and B into shared memory
 //     with TMA (cp.async.bulk.tensor, 128-byte swizzle), four stages on
 //     mbarriers;
@@ -79,8 +80,9 @@ struct GemmSmem {
     uint32_t tmem_base;
     int abort;
 };
-// the epilogue's per-warp staging (6 KB a warp) reuses a[] and b[]
+// the epilogue's per-warp staging (6 KB a warp that has columns) reuses a[] and b[]
 static_assert((GEMM_THREADS / 32) * 6144 <= STAGES * (TILE_A + tile_b<128>()), "epilogue staging");
+static_assert(4 * 6144 <= STAGES * TILE_A, "epilogue staging of one column chunk");
 
 struct GemmArgs {
     int M, N, K;
@@ -488,17 +490,17 @@ __global__ void k_cast_weights(int64_t n, LayerTab T, const float* __restrict__ 
     }
 }
 
-// Per-row chi-squared of a surrogate curve: flux_j = exp(pred_j * sd_j + mean_j),
-// optionally scaled by the least-squares factor (orchestration.rs:361-401 re_scale).
-__global__ void k_logflux_chisq(int rows, int n, const float* __restrict__ pred, const float* __restrict__ mean,
-                                const float* __restrict__ sd, const double* __restrict__ flux,
-                                const double* __restrict__ ferr, int scale, double* __restrict__ out) {
-    __shared__ double red[3][8];
-    const int r = blockIdx.x;
-    if (r >= rows) return;
+// Chi-squared of one surrogate curve: flux_j = exp(pred_j * sd_j + mean_j),
+// optionally scaled by the least-squares factor (orchestration.rs:361-401
+// re_scale); by a block of kChisqThreads, the value on thread 0.
+constexpr int kChisqThreads = 128;
+__device__ __forceinline__ double row_chisq(int n, const float* __restrict__ pred, const float* __restrict__ mean,
+                                            const float* __restrict__ sd, const double* __restrict__ flux,
+                                            const double* __restrict__ ferr, int scale) {
+    __shared__ double red[3][kChisqThreads / 32];
     double sff = 0, sfd = 0, sdd = 0;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        const double f = exp((double)pred[(size_t)r * n + j] * sd[j] + mean[j]);
+    for (int j = threadIdx.x; j < n; j += kChisqThreads) {
+        const double f = exp((double)pred[j] * sd[j] + mean[j]);
         const double w = 1.0 / (ferr[j] * ferr[j]);
         sff += w * f * f;
         sfd += w * f * flux[j];
@@ -516,16 +518,24 @@ __global__ void k_logflux_chisq(int rows, int n, const float* __restrict__ pred,
         red[2][wid] = sdd;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double a = 0, b = 0, c = 0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) {
-            a += red[0][k];
-            b += red[1][k];
-            c += red[2][k];
-        }
-        const double s = scale ? (a > 0 ? b / a : 0.0) : 1.0;
-        out[r] = c - 2 * s * b + s * s * a;  // sum w (d - s f)^2
+    double a = 0, b = 0, c = 0;
+    for (int k = 0; k < kChisqThreads / 32; ++k) {
+        a += red[0][k];
+        b += red[1][k];
+        c += red[2][k];
     }
+    const double s = scale ? (a > 0 ? b / a : 0.0) : 1.0;
+    return c - 2 * s * b + s * s * a;  // sum w (d - s f)^2
+}
+
+__global__ void __launch_bounds__(kChisqThreads) k_logflux_chisq(int n, const float* __restrict__ pred,
+                                                                 const float* __restrict__ mean, const float* __restrict__ sd,
+                                                                 const double* __restrict__ flux,
+                                                                 const double* __restrict__ ferr, int scale,
+                                                                 double* __restrict__ out) {
+    const int r = blockIdx.x;
+    const double chi = row_chisq(n, pred + (size_t)r * n, mean, sd, flux, ferr, scale);
+    if (threadIdx.x == 0) out[r] = chi;
 }
 
 // ---------------------------------------------------------------------------
@@ -547,7 +557,8 @@ struct StretchArgs {
     double* lz;            // n: log proposal-density ratio, or -inf outside the prior box
     double* lq;            // n: KDE log density at the current positions
     double* lqp;           // n: KDE log density at the proposals
-    float* xin;            // n x n_in network inputs
+    __nv_bfloat16* xin;    // n x ld network inputs, padded with zeros
+    int ld;
     double lo[kMaxDim], hi[kMaxDim];
     float fmul[kMaxDim], fadd[kMaxDim];
     int frecip[kMaxDim];
@@ -557,21 +568,40 @@ struct StretchArgs {
                            // parameter, so one captured graph serves every half-step
 };
 
+// The network's input row of a proposal: fadd + fmul * (v or 1/v) per dimension,
+// separate multiply and add (no contraction: the host computes the inputs the
+// same way), rounded to float and then to bfloat16 as the packed inputs are.
+__device__ __forceinline__ void put_input(const StretchArgs& A, int i, int k, double v) {
+    const double f = A.frecip[k] ? 1.0 / v : v;
+    A.xin[(size_t)i * A.ld + k] =
+        __float2bfloat16_rn((float)__dadd_rn((double)A.fadd[k], __dmul_rn((double)A.fmul[k], f)));
+}
+
 // log of the Gaussian KDE of the complementary walkers at v (up to a constant),
 // log sum_j exp(-(v - c_j)^T prec (v - c_j) / 2), computed by one warp: each lane
 // takes every 32nd component, then a log-sum-exp across the warp.  Every lane
-// returns the value.
-__device__ double kde_logq_warp(const StretchArgs& A, const double* v) {
+// returns the value.  D: the dimension, known to the compiler, so that the
+// kernel covariance's inverse and the differences stay in registers.
+template <int D>
+__device__ __forceinline__ double kde_logq_warp(const StretchArgs& A, const double* v) {
     const int lane = threadIdx.x & 31;
-    const double* prec = A.kde + kMaxDim * kMaxDim;
+    double prec[D][D];
+#pragma unroll
+    for (int k = 0; k < D; ++k)
+#pragma unroll
+        for (int l = 0; l < D; ++l) prec[k][l] = __ldg(A.kde + kMaxDim * kMaxDim + k * kMaxDim + l);
     double mx = -INFINITY, acc = 0.0;
+#pragma unroll 2
     for (int j = lane; j < A.m; j += 32) {
-        double dv[kMaxDim];
-        for (int k = 0; k < A.d; ++k) dv[k] = v[k] - A.comp[(size_t)j * A.d + k];
+        double dv[D];
+#pragma unroll
+        for (int k = 0; k < D; ++k) dv[k] = v[k] - A.comp[(size_t)j * D + k];
         double qf = 0.0;
-        for (int k = 0; k < A.d; ++k) {
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
             double t = 0.0;
-            for (int l = 0; l < A.d; ++l) t += prec[k * kMaxDim + l] * dv[l];
+#pragma unroll
+            for (int l = 0; l < D; ++l) t += prec[k][l] * dv[l];
             qf += dv[k] * t;
         }
         const double e = -0.5 * qf;
@@ -589,44 +619,51 @@ __device__ double kde_logq_warp(const StretchArgs& A, const double* v) {
     return wmx + log(part);
 }
 
-constexpr int kWalkersPerBlock = 4;  // one warp per walker in the KDE kernels
-
-__global__ void k_kde_logq(StretchArgs A) {
-    const int i = blockIdx.x * kWalkersPerBlock + (threadIdx.x >> 5);
-    if (i >= A.n || A.move != MOVE_KDE) return;  // uniform per warp
-    double v[kMaxDim];
-    for (int k = 0; k < A.d; ++k) v[k] = A.y[(size_t)i * A.d + k];
-    const double lq = kde_logq_warp(A, v);
-    if ((threadIdx.x & 31) == 0) A.lq[i] = lq;
-}
+constexpr int kWalkersPerBlock = 2;  // one warp per walker in the KDE kernels
 
 // KDE move (emcee's KDEMove): an independence proposal from the Gaussian KDE
 // of the complementary walkers, y' = c_j + chol eps, for walker i (one warp);
 // writes y', its network inputs and the log density ratio log q(y) - log q(y'),
-// or -inf outside the prior box.
-__global__ void k_kde_propose(StretchArgs A, int step) {
+// or -inf outside the prior box.  The first step also computes log q(y).
+template <int D>
+__global__ void __launch_bounds__(32 * kWalkersPerBlock) k_kde_propose(StretchArgs A, int step) {
     const int i = blockIdx.x * kWalkersPerBlock + (threadIdx.x >> 5);
     if (i >= A.n) return;  // uniform per warp
-    const bool lead = (threadIdx.x & 31) == 0;
+    const int lane = threadIdx.x & 31;
     const double* r = A.rnd + ((size_t)step * A.n + i) * A.rstride;
     const int j = min((int)(r[0] * A.m), A.m - 1);
-    double v[kMaxDim];
+    double v[D];
     bool inside = true;
-    for (int k = 0; k < A.d; ++k) {
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
         double t = 0.0;
-        for (int l = 0; l <= k; ++l) t += A.kde[k * kMaxDim + l] * r[3 + l];
-        v[k] = A.comp[(size_t)j * A.d + k] + t;
+#pragma unroll
+        for (int l = 0; l <= k; ++l) t += __ldg(A.kde + k * kMaxDim + l) * r[3 + l];
+        v[k] = A.comp[(size_t)j * D + k] + t;
         inside = inside && v[k] >= A.lo[k] && v[k] <= A.hi[k];
-        if (lead) {
-            A.yp[(size_t)i * A.d + k] = v[k];
-            const double f = A.frecip[k] ? 1.0 / v[k] : v[k];
-            A.xin[(size_t)i * A.n_in + k] = (float)__dadd_rn((double)A.fadd[k], __dmul_rn((double)A.fmul[k], f));
-        }
     }
-    const double lqp = kde_logq_warp(A, v);
-    if (lead) {
+    double own = v[0];  // a dimension per lane
+#pragma unroll
+    for (int k = 1; k < D; ++k)
+        if (lane == k) own = v[k];
+    if (lane < D) {
+        A.yp[(size_t)i * D + lane] = own;
+        put_input(A, i, lane, own);
+    }
+    const double lqp = kde_logq_warp<D>(A, v);
+    double lq;
+    if (step == 0) {
+        double y[D];
+#pragma unroll
+        for (int k = 0; k < D; ++k) y[k] = A.y[(size_t)i * D + k];
+        lq = kde_logq_warp<D>(A, y);
+    } else {
+        lq = A.lq[i];
+    }
+    if (lane == 0) {
+        if (step == 0) A.lq[i] = lq;
         A.lqp[i] = lqp;
-        A.lz[i] = inside ? A.lq[i] - lqp : -INFINITY;
+        A.lz[i] = inside ? lq - lqp : -INFINITY;
     }
 }
 
@@ -648,21 +685,24 @@ __global__ void k_stretch_propose(StretchArgs A, int step) {
         const double v = __dadd_rn(c, __dmul_rn(z, __dsub_rn(A.y[(size_t)i * A.d + k], c)));
         A.yp[(size_t)i * A.d + k] = v;
         inside = inside && v >= A.lo[k] && v <= A.hi[k];
-        const double f = A.frecip[k] ? 1.0 / v : v;
-        // separate multiply and add (no contraction): the host computes the inputs the same way
-        A.xin[(size_t)i * A.n_in + k] = (float)__dadd_rn((double)A.fadd[k], __dmul_rn((double)A.fmul[k], f));
+        put_input(A, i, k, v);
     }
     A.lz[i] = inside ? (A.d - 1) * log(z) : -INFINITY;
 }
 
 // Metropolis step of the sub-chain: accept y' with min(1, z^(d-1) exp(l~(y') - l~(y))),
-// l~ = -chisq / 2 inside the prior box.
-__global__ void k_stretch_accept(StretchArgs A, const double* __restrict__ chi, int step) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= A.n) return;
+// l~ = -chisq / 2 inside the prior box; walker r's chi-squared by the block that
+// decides on it.
+__global__ void __launch_bounds__(kChisqThreads) k_chisq_accept(StretchArgs A, int n, const float* __restrict__ pred,
+                                                                const float* __restrict__ mean, const float* __restrict__ sd,
+                                                                const double* __restrict__ flux,
+                                                                const double* __restrict__ ferr, int scale, int step) {
+    const int i = blockIdx.x;
+    const double chi = row_chisq(n, pred + (size_t)i * n, mean, sd, flux, ferr, scale);
+    if (threadIdx.x != 0) return;
     const double lz = A.lz[i];
     if (lz == -INFINITY) return;
-    double lsp = -0.5 * chi[i];
+    double lsp = -0.5 * chi;
     if (!(lsp == lsp)) lsp = -INFINITY;
     const double logu = A.rnd[((size_t)step * A.n + i) * A.rstride + 2];
     if (logu < lz + lsp - A.ls[i]) {
@@ -753,10 +793,19 @@ void prepare_gemm_attributes() {
     LCB_SMEM_ATTR(EPI_DGELU, 128);
     LCB_SMEM_ATTR(EPI_F32, 256); LCB_SMEM_ATTR(EPI_BIAS_GELU, 256); LCB_SMEM_ATTR(EPI_BIAS_F32, 256);
     LCB_SMEM_ATTR(EPI_DGELU, 256);
+    LCB_SMEM_ATTR(EPI_F32, 32); LCB_SMEM_ATTR(EPI_BIAS_GELU, 32); LCB_SMEM_ATTR(EPI_BIAS_F32, 32);
+    LCB_SMEM_ATTR(EPI_DGELU, 32);
 #undef LCB_SMEM_ATTR
 }
 
 int tile_n(int64_t N) { return N >= 256 ? 256 : 128; }  // 128 x 256 tiles where N allows
+// ... unless they fill less than an eighth of the SMs: then 128 x 32 tiles, whose epilogue (a GELU of
+// every element) is spread over up to eight times the SMs.  128 x 512 x 512 with GELU: 16 us on two
+// CTAs of 128 x 256, 5 us on sixteen of 128 x 32; at 8 and more row tiles the wide ones win (the
+// operands are read once per tile).
+bool narrow_tiles(int64_t M, int64_t N) {
+    return ((M + BM - 1) / BM) * ((N + tile_n(N) - 1) / tile_n(N)) * 8 < 148;
+}
 
 // Number of K-splits for an FP32-output GEMM: enough CTAs to cover `sms` SMs, none of them empty.
 int split_count(int64_t M, int64_t N, int64_t K, int sms) {
@@ -787,18 +836,22 @@ void gemm(int mode, int64_t M, int64_t N, int64_t K, const void* A, const void* 
     const int nk = (int)((K + BK - 1) / BK), kchunks = (nk + splits - 1) / std::max(splits, 1);
     if (splits < 1 || (splits > 1 && mode != EPI_F32) || (nk + kchunks - 1) / kchunks != splits)
         throw Fail(LCB_ERR_INVALID, "GEMM K-split must be an FP32-output split with no empty part");
-    const bool wide = tile_n(N) == 256;
-    const CUtensorMap ta = bf16_map(A, M, K, 128u), tb = bf16_map(B, N, K, wide ? 256u : 128u);
+    const int width = splits == 1 && narrow_tiles(M, N) ? 2 : tile_n(N) == 256 ? 1 : 0;
+    const CUtensorMap ta = bf16_map(A, M, K, 128u), tb = bf16_map(B, N, K, width == 2 ? 32u : width ? 256u : 128u);
     GemmArgs g{(int)M, (int)N, (int)K, kchunks, M * N, bias, aux, out, out2, outT, err};
-    switch (mode * 2 + (wide ? 1 : 0)) {
-        case EPI_F32 * 2: launch_gemm_mode<EPI_F32, 128>(ta, tb, g, s); break;
-        case EPI_F32 * 2 + 1: launch_gemm_mode<EPI_F32, 256>(ta, tb, g, s); break;
-        case EPI_BIAS_GELU * 2: launch_gemm_mode<EPI_BIAS_GELU, 128>(ta, tb, g, s); break;
-        case EPI_BIAS_GELU * 2 + 1: launch_gemm_mode<EPI_BIAS_GELU, 256>(ta, tb, g, s); break;
-        case EPI_BIAS_F32 * 2: launch_gemm_mode<EPI_BIAS_F32, 128>(ta, tb, g, s); break;
-        case EPI_BIAS_F32 * 2 + 1: launch_gemm_mode<EPI_BIAS_F32, 256>(ta, tb, g, s); break;
-        case EPI_DGELU * 2: launch_gemm_mode<EPI_DGELU, 128>(ta, tb, g, s); break;
-        case EPI_DGELU * 2 + 1: launch_gemm_mode<EPI_DGELU, 256>(ta, tb, g, s); break;
+    switch (mode * 3 + width) {
+        case EPI_F32 * 3 + 0: launch_gemm_mode<EPI_F32, 128>(ta, tb, g, s); break;
+        case EPI_F32 * 3 + 1: launch_gemm_mode<EPI_F32, 256>(ta, tb, g, s); break;
+        case EPI_F32 * 3 + 2: launch_gemm_mode<EPI_F32, 32>(ta, tb, g, s); break;
+        case EPI_BIAS_GELU * 3 + 0: launch_gemm_mode<EPI_BIAS_GELU, 128>(ta, tb, g, s); break;
+        case EPI_BIAS_GELU * 3 + 1: launch_gemm_mode<EPI_BIAS_GELU, 256>(ta, tb, g, s); break;
+        case EPI_BIAS_GELU * 3 + 2: launch_gemm_mode<EPI_BIAS_GELU, 32>(ta, tb, g, s); break;
+        case EPI_BIAS_F32 * 3 + 0: launch_gemm_mode<EPI_BIAS_F32, 128>(ta, tb, g, s); break;
+        case EPI_BIAS_F32 * 3 + 1: launch_gemm_mode<EPI_BIAS_F32, 256>(ta, tb, g, s); break;
+        case EPI_BIAS_F32 * 3 + 2: launch_gemm_mode<EPI_BIAS_F32, 32>(ta, tb, g, s); break;
+        case EPI_DGELU * 3 + 0: launch_gemm_mode<EPI_DGELU, 128>(ta, tb, g, s); break;
+        case EPI_DGELU * 3 + 1: launch_gemm_mode<EPI_DGELU, 256>(ta, tb, g, s); break;
+        case EPI_DGELU * 3 + 2: launch_gemm_mode<EPI_DGELU, 32>(ta, tb, g, s); break;
         default: throw Fail(LCB_ERR_INVALID, "unknown GEMM epilogue mode");
     }
 }
@@ -854,8 +907,7 @@ struct lcb_mlp {
     DBuf<float> wsplit;               // FP32 partial products of the K-split weight-gradient GEMMs
     DBuf<int> err;
     DBuf<double> loss;
-    DBuf<float> sub_x;                   // sub-chain: network inputs
-    DBuf<double> sub_yp, sub_lz, sub_chi;  // proposals, log proposal ratio, chi-squared
+    DBuf<double> sub_yp, sub_lz;           // sub-chain: proposals, log proposal ratio
     DBuf<double> sub_lq, sub_lqp;          // KDE log densities (current, proposed)
     DBuf<double> sub_kde;                  // KDE factors of the current call
     DBuf<double> sub_y, sub_ls, sub_comp, sub_rnd;  // fixed copies of the sub-chain's inputs (graph operands)
@@ -877,7 +929,7 @@ struct lcb_mlp {
         p.free(); m.free(); v.free(); g.free(); wbf.free(); wtbf.free(); x0.free(); pred.free(); dzt.free(); xt.free();
         wsplit.free();
         dz[0].free(); dz[1].free(); err.free(); loss.free();
-        sub_x.free(); sub_yp.free(); sub_lz.free(); sub_chi.free(); sub_lq.free(); sub_lqp.free(); sub_kde.free();
+        sub_yp.free(); sub_lz.free(); sub_lq.free(); sub_lqp.free(); sub_kde.free();
         sub_y.free(); sub_ls.free(); sub_comp.free(); sub_rnd.free(); sub_stage.free();
         if (sub_pinned) cudaFreeHost(sub_pinned);
         sub_pinned = nullptr;
@@ -901,9 +953,11 @@ struct lcb_mlp {
     // keep_t: also store each hidden activation transposed (yT), for the weight gradients
     void forward(const float* x, int64_t B, float* y_out, bool keep_t = false) {
         if (B <= 0 || B > max_batch) throw Fail(LCB_ERR_INVALID, "batch size out of range");
-        const int64_t nx = B * in[0];
-        k_pack_input<<<(unsigned)((nx + 255) / 256), 256, 0, stream>>>((int)B, n_in, in[0], x, x0.p);
-        CK(cudaGetLastError());
+        if (x) {  // else x0 holds the packed rows already
+            const int64_t nx = B * in[0];
+            k_pack_input<<<(unsigned)((nx + 255) / 256), 256, 0, stream>>>((int)B, n_in, in[0], x, x0.p);
+            CK(cudaGetLastError());
+        }
         const void* a = x0.p;
         for (int l = 0; l < nl; ++l) {
             if (l + 1 < nl) {
@@ -1033,10 +1087,8 @@ int lcb_mlp_create(int device, int n_in, int width, int n_hidden, int n_out, int
         N->wsplit.alloc(nsplit);
         N->err.alloc(1);
         N->loss.alloc(1);
-        N->sub_x.alloc(B * N->in[0]);
         N->sub_yp.alloc(B * kMaxDim);
         N->sub_lz.alloc(B);
-        N->sub_chi.alloc(B);
         N->sub_lq.alloc(B);
         N->sub_lqp.alloc(B);
         N->sub_kde.alloc(2 * kMaxDim * kMaxDim);
@@ -1251,6 +1303,17 @@ int lcb_mlp_gemm(int mode, int64_t M, int64_t N, int64_t K, const void* a, const
     return guard([&] { gemm(mode, M, N, K, a, b, bias, aux, out, out2, err_dev, (cudaStream_t)stream); });
 }
 
+static void kde_propose(const StretchArgs& A, unsigned grid, int step, cudaStream_t s) {
+    switch (A.d) {
+#define LCB_KDE_D(D) \
+    case D: k_kde_propose<D><<<grid, 32 * kWalkersPerBlock, 0, s>>>(A, step); break
+        LCB_KDE_D(1); LCB_KDE_D(2); LCB_KDE_D(3); LCB_KDE_D(4);
+        LCB_KDE_D(5); LCB_KDE_D(6); LCB_KDE_D(7); LCB_KDE_D(8);
+#undef LCB_KDE_D
+        default: break;
+    }
+}
+
 int lcb_surrogate_subchain(lcb_mlp* net, int64_t n, int64_t m, int d, double* y_dev, double* ls_dev,
                            const double* comp_dev, const double* rnd_dev, int steps, double a, const double* lo,
                            const double* hi, const int* recip, const float* fmul, const float* fadd,
@@ -1280,7 +1343,7 @@ int lcb_surrogate_subchain(lcb_mlp* net, int64_t n, int64_t m, int d, double* y_
         StretchArgs A{};
         A.n = (int)n; A.m = (int)m; A.d = d; A.n_in = net->n_in;  // rows of lcb_mlp_forward input: n_in wide
         A.y = net->sub_y.p; A.ls = net->sub_ls.p; A.comp = net->sub_comp.p; A.rnd = net->sub_rnd.p;
-        A.yp = net->sub_yp.p; A.lz = net->sub_lz.p; A.xin = net->sub_x.p;
+        A.yp = net->sub_yp.p; A.lz = net->sub_lz.p; A.xin = net->x0.p; A.ld = net->in[0];
         A.lq = net->sub_lq.p; A.lqp = net->sub_lqp.p;
         A.move = move; A.rstride = rstride;
         double kde[2 * kMaxDim * kMaxDim] = {};
@@ -1315,19 +1378,13 @@ int lcb_surrogate_subchain(lcb_mlp* net, int64_t n, int64_t m, int d, double* y_
         auto enqueue = [&] {
             const unsigned g = (unsigned)((n + 127) / 128);
             const unsigned gw = (unsigned)((n + kWalkersPerBlock - 1) / kWalkersPerBlock);  // a warp per walker
-            if (move == MOVE_KDE) {
-                k_kde_logq<<<gw, 32 * kWalkersPerBlock, 0, st>>>(A);
-                CK(cudaGetLastError());
-            }
             for (int k = 0; k < steps; ++k) {
-                if (move == MOVE_KDE) k_kde_propose<<<gw, 32 * kWalkersPerBlock, 0, st>>>(A, k);
+                if (move == MOVE_KDE) kde_propose(A, gw, k, st);
                 else k_stretch_propose<<<g, 128, 0, st>>>(A, k);
                 CK(cudaGetLastError());
-                net->forward(net->sub_x.p, n, nullptr);
-                k_logflux_chisq<<<(unsigned)n, 128, 0, st>>>((int)n, net->n_out, net->pred.p, mean_dev, sd_dev,
-                                                            flux_dev, ferr_dev, scale, net->sub_chi.p);
-                CK(cudaGetLastError());
-                k_stretch_accept<<<g, 128, 0, st>>>(A, net->sub_chi.p, k);
+                net->forward(nullptr, n, nullptr);  // the proposal kernels packed its rows
+                k_chisq_accept<<<(unsigned)n, kChisqThreads, 0, st>>>(A, net->n_out, net->pred.p, mean_dev, sd_dev, flux_dev,
+                                                                     ferr_dev, scale, k);
                 CK(cudaGetLastError());
             }
         };
@@ -1408,8 +1465,8 @@ int lcb_logflux_chisq(int64_t rows, int n, const float* pred, const float* mean,
                       const double* ferr, int scale, double* chisq_out, void* stream) {
     if (rows <= 0 || n <= 0 || !pred || !mean || !sd || !flux || !ferr || !chisq_out) return LCB_ERR_INVALID;
     return guard([&] {
-        k_logflux_chisq<<<(unsigned)rows, 128, 0, (cudaStream_t)stream>>>((int)rows, n, pred, mean, sd, flux, ferr,
-                                                                          scale, chisq_out);
+        k_logflux_chisq<<<(unsigned)rows, kChisqThreads, 0, (cudaStream_t)stream>>>(n, pred, mean, sd, flux, ferr, scale,
+                                                                                    chisq_out);
         CK(cudaGetLastError());
     });
 }
