@@ -26,7 +26,9 @@
 //       EPI_BIAS_GELU  z = acc + bias; out = bf16(gelu(z)); out2 = z  (hidden layers)
 //       EPI_BIAS_F32   out = acc + bias                           (output layer)
 //       EPI_DGELU      out = bf16(acc * gelu'(aux))               (backward through GELU)
-//     the two BF16 modes optionally also write out transposed (outT).
+//       EPI_MSE        d = acc + bias - aux; out = bf16(2 d inv); loss += d^2 inv
+//                      (output layer of a training step: the gradient of the loss)
+//     the BF16 modes optionally also write out transposed (outT).
 // Every mbarrier wait is bounded; a time-out sets the error word and the CTA
 // still releases its tensor memory.
 //
@@ -70,7 +72,7 @@ constexpr uint32_t TILE_A = BM * BK * 2;
 template <int TBN>
 __host__ __device__ constexpr uint32_t tile_b() { return (uint32_t)TBN * BK * 2; }
 
-enum { EPI_F32 = 0, EPI_BIAS_GELU = 1, EPI_BIAS_F32 = 2, EPI_DGELU = 3 };
+enum { EPI_F32 = 0, EPI_BIAS_GELU = 1, EPI_BIAS_F32 = 2, EPI_DGELU = 3, EPI_MSE = 4 };
 
 template <int TBN>
 struct GemmSmem {
@@ -92,8 +94,10 @@ struct GemmArgs {
     const float* aux;
     void* out;
     void* out2;
-    void* outT;       // optional (EPI_BIAS_GELU, EPI_DGELU): bf16 copy of out, transposed (N x M)
+    void* outT;       // optional (BF16 modes): bf16 copy of out, transposed (N x M)
     int* err;
+    float inv;        // EPI_MSE: 1 / (rows x columns)
+    double* loss;     // EPI_MSE: accumulator
 };
 
 __device__ __forceinline__ uint32_t s_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -249,13 +253,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     uint8_t* stb = stage + 4096;
     auto f32_at = [&](int i, int c) { return reinterpret_cast<float4*>(stf + i * 32 + ((c ^ (i & 7)) << 2)); };
     auto b16_at = [&](int i, int c) { return reinterpret_cast<uint4*>(stb + i * 64 + ((c ^ ((i >> 1) & 3)) << 4)); };
+    float loss = 0.f;  // EPI_MSE
     if (ok && rows > 0) {
         for (int c0 = (warp >> 2) * 32; c0 < TBN && n0 + c0 < g.N; c0 += 32 * EPI_GROUPS) {
             uint32_t v[32];
             tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, v);
             const int nb = n0 + c0;
             const int nv = min(32, g.N - nb);  // multiple of 8 (N % 8 == 0)
-            if (MODE == EPI_DGELU) {  // pre-activations in, row-contiguous
+            if (MODE == EPI_DGELU || MODE == EPI_MSE) {  // pre-activations or targets in, row-contiguous
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
                     const int i = k * 4 + (lane >> 3), c = lane & 7;
@@ -286,6 +291,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                         }
                         *f32_at(lane, j >> 2) = make_float4(z[0], z[1], z[2], z[3]);
                         *f32_at(lane, (j >> 2) + 1) = make_float4(z[4], z[5], z[6], z[7]);
+                    } else if (MODE == EPI_MSE) {
+                        const float4 a0 = *f32_at(lane, j >> 2), a1 = *f32_at(lane, (j >> 2) + 1);
+                        const float tt[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+                        for (int t = 0; t < 8; ++t) {
+                            const float d = __uint_as_float(v[j + t]) + __ldg(g.bias + nb + j + t) - tt[t];
+                            y[t] = 2.f * d * g.inv;
+                            if (lane < rows) loss += d * d;
+                        }
                     } else {  // EPI_DGELU
                         const float4 a0 = *f32_at(lane, j >> 2), a1 = *f32_at(lane, (j >> 2) + 1);
                         const float zz[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
@@ -318,7 +332,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             }
             __syncwarp();
             // staging -> global, row-contiguous (8 lanes per 128-byte FP32 row, 4 per 64-byte BF16 row)
-            if (MODE != EPI_DGELU) {
+            if (MODE != EPI_DGELU && MODE != EPI_MSE) {
                 float* dst = MODE == EPI_BIAS_GELU ? reinterpret_cast<float*>(g.out2)
                                                    : reinterpret_cast<float*>(g.out) + (size_t)blockIdx.z * g.zstride;
 #pragma unroll
@@ -328,7 +342,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                         *reinterpret_cast<float4*>(dst + (size_t)(rbase + i) * g.N + nb + c * 4) = *f32_at(i, c);
                 }
             }
-            if (MODE == EPI_BIAS_GELU || MODE == EPI_DGELU) {
+            if (MODE == EPI_BIAS_GELU || MODE == EPI_DGELU || MODE == EPI_MSE) {
                 __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(g.out);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
@@ -339,6 +353,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             }
             __syncwarp();  // the staging tiles are rewritten by the next chunk
         }
+    }
+    if (MODE == EPI_MSE) {
+        for (int o = 16; o; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+        if (lane == 0 && loss != 0.f) atomicAdd(g.loss, (double)loss * g.inv);
     }
     tc_fence_before();
     __syncthreads();
@@ -356,43 +374,51 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 // ---------------------------------------------------------------------------
 // element-wise / reduction kernels
 // ---------------------------------------------------------------------------
-// out[c][r] = in[r][c] (bf16), 32 x 32 tiles through shared memory.
-__global__ void k_transpose(int rows, int cols, const uint16_t* __restrict__ in, uint16_t* __restrict__ out) {
-    __shared__ uint16_t t[32][33];
-    const int c = blockIdx.x * 32 + threadIdx.x;
-    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const int r = blockIdx.y * 32 + k;
-        t[k][threadIdx.x] = (r < rows && c < cols) ? in[(size_t)r * cols + c] : 0;
-    }
-    __syncthreads();
-    const int r2 = blockIdx.y * 32 + threadIdx.x;
-    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const int c2 = blockIdx.x * 32 + k;
-        if (c2 < cols && r2 < rows) out[(size_t)c2 * rows + r2] = t[threadIdx.x][k];
-    }
-}
-
-// out[i] = part[0][i] + part[1][i] + ... in that order: the FP32 partial products of a K-split GEMM
-// (n a multiple of 4; the order is fixed, so the sum is the same on every run).
-__global__ void k_sum_splits(int64_t n4, int splits, const float4* __restrict__ part, float4* __restrict__ out) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
-        float4 s = __ldcs(part + i);
-        for (int z = 1; z < splits; ++z) {
-            const float4 t = __ldcs(part + (int64_t)z * n4 + i);
+// The gradients of every layer in one launch.  Blocks [0, first[n]): weight
+// gradients, the FP32 partial products of a layer's K-split GEMM added in their
+// order (fixed, so the same sum on every run); layers without a split are
+// already in place.  Then one block per output of every layer: its bias
+// gradient, the sum of a row of dz^T (bf16; cols a multiple of 8), in a fixed
+// order too.  Bound by reading the partial products (out of L2 mostly).
+struct GradTab {
+    int n;                       // layers
+    int first[9];                // first block of a layer's weight sum; first[n] the first bias block
+    int row[9];                  // first bias block of a layer, after first[n]
+    int splits[8];
+    int64_t n4[8];               // float4s of a layer's weights
+    const float4* part[8];
+    float4* w[8];
+    const __nv_bfloat16* dzt[8];
+    float* b[8];
+    int cols;                    // rows of the batch
+};
+constexpr int kGradThreads = 256;
+__global__ void __launch_bounds__(kGradThreads) k_reduce_grads(GradTab T) {
+    const int blk = blockIdx.x;
+    if (blk < T.first[T.n]) {
+        int l = 0;
+        while (blk >= T.first[l + 1]) ++l;
+        const int64_t i = (int64_t)(blk - T.first[l]) * kGradThreads + threadIdx.x;
+        if (i >= T.n4[l]) return;
+        const float4* part = T.part[l] + i;
+        float4 s = __ldcs(part);
+#pragma unroll 6
+        for (int z = 1; z < T.splits[l]; ++z) {
+            const float4 t = __ldcs(part + z * T.n4[l]);
             s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
         }
-        out[i] = s;
+        T.w[l][i] = s;
+        return;
     }
-}
-
-// out[r] = sum over the columns of in[r][c] (bf16 in, fp32 out; cols a multiple of 8): one 256-thread
-// block per row, 16-byte loads, a fixed summation order.
-__global__ void __launch_bounds__(256) k_rowsum(int cols, const __nv_bfloat16* __restrict__ in, float* __restrict__ out) {
     __shared__ float red[8];
-    const uint4* row = reinterpret_cast<const uint4*>(in + (size_t)blockIdx.x * cols);
+    const int r0 = blk - T.first[T.n];
+    int l = 0;
+    while (r0 >= T.row[l + 1]) ++l;
+    const int out = r0 - T.row[l];
+    const uint4* row = reinterpret_cast<const uint4*>(T.dzt[l] + (size_t)out * T.cols);
     float s = 0.f;
 #pragma unroll 4
-    for (int c = threadIdx.x; c < cols / 8; c += 256) {
+    for (int c = threadIdx.x; c < T.cols / 8; c += kGradThreads) {
         const uint4 q = __ldg(row + c);
         const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&q);
 #pragma unroll
@@ -407,37 +433,20 @@ __global__ void __launch_bounds__(256) k_rowsum(int cols, const __nv_bfloat16* _
     if (threadIdx.x == 0) {
         float t = 0.f;
         for (int w = 0; w < 8; ++w) t += red[w];
-        out[blockIdx.x] = t;
+        T.b[l][out] = t;
     }
 }
 
-// Input rows (fp32, n_in wide) -> bf16 rows padded with zeros to ld columns.
-__global__ void k_pack_input(int rows, int n_in, int ld, const float* __restrict__ x, __nv_bfloat16* __restrict__ out) {
+// Input rows (fp32, n_in wide) -> bf16 rows padded with zeros to ld columns, and
+// with outT also transposed (ld x rows).
+__global__ void k_pack_input(int rows, int n_in, int ld, const float* __restrict__ x, __nv_bfloat16* __restrict__ out,
+                             __nv_bfloat16* __restrict__ outT) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)rows * ld) return;
     const int r = (int)(i / ld), c = (int)(i % ld);
-    out[i] = __float2bfloat16_rn(c < n_in ? x[(size_t)r * n_in + c] : 0.f);
-}
-
-// Mean-squared-error gradient: g = 2 (pred - target) / (rows * cols) as bf16;
-// loss accumulates sum (pred - target)^2 / (rows * cols).
-__global__ void k_mse_grad(int64_t n, float inv, const float* __restrict__ pred, const float* __restrict__ target,
-                           __nv_bfloat16* __restrict__ g, double* loss) {
-    __shared__ float red[32];
-    float acc = 0.f;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float d = pred[i] - target[i];
-        g[i] = __float2bfloat16_rn(2.f * d * inv);
-        acc += d * d;
-    }
-    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        float a = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.f;
-        for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (threadIdx.x == 0 && loss) atomicAdd(loss, (double)a * inv);
-    }
+    const __nv_bfloat16 h = __float2bfloat16_rn(c < n_in ? x[(size_t)r * n_in + c] : 0.f);
+    out[i] = h;
+    if (outT) outT[(size_t)c * rows + r] = h;
 }
 
 struct LayerTab {
@@ -795,6 +804,7 @@ void prepare_gemm_attributes() {
     LCB_SMEM_ATTR(EPI_DGELU, 256);
     LCB_SMEM_ATTR(EPI_F32, 32); LCB_SMEM_ATTR(EPI_BIAS_GELU, 32); LCB_SMEM_ATTR(EPI_BIAS_F32, 32);
     LCB_SMEM_ATTR(EPI_DGELU, 32);
+    LCB_SMEM_ATTR(EPI_MSE, 128); LCB_SMEM_ATTR(EPI_MSE, 256); LCB_SMEM_ATTR(EPI_MSE, 32);
 #undef LCB_SMEM_ATTR
 }
 
@@ -820,25 +830,51 @@ int max_split_count(int64_t M, int64_t N, int sms) {
     return (int)std::max<int64_t>(1, sms / tiles);
 }
 
-// splits > 1 (EPI_F32 only): split z writes its partial product to out + z * M * N.
+// Tensor maps of a network's own buffers by (pointer, rows, columns, box rows): encoding one takes the
+// host about a microsecond, a training step uses thirty.  At most kMaps, then it starts anew.
+struct MapCache {
+    static constexpr size_t kMaps = 128;
+    struct Entry {
+        const void* p;
+        int64_t rows, cols;
+        uint32_t box;
+        CUtensorMap map;
+    };
+    std::vector<Entry> entries;
+    const CUtensorMap& get(const void* p, int64_t rows, int64_t cols, uint32_t box) {
+        for (const Entry& e : entries)
+            if (e.p == p && e.rows == rows && e.cols == cols && e.box == box) return e.map;
+        if (entries.size() >= kMaps) entries.clear();
+        entries.reserve(kMaps);
+        entries.push_back({p, rows, cols, box, bf16_map(p, rows, cols, box)});
+        return entries.back().map;
+    }
+};
+
+// splits > 1 (EPI_F32 only): split z writes its partial product to out + z * M * N.  `maps`: the cache
+// of a network whose own buffers the operands are.
 void gemm(int mode, int64_t M, int64_t N, int64_t K, const void* A, const void* B, const float* bias, const float* aux,
-          void* out, void* out2, int* err, cudaStream_t s, int splits = 1, void* outT = nullptr) {
+          void* out, void* out2, int* err, cudaStream_t s, MapCache* maps = nullptr, int splits = 1, void* outT = nullptr,
+          float inv = 0.f, double* loss = nullptr) {
     if (M <= 0 || N <= 0 || K <= 0 || N % 8 || K % 8 || M > INT32_MAX || N > 65535 * (int64_t)128)
         throw Fail(LCB_ERR_INVALID, "GEMM sizes: M, N, K > 0 and N, K multiples of 8 required");
     if (((uintptr_t)out & 15) || (out2 && ((uintptr_t)out2 & 15)) || (aux && ((uintptr_t)aux & 15)))
         throw Fail(LCB_ERR_INVALID, "GEMM outputs must be 16-byte aligned");
-    if ((mode == EPI_BIAS_GELU || mode == EPI_BIAS_F32) && !bias) throw Fail(LCB_ERR_INVALID, "bias required");
+    if ((mode == EPI_BIAS_GELU || mode == EPI_BIAS_F32 || mode == EPI_MSE) && !bias) throw Fail(LCB_ERR_INVALID, "bias required");
     if (mode == EPI_BIAS_GELU && !out2) throw Fail(LCB_ERR_INVALID, "pre-activation output required");
     if (mode == EPI_DGELU && !aux) throw Fail(LCB_ERR_INVALID, "pre-activation input required");
     if (!err) throw Fail(LCB_ERR_INVALID, "error word required");
-    if (outT && ((mode != EPI_BIAS_GELU && mode != EPI_DGELU) || M % 2 || ((uintptr_t)outT & 3)))
+    if (mode == EPI_MSE && (!aux || !loss)) throw Fail(LCB_ERR_INVALID, "target and loss required");
+    if (outT && ((mode != EPI_BIAS_GELU && mode != EPI_DGELU && mode != EPI_MSE) || M % 2 || ((uintptr_t)outT & 3)))
         throw Fail(LCB_ERR_INVALID, "transposed copy: bf16 modes, even M, 4-byte aligned");
     const int nk = (int)((K + BK - 1) / BK), kchunks = (nk + splits - 1) / std::max(splits, 1);
     if (splits < 1 || (splits > 1 && mode != EPI_F32) || (nk + kchunks - 1) / kchunks != splits)
         throw Fail(LCB_ERR_INVALID, "GEMM K-split must be an FP32-output split with no empty part");
     const int width = splits == 1 && narrow_tiles(M, N) ? 2 : tile_n(N) == 256 ? 1 : 0;
-    const CUtensorMap ta = bf16_map(A, M, K, 128u), tb = bf16_map(B, N, K, width == 2 ? 32u : width ? 256u : 128u);
-    GemmArgs g{(int)M, (int)N, (int)K, kchunks, M * N, bias, aux, out, out2, outT, err};
+    const uint32_t box = width == 2 ? 32u : width ? 256u : 128u;
+    const CUtensorMap ta = maps ? maps->get(A, M, K, 128u) : bf16_map(A, M, K, 128u);
+    const CUtensorMap tb = maps ? maps->get(B, N, K, box) : bf16_map(B, N, K, box);
+    GemmArgs g{(int)M, (int)N, (int)K, kchunks, M * N, bias, aux, out, out2, outT, err, inv, loss};
     switch (mode * 3 + width) {
         case EPI_F32 * 3 + 0: launch_gemm_mode<EPI_F32, 128>(ta, tb, g, s); break;
         case EPI_F32 * 3 + 1: launch_gemm_mode<EPI_F32, 256>(ta, tb, g, s); break;
@@ -852,21 +888,11 @@ void gemm(int mode, int64_t M, int64_t N, int64_t K, const void* A, const void* 
         case EPI_DGELU * 3 + 0: launch_gemm_mode<EPI_DGELU, 128>(ta, tb, g, s); break;
         case EPI_DGELU * 3 + 1: launch_gemm_mode<EPI_DGELU, 256>(ta, tb, g, s); break;
         case EPI_DGELU * 3 + 2: launch_gemm_mode<EPI_DGELU, 32>(ta, tb, g, s); break;
+        case EPI_MSE * 3 + 0: launch_gemm_mode<EPI_MSE, 128>(ta, tb, g, s); break;
+        case EPI_MSE * 3 + 1: launch_gemm_mode<EPI_MSE, 256>(ta, tb, g, s); break;
+        case EPI_MSE * 3 + 2: launch_gemm_mode<EPI_MSE, 32>(ta, tb, g, s); break;
         default: throw Fail(LCB_ERR_INVALID, "unknown GEMM epilogue mode");
     }
-}
-
-void sum_splits(int64_t n, int splits, const float* part, float* out, cudaStream_t s) {
-    const int64_t n4 = n / 4;
-    k_sum_splits<<<(unsigned)std::min<int64_t>((n4 + 255) / 256, 1184), 256, 0, s>>>(
-        n4, splits, reinterpret_cast<const float4*>(part), reinterpret_cast<float4*>(out));
-    CK(cudaGetLastError());
-}
-
-void transpose(int64_t rows, int64_t cols, const void* in, void* out, cudaStream_t s) {
-    dim3 grid((unsigned)((cols + 31) / 32), (unsigned)((rows + 31) / 32));
-    k_transpose<<<grid, dim3(32, 8), 0, s>>>((int)rows, (int)cols, (const uint16_t*)in, (uint16_t*)out);
-    CK(cudaGetLastError());
 }
 
 template <class T>
@@ -901,10 +927,12 @@ struct lcb_mlp {
     DBuf<__nv_bfloat16> x0;           // packed input
     std::vector<DBuf<__nv_bfloat16>> y;  // hidden activations (bf16)
     std::vector<DBuf<float>> z;          // hidden pre-activations (fp32)
-    std::vector<DBuf<__nv_bfloat16>> yT; // hidden activations transposed (training only)
+    std::vector<DBuf<__nv_bfloat16>> yT; // training: hidden activations transposed, then that layer's gradient transposed
     DBuf<float> pred;
     DBuf<__nv_bfloat16> dz[2], dzt, xt;
-    DBuf<float> wsplit;               // FP32 partial products of the K-split weight-gradient GEMMs
+    MapCache maps;
+    DBuf<float> wsplit;               // FP32 partial products of the K-split weight-gradient GEMMs, layer after layer
+    std::vector<int64_t> wsplit_off;  // where each layer's start (nl + 1 entries)
     DBuf<int> err;
     DBuf<double> loss;
     DBuf<double> sub_yp, sub_lz;           // sub-chain: proposals, log proposal ratio
@@ -950,60 +978,74 @@ struct lcb_mlp {
         if (h) throw Fail(LCB_ERR_DEVICE_CHECK, "a bounded wait in the surrogate GEMM timed out");
     }
 
-    // keep_t: also store each hidden activation transposed (yT), for the weight gradients
-    void forward(const float* x, int64_t B, float* y_out, bool keep_t = false) {
+    // target: a training step's; each hidden activation and the input are then also stored transposed
+    // (the weight gradients' operands) and the output layer writes the loss gradient, dz[0] and its
+    // transpose, in place of predictions.  x null: x0 holds the packed rows already.
+    void forward(const float* x, int64_t B, float* y_out, const float* target = nullptr) {
         if (B <= 0 || B > max_batch) throw Fail(LCB_ERR_INVALID, "batch size out of range");
-        if (x) {  // else x0 holds the packed rows already
+        if (x) {
             const int64_t nx = B * in[0];
-            k_pack_input<<<(unsigned)((nx + 255) / 256), 256, 0, stream>>>((int)B, n_in, in[0], x, x0.p);
+            k_pack_input<<<(unsigned)((nx + 255) / 256), 256, 0, stream>>>((int)B, n_in, in[0], x, x0.p,
+                                                                          target ? xt.p : nullptr);
             CK(cudaGetLastError());
         }
         const void* a = x0.p;
         for (int l = 0; l < nl; ++l) {
+            const __nv_bfloat16* w = wbf.p + tab.wbf[l];
             if (l + 1 < nl) {
-                gemm(EPI_BIAS_GELU, B, out[l], in[l], a, wbf.p + tab.wbf[l], b(l), nullptr, y[l].p, z[l].p, err.p, stream,
-                     1, keep_t ? yT[l].p : nullptr);
+                gemm(EPI_BIAS_GELU, B, out[l], in[l], a, w, b(l), nullptr, y[l].p, z[l].p, err.p, stream, &maps, 1,
+                     target ? yT[l].p : nullptr);
                 a = y[l].p;
+            } else if (target) {
+                gemm(EPI_MSE, B, out[l], in[l], a, w, b(l), target, dz[0].p, nullptr, err.p, stream, &maps, 1, dzt.p,
+                     1.0f / (float)(B * n_out), loss.p);
             } else {
-                gemm(EPI_BIAS_F32, B, out[l], in[l], a, wbf.p + tab.wbf[l], b(l), nullptr, y_out ? y_out : pred.p,
-                     nullptr, err.p, stream);
+                gemm(EPI_BIAS_F32, B, out[l], in[l], a, w, b(l), nullptr, y_out ? y_out : pred.p, nullptr, err.p, stream,
+                     &maps);
             }
         }
     }
 
     void backward(const float* x, const float* target, int64_t B) {
         if (B % 8) throw Fail(LCB_ERR_INVALID, "training batch must be a multiple of 8");
-        forward(x, B, nullptr, true);
-        const int64_t npred = B * n_out;
-        CK(cudaMemsetAsync(g.p, 0, nparam * sizeof(float), stream));
-        k_mse_grad<<<(unsigned)std::min<int64_t>((npred + 255) / 256, 1184), 256, 0, stream>>>(
-            npred, 1.0f / (float)npred, pred.p, target, dz[0].p, loss.p);
-        CK(cudaGetLastError());
-        // dzt holds the current layer's output gradient transposed: made here for the last layer, then by
-        // the dGELU GEMM that produces each earlier layer's gradient
-        transpose(B, n_out, dz[0].p, dzt.p, stream);
-        int cur = 0;
+        if ((uintptr_t)target & 15) {  // the output layer reads targets 16 bytes at a time
+            CK(cudaMemcpyAsync(pred.p, target, B * n_out * sizeof(float), cudaMemcpyDeviceToDevice, stream));
+            target = pred.p;
+        }
+        forward(x, B, nullptr, target);
+        GradTab T{};
+        T.n = nl;
+        T.cols = (int)B;
+        int cur = 0, blocks = 0;
         for (int l = nl - 1; l >= 0; --l) {
+            const __nv_bfloat16* dzl = l + 1 < nl ? yT[l].p : dzt.p;  // this layer's output gradient, transposed
             const void* xlt = l > 0 ? (const void*)yT[l - 1].p : (const void*)xt.p;
-            if (l == 0) transpose(B, in[0], x0.p, xt.p, stream);
             // dW = dz^T x: K = batch is long and the output small, so K is split across the SMs
             const int ns = split_count(out[l], in[l], B, sms);
-            if (ns > 1) {
-                if ((int64_t)ns * out[l] * in[l] > (int64_t)wsplit.n) throw Fail(LCB_ERR_INVALID, "weight-gradient split workspace too small");
-                gemm(EPI_F32, out[l], in[l], B, dzt.p, xlt, nullptr, nullptr, wsplit.p, nullptr, err.p, stream, ns);
-                sum_splits((int64_t)out[l] * in[l], ns, wsplit.p, gW(l), stream);
-            } else {
-                gemm(EPI_F32, out[l], in[l], B, dzt.p, xlt, nullptr, nullptr, gW(l), nullptr, err.p, stream);
-            }
-            // db = row sums of dz^T
-            k_rowsum<<<(unsigned)out[l], 256, 0, stream>>>((int)B, dzt.p, gb(l));
-            CK(cudaGetLastError());
-            if (l > 0) {  // stream order: the GEMMs above have read dzt before this one rewrites it
+            float* part = ns > 1 ? wsplit.p + wsplit_off[l] : gW(l);
+            if (ns > 1 && (int64_t)ns * out[l] * in[l] > wsplit_off[l + 1] - wsplit_off[l])
+                throw Fail(LCB_ERR_INVALID, "weight-gradient split workspace too small");
+            gemm(EPI_F32, out[l], in[l], B, dzl, xlt, nullptr, nullptr, part, nullptr, err.p, stream, &maps, ns);
+            T.splits[l] = ns;
+            T.n4[l] = ns > 1 ? (int64_t)out[l] * in[l] / 4 : 0;
+            T.part[l] = reinterpret_cast<const float4*>(part);
+            T.w[l] = reinterpret_cast<float4*>(gW(l));
+            T.dzt[l] = dzl;
+            T.b[l] = gb(l);
+            if (l > 0) {  // stream order: the GEMM above has read yT[l - 1] before this one rewrites it
                 gemm(EPI_DGELU, B, in[l], out[l], dz[cur].p, wtbf.p + tab.wbf[l], nullptr, z[l - 1].p, dz[cur ^ 1].p,
-                     nullptr, err.p, stream, 1, dzt.p);
+                     nullptr, err.p, stream, &maps, 1, yT[l - 1].p);
                 cur ^= 1;
             }
         }
+        for (int l = 0; l < nl; ++l) {
+            T.first[l] = blocks;
+            blocks += (int)((T.n4[l] + kGradThreads - 1) / kGradThreads);
+        }
+        T.first[nl] = blocks;
+        for (int l = 0; l < nl; ++l) T.row[l + 1] = T.row[l] + out[l];
+        k_reduce_grads<<<(unsigned)(blocks + T.row[nl]), kGradThreads, 0, stream>>>(T);
+        CK(cudaGetLastError());
     }
 
     void adam(float lr, float b1, float b2, float eps, float wd) {
@@ -1079,11 +1121,14 @@ int lcb_mlp_create(int device, int n_in, int width, int n_hidden, int n_out, int
         N->pred.alloc(B * n_out);
         N->dz[0].alloc(B * wmax);
         N->dz[1].alloc(B * wmax);
-        N->dzt.alloc(B * wmax);
+        N->dzt.alloc(B * n_out);
         N->xt.alloc(B * N->in[0]);
         int64_t nsplit = 0;
-        for (int l = 0; l < N->nl; ++l)
-            nsplit = std::max(nsplit, (int64_t)max_split_count(N->out[l], N->in[l], N->sms) * N->out[l] * N->in[l]);
+        for (int l = 0; l < N->nl; ++l) {
+            N->wsplit_off.push_back(nsplit);
+            nsplit += (int64_t)max_split_count(N->out[l], N->in[l], N->sms) * N->out[l] * N->in[l];
+        }
+        N->wsplit_off.push_back(nsplit);
         N->wsplit.alloc(nsplit);
         N->err.alloc(1);
         N->loss.alloc(1);
@@ -1300,7 +1345,10 @@ int lcb_mlp_sync(lcb_mlp* net) {
 
 int lcb_mlp_gemm(int mode, int64_t M, int64_t N, int64_t K, const void* a, const void* b, const float* bias,
                  const float* aux, void* out, void* out2, int* err_dev, void* stream) {
-    return guard([&] { gemm(mode, M, N, K, a, b, bias, aux, out, out2, err_dev, (cudaStream_t)stream); });
+    return guard([&] {
+        if (mode < EPI_F32 || mode > EPI_DGELU) throw Fail(LCB_ERR_INVALID, "unknown GEMM epilogue mode");
+        gemm(mode, M, N, K, a, b, bias, aux, out, out2, err_dev, (cudaStream_t)stream);
+    });
 }
 
 static void kde_propose(const StretchArgs& A, unsigned grid, int step, cudaStream_t s) {
