@@ -249,19 +249,35 @@ __device__ __forceinline__ FaceRoot face_root(const RocheEcl& s, double ux, doub
     return FaceRoot{r, ok ? 1e-12 + 1e-13 * fmax(1.0, fabs(s.pref)) / slope : (double)INFINITY};
 }
 
+// x^(1/4): two square roots, a fifth of pow's FP64 instructions.
+__device__ __forceinline__ double fourth_root(double x) { return sqrt(sqrt(x)); }
+
+// The interval that bisecting (r, 2 r] down to a width <= acc ends with when every step is decided by
+// the root, as its middle; 0 where a step would come within `tol` of it, or the steps are too many to
+// count by exponents.  Every mid-point is a multiple of the last width from r, and the two nearest to
+// the root are that interval's ends.  (27 steps of a serial add, halve and compare before.)
+__device__ __forceinline__ double bisected(const FaceRoot& root, double r, double acc) {
+    const double x = r / acc;  // the first width is r
+    if (!(x > 1.0 && x < 1e12 && root.r > r && root.r < 2.0 * r)) return 0.0;
+    const int e = ((__double2hiint(x) >> 20) & 0x7ff) - 1023;
+    const double up = __hiloint2double((1023 + e) << 20, 0), steps = up < x ? 2.0 * up : up;  // 2^n >= x
+    const double h = r / steps, t = (root.r - r) / h, j = floor(t);
+    return (t - j) * h > root.tol && (j + 1.0 - t) * h > root.tol ? fma(j + 0.5, h, r) : 0.0;
+}
+
 // Irradiated temperature (brightness.rs:150-174) -> temp, geom.
 __device__ __forceinline__ double irradiate(double tbase, double gravity, double gdcbol, double absorb, double tirr,
                                             double mu, double r, double rirr, double& geom) {
-    double tg = tbase * pow(gravity, gdcbol);
+    double tg = gravity == 1.0 ? tbase : tbase * pow(gravity, gdcbol);  // 1 on spheres
     double tg4 = sq(tg) * sq(tg), ti4 = sq(tirr) * sq(tirr);
     if (mu >= rirr) {
         geom = sq(rirr / r) * mu;
-        return pow(tg4 + absorb * ti4 * geom, 0.25);
+        return fourth_root(tg4 + absorb * ti4 * geom);
     }
     if (mu > -rirr) {
         double x0 = -mu / rirr;
         geom = sq(rirr / r) * rirr * (sqrt(1.0 - x0 * x0) * (2.0 + x0 * x0) / 3.0 - x0 * (kPi / 2.0 - asin(x0))) / kPi;
-        return pow(tg4 + absorb * ti4 * geom, 0.25);
+        return fourth_root(tg4 + absorb * ti4 * geom);
     }
     geom = 0.0;
     return tg;
@@ -371,12 +387,15 @@ __global__ void __launch_bounds__(kElemThreads) k_elements(ElemArgs A) {
                 above = side(rlo) == 0;
                 if (above) rhi = rlo;
             }
-            for (int k = 0; k < 100 && rhi - rlo > M.acc_face; ++k) {
-                double mid = (rlo + rhi) / 2.0;
-                if (side(mid) == 1) rlo = mid;
-                else rhi = mid;
+            rad = bisected(root, rlo, M.acc_face);
+            if (rad == 0.0) {
+                for (int k = 0; k < 100 && rhi - rlo > M.acc_face; ++k) {
+                    double mid = (rlo + rhi) / 2.0;
+                    if (side(mid) == 1) rlo = mid;
+                    else rhi = mid;
+                }
+                rad = (rlo + rhi) / 2.0;
             }
-            rad = (rlo + rhi) / 2.0;
             px = cofm + rad * ux; py = rad * uy; pz = rad * uz;
             double gx, gy, gz;
             dpot_exact(primary, M.q, ssq, px, py, pz, gx, gy, gz);
@@ -481,11 +500,11 @@ __global__ void __launch_bounds__(kElemThreads) k_elements(ElemArgs A) {
         double temp, r2 = M.r2e, t4 = sq(M.tedge) * sq(M.tedge), i4 = sq(M.t2abs) * sq(M.t2abs);
         if (mu >= r2) {
             double geom = sq(r2 / r) * mu;
-            temp = pow(t4 + M.absorb_edge * i4 * geom, 0.25);
+            temp = fourth_root(t4 + M.absorb_edge * i4 * geom);
         } else if (mu > -r2) {
             double x0 = -mu / r2;
             double geom = sq(r2 / r) * r2 * (sqrt(1.0 - x0 * x0) * (2.0 + x0 * x0) / 3.0 - x0 * (kPi / 2.0 - asin(x0))) / kPi;
-            temp = pow(t4 + M.absorb_edge * i4 * geom, 0.25);
+            temp = fourth_root(t4 + M.absorb_edge * i4 * geom);
         } else {
             temp = M.tedge;
         }
