@@ -83,7 +83,7 @@ constexpr int kChopMinBlocks = LCB_CHOP_MIN_BLOCKS;  // and for its bisection ke
 #define LCB_LIMB_UNROLL 2
 #endif
 #ifndef LCB_GENERIC_UNROLL
-#define LCB_GENERIC_UNROLL 2
+#define LCB_GENERIC_UNROLL 1
 #endif
 #ifndef LCB_FLUX_MIN_BLOCKS
 #define LCB_FLUX_MIN_BLOCKS 4
@@ -1193,14 +1193,83 @@ struct Contrib {
     }
 };
 
-// FP32 LDC::imu for the beaming path (types.rs:101-119)
-__device__ __forceinline__ float imu_f(const float* l, int lt, float mu) {
-    if (mu <= 0.f) return 0.f;
-    mu = fminf(mu, 1.f);
-    float om = 1.f - mu;
-    if (lt == 0) return 1.f - om * (l[0] + om * (l[1] + om * (l[2] + om * l[3])));
-    float ms = mu * rsqrtf(mu);
-    return (1.f - (l[0] + l[1] + l[2] + l[3])) + ms * (l[0] + ms * (l[1] + ms * (l[2] + ms * l[3])));
+// 1/x of a normal x by the hardware estimate.
+__device__ __forceinline__ float rcp_normal(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// Quotients and square roots, two at a time, of arguments far from the ends of
+// the range: a hardware estimate and one Newton correction from its exact FMA
+// residual (Markstein 1990), which rounds as / and sqrtf round but for a quotient
+// within the estimate's error squared (~2^-44) of a tie: one of 2.7 10^8 random ones.
+// The general ones test each argument for the ends; the generic stars' terms are
+// bound by issue slots, and by the special-function unit where they are lensed,
+// so a square root's estimate serves the divisions by it as well.  Beaming alone,
+// 73 and 151 latitudes at 3711 sub-phases (k_flux): 0.336 -> 0.197 ms; the lensed star's
+// share of 5 million elements at 110,000 sub-phases: 351 -> 312 ms in all.
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+// a b + c d (+ e f), rounded as the compiler rounds the scalar expression.
+__device__ __forceinline__ float2 dot_pair(float2 a, float2 b, float2 c, float2 d) {
+    return __ffma2_rn(a, b, __fmul2_rn(c, d));
+}
+__device__ __forceinline__ float2 dot_pair(float2 a, float2 b, float2 c, float2 d, float2 e, float2 f) {
+    return __ffma2_rn(e, f, dot_pair(a, b, c, d));
+}
+__device__ __forceinline__ float2 div_pair(float2 a, float2 b, float2 r) {  // r: an estimate of 1 / b
+    const float2 q = __fmul2_rn(a, r);
+    return __ffma2_rn(__ffma2_rn(neg2(b), q, a), r, q);
+}
+__device__ __forceinline__ float2 sqrt_pair(float2 x, float2 y) {  // y: an estimate of 1 / sqrt(x)
+    const float2 s = __fmul2_rn(x, y);
+    return __ffma2_rn(__ffma2_rn(neg2(s), s, x), __fmul2_rn(y, make_float2(0.5f, 0.5f)), s);
+}
+
+// Lensing magnification (flux.rs:390-406) at impact parameter sqrt(p2), Einstein
+// radius squared rd.  Arguments near the ends of the range (a line of sight
+// through the lens, say) take the scalar form, a lane at a time: a call instead
+// of the loop cost beaming stars, which share this code, 40%.
+__device__ __forceinline__ float2 lens_mag_pair(float2 p2, float2 rd) {
+    const float lo = 1e-20f, hi = 1e20f;
+    if (!(fminf(p2.x, p2.y) > lo && fmaxf(p2.x, p2.y) < hi && fmaxf(rd.x, rd.y) < hi)) {  // or a NaN
+        float2 mag = p2;
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {
+            const float e = c ? rd.y : rd.x, pp = sqrtf(c ? p2.y : p2.x), phh = pp * 0.5f, phsq = phh * phh;
+            const float pd = phsq > 25.f * e ? pp + e / pp : phh + sqrtf(fmaf(phh, phh, e));
+            const float m = pd * pd / (pd - phh) / phh * 0.25f;
+            if (c) mag.y = m;
+            else mag.x = m;
+        }
+        return mag;
+    }
+    const float2 half = make_float2(0.5f, 0.5f), y = make_float2(rsqrt_normal(p2.x), rsqrt_normal(p2.y));
+    const float2 pp = sqrt_pair(p2, y), phh = __fmul2_rn(pp, half), phsq = __fmul2_rn(phh, phh);
+    float2 pd = __fadd2_rn(pp, div_pair(rd, pp, y));
+    const bool nx = !(phsq.x > 25.f * rd.x), ny = !(phsq.y > 25.f * rd.y);
+    if (nx || ny) {  // seldom: the line of sight passes within ten Einstein radii
+        const float2 in = __ffma2_rn(phh, phh, rd);
+        const float2 near = __fadd2_rn(phh, sqrt_pair(in, make_float2(rsqrt_normal(in.x), rsqrt_normal(in.y))));
+        if (nx) pd.x = near.x;
+        if (ny) pd.y = near.y;
+    }
+    const float2 b = __fadd2_rn(pd, neg2(phh));
+    const float2 q = div_pair(__fmul2_rn(pd, pd), b, make_float2(rcp_normal(b.x), rcp_normal(b.y)));
+    const float2 mag = div_pair(q, phh, __fadd2_rn(y, y));
+    return __fmul2_rn(mag, make_float2(0.25f, 0.25f));
+}
+
+// LDC::imu of two sub-phases (types.rs:101-119).
+__device__ __forceinline__ float2 imu_pair(const float (&l)[4], float sumc, int lt, float2 mu) {
+    const float2 one = make_float2(1.f, 1.f), m = make_float2(fminf(mu.x, 1.f), fminf(mu.y, 1.f));
+    const float2 l0 = make_float2(l[0], l[0]), l1 = make_float2(l[1], l[1]), l2 = make_float2(l[2], l[2]);
+    const float2 l3 = make_float2(l[3], l[3]);
+    const float2 x = lt == 0 ? __fadd2_rn(one, neg2(m)) : __fmul2_rn(m, make_float2(rsqrtf(m.x), rsqrtf(m.y)));
+    const float2 h = __ffma2_rn(x, __ffma2_rn(x, __ffma2_rn(x, l3, l2), l1), l0);
+    const float2 c = lt == 0 ? one : make_float2(1.f - sumc, 1.f - sumc);
+    const float2 im = __ffma2_rn(lt == 0 ? neg2(x) : x, h, c);
+    return make_float2(mu.x <= 0.f ? 0.f : im.x, mu.y <= 0.f ? 0.f : im.y);
 }
 
 // A unit's sub-phases are worked on in quarters of 32 n consecutive ones, n =
@@ -1361,7 +1430,8 @@ __device__ __forceinline__ void flux_unit(const FluxArgs& A, const FluxUnit& U, 
     constexpr int kPlainUnroll = KIND == UK_DISC || KIND == UK_DISC_LIN ? LCB_DISC_UNROLL : LCB_FLUX_UNROLL;
     constexpr int kTestUnroll = KIND == UK_STAR_GENERIC ? LCB_GENERIC_UNROLL : LCB_LIMB_UNROLL;
     // generic-path constants
-    const float* ldg = U.star == 1 ? M.ld1f : M.ld2f;
+    const float ldc[4] = {C.a0, C.a1, C.a2, C.a3};
+    const float vfac = M.vfacf, xcofm = M.xcofmf, rlens = M.rlens1f;
     const int ltg = U.star == 1 ? M.ltype1 : M.ltype2;
     const float beam = U.star == 1 ? M.beam1f : M.beam2f;
     const float spin = U.star == 1 ? M.spin1f : M.spin2f;
@@ -1478,34 +1548,36 @@ __device__ __forceinline__ void flux_unit(const FluxArgs& A, const FluxUnit& U, 
                         if (KIND == UK_STAR_GENERIC) {
                             const float4 p = __ldg(A.el_pos + U.e0 + g * 32 + i + n);
                             float vx, vy;
-                            if (U.star == 1) { vx = -M.vfacf * spin * p.y; vy = M.vfacf * (spin * p.x - M.xcofmf); }
-                            else { vx = -M.vfacf * spin * p.y; vy = M.vfacf * (spin * (p.x - 1.f) + 1.f - M.xcofmf); }
+                            if (U.star == 1) { vx = -vfac * spin * p.y; vy = vfac * (spin * p.x - xcofm); }
+                            else { vx = -vfac * spin * p.y; vy = vfac * (spin * (p.x - 1.f) + 1.f - xcofm); }
                             const float vn = r.x * vx + r.y * vy;
+                            const float2 rx = make_float2(r.x, r.x), ry = make_float2(r.y, r.y), rz = make_float2(r.z, r.z);
+                            const float2 px = make_float2(p.x, p.x), py = make_float2(p.y, p.y), pz = make_float2(p.z, p.z);
 #pragma unroll
-                            for (int k = 0; k < kFluxR; ++k) {
-                                float& sum = (k & 1) ? part[k / 2].y : part[k / 2].x;
-                                float mu = ex[k] * r.x + ey[k] * r.y + ez[k] * r.z;
-                                bool v = mu > C.thr && !((hid >> k) & 1u);
-                                if (v) {
-                                    float mag = 1.f;
-                                    if (lens) {
-                                        float d = -(p.x * ex[k] + p.y * ey[k] + p.z * ez[k]);
-                                        if (d > 0.f) {
-                                            float ax = p.x + d * ex[k], ay = p.y + d * ey[k], az = p.z + d * ez[k];
-                                            float pp = sqrtf(ax * ax + ay * ay + az * az), phh = pp * 0.5f, phsq = phh * phh;
-                                            float rd = M.rlens1f * d;
-                                            float pd = phsq > 25.f * rd ? pp + rd / pp : phh + sqrtf(phsq + rd);
-                                            mag = pd * pd / (pd - phh) / phh * 0.25f;
-                                        }
-                                    }
-                                    if (beam != 0.f) {
-                                        float vr = -(ex[k] * vx + ey[k] * vy);
-                                        float mud = mu - mu * vr - vn;
-                                        sum += mu * mag * r.w * (1.f - beam * vr) * imu_f(ldg, ltg, mud);
-                                    } else {
-                                        sum += mu * mag * r.w * imu_f(ldg, ltg, mu);
-                                    }
+                            for (int k = 0; k < kFluxR / 2; ++k) {
+                                const float2 mu = dot_pair(ex2[k], rx, ey2[k], ry, ez2[k], rz);
+                                const bool sx = mu.x > C.thr && !((hid >> (2 * k)) & 1u);
+                                const bool sy = mu.y > C.thr && !((hid >> (2 * k + 1)) & 1u);
+                                if (!(sx || sy)) continue;
+                                float2 t = mu, im = mu;
+                                if (lens) {
+                                    const float2 d = neg2(dot_pair(px, ex2[k], py, ey2[k], pz, ez2[k]));
+                                    const float2 ax = __ffma2_rn(d, ex2[k], px), ay = __ffma2_rn(d, ey2[k], py), az = __ffma2_rn(d, ez2[k], pz);
+                                    const float2 p2 = dot_pair(ax, ax, ay, ay, az, az);
+                                    float2 mag = lens_mag_pair(p2, __fmul2_rn(make_float2(rlens, rlens), d));
+                                    if (!(d.x > 0.f)) mag.x = 1.f;
+                                    if (!(d.y > 0.f)) mag.y = 1.f;
+                                    t = __fmul2_rn(mu, mag);
                                 }
+                                t = __fmul2_rn(t, make_float2(r.w, r.w));
+                                if (beam != 0.f) {
+                                    const float2 vr = neg2(dot_pair(ex2[k], make_float2(vx, vx), ey2[k], make_float2(vy, vy)));
+                                    im = __fadd2_rn(__ffma2_rn(neg2(mu), vr, mu), make_float2(-vn, -vn));
+                                    t = __fmul2_rn(t, __ffma2_rn(make_float2(-beam, -beam), vr, make_float2(1.f, 1.f)));
+                                }
+                                const float2 sum = __ffma2_rn(t, imu_pair(ldc, C.sumc, ltg, im), part[k]);
+                                if (sx) part[k].x = sum.x;
+                                if (sy) part[k].y = sum.y;
                             }
                         } else {
 #pragma unroll
