@@ -646,7 +646,7 @@ def main():
         "spot_stream": spot,
         "cpu_baseline": cpu,
         "e2e": e2e,
-        "gpu_launches": 6 * args.steps,
+        "gpu_launches": 9 * args.steps,  # k_phase, k_elements, k_roche, _open, _chop2, k_aux, k_flux, k_curve, k_results
         "clocks": clk.summary(),
         "mcmc": mcmc if mcmc is not None else {"skipped": "multi-GPU run or --no-mcmc; the MCMC comparison runs on 1 GPU"},
     }

@@ -207,15 +207,18 @@ int  lcb_batch_results(lcb_batch* b, double* chisq_out, double* calc_out, lcb_re
 int  lcb_batch_stats(const lcb_batch* b, int64_t* out8);
 /* Eclipse-search counters of the last run: [potential evaluations, gradient
  * evaluations, line-of-sight searches, miss-proof nodes (a potential and a
- * gradient evaluation each), successful miss proofs (one line of sight, or one
- * block of consecutive phase-scan steps proven together)].  The line-of-sight
- * searches are exactly the reference path's (eclipse.rs:123-197 calls). */
+ * gradient evaluation each), successful miss proofs (one line of sight, one
+ * block of consecutive phase-scan steps proven together, or one side of an
+ * element's eclipse bounded by a limb contact)].  The line-of-sight searches
+ * are exactly the reference path's (eclipse.rs:123-197 calls), made or stood
+ * for by a proof. */
 int  lcb_batch_search_counts(const lcb_batch* b, int64_t* out5);
 /* Launch-shape choices of a resident batch, for an autotuner (no reference
  * counterpart; the reference GPU crate launches one fixed shape, 256-thread
  * blocks, crates/lcurve-cuda/kernels/flux_kernel.cu:81, 543-545): elements
  * per flux work unit in chunks of 256 (1..16), threads per Roche-eclipsed
- * element in the phase scan (1..16; only where the batch has such elements)
+ * element in the general phase scan (1..16; it runs only for elements whose
+ * eclipse the limb contacts leave undecided)
  * and persistent flux blocks per SM (>= 1, capped at the occupancy limit);
  * 0 keeps the planner's heuristic for that choice.  Re-plans the batch;
  * results are unchanged up to the FP32 summation order of the flux sum.
@@ -228,7 +231,7 @@ int  lcb_batch_get_tuning(const lcb_batch* b, int* out3);
 int  lcb_batch_profile(lcb_batch* b, int scale);
 /* Device time (ms) of each stage of the last lcb_batch_profile, measured with
  * CUDA events on the launching stream: [phase, elements (grid + continuum +
- * analytic eclipses), roche (FP64 ray-march), aux (per-model sums), flux,
+ * analytic eclipses), roche (FP64 eclipse search), aux (per-model sums), flux,
  * epilogue]. */
 int  lcb_batch_stage_ms(const lcb_batch* b, double* out6);
 
@@ -258,7 +261,7 @@ int lcb_stream_points(lcb_ctx* ctx, const double* q, const double* radius, int64
  * lcb_ctx_set_search_cap lowers that bound for the context's later calls
  * (0 restores the default), so the failure path can be exercised.
  * lcb_wait_probe runs one block that waits on a barrier nothing completes,
- * with the same bounded wait the flux kernel's copy pipeline uses, limited to
+ * with a bounded mbarrier wait of at most
  * limit_cycles SM cycles (<= 4e9); it returns LCB_ERR_DEVICE_CHECK when the
  * wait gives up, as it must, and leaves the context usable. */
 int lcb_ctx_set_search_cap(lcb_ctx* ctx, int evals);

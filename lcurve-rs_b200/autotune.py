@@ -1,8 +1,8 @@
 """Autotuner of a resident batch's launch shapes, with a JSON cache.
 
 The planner picks three launch-shape choices by heuristic: elements per flux
-work unit (in chunks of 256), threads per Roche-eclipsed element in the
-phase scan, and persistent flux blocks per SM (lcb_batch_set_tuning in
+work unit (in chunks of 256), threads per element of the general
+eclipse scan, and persistent flux blocks per SM (lcb_batch_set_tuning in
 lcurve_b200.h).  `autotune` times candidates for each choice on the batch
 itself -- one warm-up evaluation, then the device time of `repeats`
 evaluations from the library's per-stage CUDA events (Batch.profile) -- one

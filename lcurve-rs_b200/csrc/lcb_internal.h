@@ -176,7 +176,7 @@ struct FluxUnit {
 constexpr int kFluxThreads = 128;
 constexpr int kFluxR = 4;                          // sub-phases per thread
 constexpr int kFluxTile = kFluxThreads * kFluxR;   // sub-phases per work unit
-constexpr int kFluxChunk = 256;                    // elements staged per TMA chunk
+constexpr int kFluxChunk = 256;                    // elements of a chunk: its FP32 blocks of 32 start anew
 constexpr int kElemThreads = 256;
 #ifndef LCB_ROCHE_BLOCK
 #define LCB_ROCHE_BLOCK 128

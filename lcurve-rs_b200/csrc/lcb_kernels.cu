@@ -20,15 +20,15 @@
 //   k_aux      : per star element, the per-model FP64 sums of ginterp,
 //                wdwarf, log g and radii (flux.rs:115-206, 288-373).
 //   k_flux     : persistent FP32 flux sum (flux.rs:7-111) over work units of
-//                (element range x 512 sub-phases).  Element chunks arrive in
-//                shared memory by cp.async.bulk (TMA) double buffering; a
-//                classification pass lists each chunk's contributing
-//                elements; each thread keeps 4 sub-phases in registers, in
-//                pairs on the packed FP32x2 pipe, and accumulates in FP32
-//                blocks of 32 elements folded into a two-sum pair.
-//                Visibility is decided exactly in FP64 per (element, tile)
-//                and per sub-phase only where an eclipse edge falls inside
-//                the tile.
+//                (element range x 512 sub-phases), a block's or a warp's each.
+//                A first pass sorts the unit's elements into bit masks per
+//                quarter of the tile's sub-phases: out of sight, plain, on the
+//                limb, partly eclipsed; the sums then run over the masks, each
+//                thread with 4 sub-phases in registers, in pairs on the packed
+//                FP32x2 pipe, in FP32 blocks of 32 elements folded into a
+//                two-sum pair.  Visibility is decided exactly in FP64 per
+//                (element, tile) and per sub-phase only where an eclipse edge
+//                falls inside the tile.
 //   k_curve    : per datum, the slots' partial sums under the ginterp scale
 //                factors, exposure smearing, slope/third (orchestration.rs:
 //                243-310), in tiles of 32 data per block.
@@ -255,7 +255,8 @@ __device__ __forceinline__ double fourth_root(double x) { return sqrt(sqrt(x)); 
 // The interval that bisecting (r, 2 r] down to a width <= acc ends with when every step is decided by
 // the root, as its middle; 0 where a step would come within `tol` of it, or the steps are too many to
 // count by exponents.  Every mid-point is a multiple of the last width from r, and the two nearest to
-// the root are that interval's ends.  (27 steps of a serial add, halve and compare before.)
+// the root are that interval's ends.  In place of ~27 steps of a serial add, halve and compare: with the
+// fourth roots, k_elements of 1024 models 16.1 -> 14.5 ms.
 __device__ __forceinline__ double bisected(const FaceRoot& root, double r, double acc) {
     const double x = r / acc;  // the first width is r
     if (!(x > 1.0 && x < 1e12 && root.r > r && root.r < 2.0 * r)) return 0.0;
@@ -538,7 +539,7 @@ __global__ void __launch_bounds__(kElemThreads) k_elements(ElemArgs A) {
 }
 
 // ---------------------------------------------------------------------------
-// k_roche: FP64 Roche ray-march of one element per thread (eclipse.rs:270-373)
+// k_roche: eclipses by a Roche star (eclipse.rs:270-373), two threads an element
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void roche_counters(const ElemArgs& A, const EclCount& cnt);
 
@@ -565,6 +566,8 @@ __device__ __forceinline__ void group_or_warp(unsigned* grp, int64_t g, unsigned
 // convex, elements near the bounding sphere, grazes narrower than the margins)
 // go to a list that k_roche_open and k_roche_chop2 take.  Bound by FP64 latency
 // and issue: ~12 contact nodes and ~6 searches an element of ~10 evaluations.
+// 43 million elements (1024 models): 200 -> 50.6 ms, 92 evaluations an element
+// instead of ~850; one model of 5,000 elements: 0.267 -> 0.064 ms.
 __global__ void __launch_bounds__(kRocheBlock, kRocheMinBlocks) k_roche(ElemArgs A) {
     const int64_t rb = blockIdx.x >> 1;
     const int slot = (int)(blockIdx.x & 1) * (kRocheBlock / 2) + (int)(threadIdx.x >> 1);
@@ -936,7 +939,7 @@ __global__ void k_phase(PhaseArgs A) {
 }
 
 // ---------------------------------------------------------------------------
-// k_flux
+// bounded waits
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 

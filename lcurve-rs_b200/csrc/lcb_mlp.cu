@@ -810,9 +810,9 @@ void prepare_gemm_attributes() {
 
 int tile_n(int64_t N) { return N >= 256 ? 256 : 128; }  // 128 x 256 tiles where N allows
 // ... unless they fill less than an eighth of the SMs: then 128 x 32 tiles, whose epilogue (a GELU of
-// every element) is spread over up to eight times the SMs.  128 x 512 x 512 with GELU: 16 us on two
-// CTAs of 128 x 256, 5 us on sixteen of 128 x 32; at 8 and more row tiles the wide ones win (the
-// operands are read once per tile).
+// every element) is spread over up to eight times the SMs.  Two moves of 128 walkers, ten layers on
+// two CTAs each at 13 to 16 us, took 271 us a call, on sixteen CTAs 180 us; past that line the wide
+// tiles' operands, read once per tile, and their full wave are worth more.
 bool narrow_tiles(int64_t M, int64_t N) {
     return ((M + BM - 1) / BM) * ((N + tile_n(N) - 1) / tile_n(N)) * 8 < 148;
 }
@@ -1008,6 +1008,7 @@ struct lcb_mlp {
 
     void backward(const float* x, const float* target, int64_t B) {
         if (B % 8) throw Fail(LCB_ERR_INVALID, "training batch must be a multiple of 8");
+        if (B <= 0 || B > max_batch) throw Fail(LCB_ERR_INVALID, "batch size out of range");
         if ((uintptr_t)target & 15) {  // the output layer reads targets 16 bytes at a time
             CK(cudaMemcpyAsync(pred.p, target, B * n_out * sizeof(float), cudaMemcpyDeviceToDevice, stream));
             target = pred.p;
