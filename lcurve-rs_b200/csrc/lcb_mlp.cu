@@ -9,18 +9,16 @@
 //
 // GEMM kernel (k_gemm): C[M x N] = A[M x K] . B[N x K]^T, both operands BF16
 // row-major (K contiguous), FP32 accumulation in tensor memory:
-//   - one CTA per 128 x TBN output tile (TBN = 256 when N >= 256, else 128; 32
-//     where those would leave most SMs idle), sixteen warps; a K-split grid
-//     (blockIdx.z) for FP32 outputs;
+//   - one CTA per 128 x TBN output tile, TBN from 32 to 256 by the number of
+//     tiles; a K-split grid (blockIdx.z) for FP32 outputs;
 //   - warp 0 lane 0 streams 64-wide K-slices of A and B into shared memory
-//     with TMA (cp.async.bulk.tensor, 128-byte swizzle), four stages on
-//     mbarriers;
+//     with TMA (cp.async.bulk.tensor, 128-byte swizzle), three or four stages
+//     on mbarriers;
 //   - warp 1 lane 0 issues tcgen05.mma (kind::f16, M=128, N=TBN, K=16) from
 //     shared-memory descriptors into a TBN-column TMEM accumulator, and
 //     releases each stage with tcgen05.commit;
 //   - every warp reads the accumulator back with tcgen05.ld (warp w: TMEM
-//     lanes 32 (w % 4) .. + 31 = tile rows, every fourth 32-column chunk from
-//     w / 4), applies the fused epilogue and stages each 32 x 32 chunk in the
+//     lanes 32 (w % 4) .. + 31 = tile rows, 32-column chunks from w / 4 on), applies the fused epilogue and stages each 32 x 32 chunk in the
 //     idle operand buffers so the global stores are row-contiguous:
 //       EPI_F32        out = acc                                  (weight gradients)
 //       EPI_BIAS_GELU  z = acc + bias; out = bf16(gelu(z)); out2 = z  (hidden layers)
@@ -62,12 +60,17 @@ namespace {
 // ---------------------------------------------------------------------------
 // device helpers
 // ---------------------------------------------------------------------------
-// Tiles: 128 rows x TBN columns (TBN = 256 when N allows: half the CTAs, the
-// widest single-CTA MMA; 128 otherwise), K-slices of 64.
-// 16 warps: warp 0 lane 0 issues the TMA copies, warp 1 lane 0 the MMAs; in the epilogue warp w
+// Tiles: 128 rows x TBN columns, K-slices of 64.  TBN up to 128: eight warps and three stages
+// (98 KB, 128 registers), so that two CTAs share an SM and one's copies and MMAs run under the
+// other's epilogue; TBN = 256: sixteen warps and four stages, an SM each.
+// Warp 0 lane 0 issues the TMA copies, warp 1 lane 0 the MMAs; in the epilogue warp w
 // reads TMEM lanes 32 (w % 4) .. + 31 (the quarter its warp id may access) and the column
-// chunks w / 4, w / 4 + 4, ... of 32.
-constexpr int BM = 128, BK = 64, STAGES = 4, GEMM_THREADS = 512, EPI_GROUPS = GEMM_THREADS / 128;
+// chunks w / 4, w / 4 + threads / 128, ... of 32.
+constexpr int BM = 128, BK = 64;
+template <int TBN>
+__host__ __device__ constexpr int gemm_threads() { return TBN == 256 ? 512 : 256; }
+template <int TBN>
+__host__ __device__ constexpr int gemm_stages() { return TBN == 256 ? 4 : 3; }
 constexpr uint32_t TILE_A = BM * BK * 2;
 template <int TBN>
 __host__ __device__ constexpr uint32_t tile_b() { return (uint32_t)TBN * BK * 2; }
@@ -76,6 +79,7 @@ enum { EPI_F32 = 0, EPI_BIAS_GELU = 1, EPI_BIAS_F32 = 2, EPI_DGELU = 3, EPI_MSE 
 
 template <int TBN>
 struct GemmSmem {
+    static constexpr int STAGES = gemm_stages<TBN>();
     uint8_t a[STAGES][TILE_A];  // 1024-byte aligned slices (128-byte swizzle atoms)
     uint8_t b[STAGES][tile_b<TBN>()];
     uint64_t full[STAGES], empty[STAGES], done;
@@ -83,8 +87,12 @@ struct GemmSmem {
     int abort;
 };
 // the epilogue's per-warp staging (6 KB a warp that has columns) reuses a[] and b[]
-static_assert((GEMM_THREADS / 32) * 6144 <= STAGES * (TILE_A + tile_b<128>()), "epilogue staging");
-static_assert(4 * 6144 <= STAGES * TILE_A, "epilogue staging of one column chunk");
+template <int TBN>
+constexpr bool staging_fits() {
+    const int warps = 4 * (TBN / 32 < gemm_threads<TBN>() / 128 ? TBN / 32 : gemm_threads<TBN>() / 128);
+    return warps * 6144 <= gemm_stages<TBN>() * (int)(TILE_A + tile_b<TBN>());
+}
+static_assert(staging_fits<32>() && staging_fits<64>() && staging_fits<128>() && staging_fits<256>(), "epilogue staging");
 
 struct GemmArgs {
     int M, N, K;
@@ -180,11 +188,12 @@ __device__ __forceinline__ float dgelu(float z) {
 // k_gemm
 // ---------------------------------------------------------------------------
 template <int MODE, int TBN>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+__global__ void __launch_bounds__(gemm_threads<TBN>(), TBN == 256 ? 1 : 2)
     k_gemm(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, GemmArgs g) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = s_u32(smem_raw);
     GemmSmem<TBN>& S = *reinterpret_cast<GemmSmem<TBN>*>(smem_raw + (((raw + 1023u) & ~1023u) - raw));
+    constexpr int STAGES = gemm_stages<TBN>(), EPI_GROUPS = gemm_threads<TBN>() / 128;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = blockIdx.x * BM, n0 = blockIdx.y * TBN;
     const int kb = blockIdx.z * g.kchunks;                           // first K-chunk of this split
@@ -789,8 +798,16 @@ void launch_gemm_mode(const CUtensorMap& ta, const CUtensorMap& tb, const GemmAr
         cudaFuncSetAttribute(k_gemm<MODE, TBN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem<TBN>());
     CK(attr);
     dim3 grid((g.M + BM - 1) / BM, (g.N + TBN - 1) / TBN, (unsigned)(((g.K + BK - 1) / BK + g.kchunks - 1) / g.kchunks));
-    k_gemm<MODE, TBN><<<grid, GEMM_THREADS, gemm_smem<TBN>(), s>>>(ta, tb, g);
+    k_gemm<MODE, TBN><<<grid, gemm_threads<TBN>(), gemm_smem<TBN>(), s>>>(ta, tb, g);
     CK(cudaGetLastError());
+}
+
+template <int MODE>
+void launch_gemm(int cols, const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, cudaStream_t s) {
+    if (cols == 32) launch_gemm_mode<MODE, 32>(ta, tb, g, s);
+    else if (cols == 64) launch_gemm_mode<MODE, 64>(ta, tb, g, s);
+    else if (cols == 128) launch_gemm_mode<MODE, 128>(ta, tb, g, s);
+    else launch_gemm_mode<MODE, 256>(ta, tb, g, s);
 }
 
 // Sets the dynamic shared-memory limit of every GEMM variant (needed before a
@@ -798,35 +815,39 @@ void launch_gemm_mode(const CUtensorMap& ta, const CUtensorMap& tb, const GemmAr
 void prepare_gemm_attributes() {
 #define LCB_SMEM_ATTR(M, T) \
     CK(cudaFuncSetAttribute(k_gemm<M, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem<T>()))
-    LCB_SMEM_ATTR(EPI_F32, 128); LCB_SMEM_ATTR(EPI_BIAS_GELU, 128); LCB_SMEM_ATTR(EPI_BIAS_F32, 128);
-    LCB_SMEM_ATTR(EPI_DGELU, 128);
-    LCB_SMEM_ATTR(EPI_F32, 256); LCB_SMEM_ATTR(EPI_BIAS_GELU, 256); LCB_SMEM_ATTR(EPI_BIAS_F32, 256);
-    LCB_SMEM_ATTR(EPI_DGELU, 256);
-    LCB_SMEM_ATTR(EPI_F32, 32); LCB_SMEM_ATTR(EPI_BIAS_GELU, 32); LCB_SMEM_ATTR(EPI_BIAS_F32, 32);
-    LCB_SMEM_ATTR(EPI_DGELU, 32);
-    LCB_SMEM_ATTR(EPI_MSE, 128); LCB_SMEM_ATTR(EPI_MSE, 256); LCB_SMEM_ATTR(EPI_MSE, 32);
+#define LCB_SMEM_ATTRS(M) LCB_SMEM_ATTR(M, 32); LCB_SMEM_ATTR(M, 64); LCB_SMEM_ATTR(M, 128); LCB_SMEM_ATTR(M, 256)
+    LCB_SMEM_ATTRS(EPI_F32); LCB_SMEM_ATTRS(EPI_BIAS_GELU); LCB_SMEM_ATTRS(EPI_BIAS_F32);
+    LCB_SMEM_ATTRS(EPI_DGELU); LCB_SMEM_ATTRS(EPI_MSE);
+#undef LCB_SMEM_ATTRS
 #undef LCB_SMEM_ATTR
 }
 
-int tile_n(int64_t N) { return N >= 256 ? 256 : 128; }  // 128 x 256 tiles where N allows
-// ... unless they fill less than an eighth of the SMs: then 128 x 32 tiles, whose epilogue (a GELU of
-// every element) is spread over up to eight times the SMs.  Two moves of 128 walkers, ten layers on
-// two CTAs each at 13 to 16 us, took 271 us a call, on sixteen CTAs 180 us; past that line the wide
-// tiles' operands, read once per tile, and their full wave are worth more.
-bool narrow_tiles(int64_t M, int64_t N) {
-    return ((M + BM - 1) / BM) * ((N + tile_n(N) - 1) / tile_n(N)) * 8 < 148;
-}
+int64_t tiles_of(int64_t M, int64_t N, int cols) { return ((M + BM - 1) / BM) * ((N + cols - 1) / cols); }
 
+// Columns of a GEMM's tiles.  The narrowest of 32, 64 and 128 whose tiles an SM each can hold: a GELU of
+// every element makes the epilogue the longest part, and narrow tiles spread it (one training step at 128 x
+// 512 to 4096 x 512: 2 to 27% less time than with tiles of 128; allowed up to two tiles per SM they were
+// 2.5% slower, up to half of one 15%).  128 with two CTAs per SM took 5% less than 256 with one
+// where K <= 512 (8192 rows 292 -> 278 us a step, three networks at once 198 -> 182); long sums of
+// many tiles read their operands too often that way (K = 1024: 667 against 576 TFLOP/s, K = 4096: 1038
+// against 945), so they keep tiles of 256.
+constexpr int kSplitCols = 128;  // K-split GEMMs
+int tile_cols(int64_t M, int64_t N, int64_t K) {
+    constexpr int kSms = 148;
+    for (int cols = 32; cols < 128; cols *= 2)
+        if (tiles_of(M, N, cols) <= kSms) return cols;
+    return K >= 1024 && N >= 256 && tiles_of(M, N, 128) > 2 * kSms ? 256 : 128;
+}
 // Number of K-splits for an FP32-output GEMM: enough CTAs to cover `sms` SMs, none of them empty.
 int split_count(int64_t M, int64_t N, int64_t K, int sms) {
-    const int64_t tiles = ((M + BM - 1) / BM) * ((N + tile_n(N) - 1) / tile_n(N)), nk = (K + BK - 1) / BK;
+    const int64_t tiles = tiles_of(M, N, kSplitCols), nk = (K + BK - 1) / BK;
     const int64_t s = std::max<int64_t>(1, std::min<int64_t>(sms / tiles, nk)), kc = (nk + s - 1) / s;
     return (int)((nk + kc - 1) / kc);
 }
 
 // Upper bound of split_count(M, N, K, sms) over every K.
 int max_split_count(int64_t M, int64_t N, int sms) {
-    const int64_t tiles = ((M + BM - 1) / BM) * ((N + tile_n(N) - 1) / tile_n(N));
+    const int64_t tiles = tiles_of(M, N, kSplitCols);
     return (int)std::max<int64_t>(1, sms / tiles);
 }
 
@@ -870,27 +891,16 @@ void gemm(int mode, int64_t M, int64_t N, int64_t K, const void* A, const void* 
     const int nk = (int)((K + BK - 1) / BK), kchunks = (nk + splits - 1) / std::max(splits, 1);
     if (splits < 1 || (splits > 1 && mode != EPI_F32) || (nk + kchunks - 1) / kchunks != splits)
         throw Fail(LCB_ERR_INVALID, "GEMM K-split must be an FP32-output split with no empty part");
-    const int width = splits == 1 && narrow_tiles(M, N) ? 2 : tile_n(N) == 256 ? 1 : 0;
-    const uint32_t box = width == 2 ? 32u : width ? 256u : 128u;
+    const int cols = splits > 1 ? kSplitCols : tile_cols(M, N, K);
     const CUtensorMap ta = maps ? maps->get(A, M, K, 128u) : bf16_map(A, M, K, 128u);
-    const CUtensorMap tb = maps ? maps->get(B, N, K, box) : bf16_map(B, N, K, box);
+    const CUtensorMap tb = maps ? maps->get(B, N, K, (uint32_t)cols) : bf16_map(B, N, K, (uint32_t)cols);
     GemmArgs g{(int)M, (int)N, (int)K, kchunks, M * N, bias, aux, out, out2, outT, err, inv, loss};
-    switch (mode * 3 + width) {
-        case EPI_F32 * 3 + 0: launch_gemm_mode<EPI_F32, 128>(ta, tb, g, s); break;
-        case EPI_F32 * 3 + 1: launch_gemm_mode<EPI_F32, 256>(ta, tb, g, s); break;
-        case EPI_F32 * 3 + 2: launch_gemm_mode<EPI_F32, 32>(ta, tb, g, s); break;
-        case EPI_BIAS_GELU * 3 + 0: launch_gemm_mode<EPI_BIAS_GELU, 128>(ta, tb, g, s); break;
-        case EPI_BIAS_GELU * 3 + 1: launch_gemm_mode<EPI_BIAS_GELU, 256>(ta, tb, g, s); break;
-        case EPI_BIAS_GELU * 3 + 2: launch_gemm_mode<EPI_BIAS_GELU, 32>(ta, tb, g, s); break;
-        case EPI_BIAS_F32 * 3 + 0: launch_gemm_mode<EPI_BIAS_F32, 128>(ta, tb, g, s); break;
-        case EPI_BIAS_F32 * 3 + 1: launch_gemm_mode<EPI_BIAS_F32, 256>(ta, tb, g, s); break;
-        case EPI_BIAS_F32 * 3 + 2: launch_gemm_mode<EPI_BIAS_F32, 32>(ta, tb, g, s); break;
-        case EPI_DGELU * 3 + 0: launch_gemm_mode<EPI_DGELU, 128>(ta, tb, g, s); break;
-        case EPI_DGELU * 3 + 1: launch_gemm_mode<EPI_DGELU, 256>(ta, tb, g, s); break;
-        case EPI_DGELU * 3 + 2: launch_gemm_mode<EPI_DGELU, 32>(ta, tb, g, s); break;
-        case EPI_MSE * 3 + 0: launch_gemm_mode<EPI_MSE, 128>(ta, tb, g, s); break;
-        case EPI_MSE * 3 + 1: launch_gemm_mode<EPI_MSE, 256>(ta, tb, g, s); break;
-        case EPI_MSE * 3 + 2: launch_gemm_mode<EPI_MSE, 32>(ta, tb, g, s); break;
+    switch (mode) {
+        case EPI_F32: launch_gemm<EPI_F32>(cols, ta, tb, g, s); break;
+        case EPI_BIAS_GELU: launch_gemm<EPI_BIAS_GELU>(cols, ta, tb, g, s); break;
+        case EPI_BIAS_F32: launch_gemm<EPI_BIAS_F32>(cols, ta, tb, g, s); break;
+        case EPI_DGELU: launch_gemm<EPI_DGELU>(cols, ta, tb, g, s); break;
+        case EPI_MSE: launch_gemm<EPI_MSE>(cols, ta, tb, g, s); break;
         default: throw Fail(LCB_ERR_INVALID, "unknown GEMM epilogue mode");
     }
 }

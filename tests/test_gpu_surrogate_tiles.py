@@ -17,9 +17,12 @@ def _ptr(t):
     return C.c_void_p(t.data_ptr()) if t is not None else None
 
 
-# 128-row tiles x wide tiles of 128 or 256 columns: fewer than 19 take narrow ones of 32
+# 128-row tiles of 32 columns up to 148 of them, then 64, then 128; 256 for many tiles of long sums
 @pytest.mark.parametrize("M,N,K", [(1, 8, 8), (128, 512, 512), (129, 40, 72), (127, 232, 320), (18 * 128, 24, 64),
-                                   (18 * 128 + 1, 24, 64), (9 * 128, 264, 136), (9 * 128 + 2, 264, 136)])
+                                   (18 * 128 + 1, 24, 64), (9 * 128, 264, 136), (9 * 128 + 2, 264, 136),
+                                   (37 * 128, 128, 64), (37 * 128 + 1, 128, 64),  # 148 tiles of 32, 149 of 32
+                                   (1283, 504, 200), (37 * 128, 256, 8), (37 * 128 + 5, 256, 8),  # 64, and past it
+                                   (2435, 1000, 72), (37 * 128, 1024, 1024), (5119, 1000, 1032)])  # 128, 128, 256
 def test_gemm_tile_edges(lcb, M, N, K):
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     A = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
