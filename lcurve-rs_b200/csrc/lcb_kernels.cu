@@ -1235,7 +1235,7 @@ __device__ __forceinline__ float2 sqrt_pair(float2 x, float2 y) {  // y: an esti
 // of the loop cost beaming stars, which share this code, 40%.
 __device__ __forceinline__ float2 lens_mag_pair(float2 p2, float2 rd) {
     const float lo = 1e-20f, hi = 1e20f;
-    if (!(fminf(p2.x, p2.y) > lo && fmaxf(p2.x, p2.y) < hi && fmaxf(rd.x, rd.y) < hi)) {  // or a NaN
+    if (!(fminf(p2.x, p2.y) > lo && fmaxf(p2.x, p2.y) < hi && fmaxf(rd.x, rd.y) < hi)) {  // a NaN stays one either way
         float2 mag = p2;
 #pragma unroll 1
         for (int c = 0; c < 2; ++c) {

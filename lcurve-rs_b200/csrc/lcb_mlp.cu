@@ -810,16 +810,17 @@ void launch_gemm(int cols, const CUtensorMap& ta, const CUtensorMap& tb, const G
     else launch_gemm_mode<MODE, 256>(ta, tb, g, s);
 }
 
-// Sets the dynamic shared-memory limit of every GEMM variant (needed before a
+// Sets the dynamic shared-memory limit of a GEMM variant (needed before a
 // stream capture, during which the first launch of a variant cannot set it).
-void prepare_gemm_attributes() {
-#define LCB_SMEM_ATTR(M, T) \
-    CK(cudaFuncSetAttribute(k_gemm<M, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem<T>()))
-#define LCB_SMEM_ATTRS(M) LCB_SMEM_ATTR(M, 32); LCB_SMEM_ATTR(M, 64); LCB_SMEM_ATTR(M, 128); LCB_SMEM_ATTR(M, 256)
-    LCB_SMEM_ATTRS(EPI_F32); LCB_SMEM_ATTRS(EPI_BIAS_GELU); LCB_SMEM_ATTRS(EPI_BIAS_F32);
-    LCB_SMEM_ATTRS(EPI_DGELU); LCB_SMEM_ATTRS(EPI_MSE);
-#undef LCB_SMEM_ATTRS
-#undef LCB_SMEM_ATTR
+template <int MODE>
+void prepare_gemm(int cols) {
+    auto set = [](auto* kernel, size_t bytes) {
+        CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    };
+    if (cols == 32) set(k_gemm<MODE, 32>, gemm_smem<32>());
+    else if (cols == 64) set(k_gemm<MODE, 64>, gemm_smem<64>());
+    else if (cols == 128) set(k_gemm<MODE, 128>, gemm_smem<128>());
+    else set(k_gemm<MODE, 256>, gemm_smem<256>());
 }
 
 int64_t tiles_of(int64_t M, int64_t N, int cols) { return ((M + BM - 1) / BM) * ((N + cols - 1) / cols); }
@@ -1451,7 +1452,11 @@ int lcb_surrogate_subchain(lcb_mlp* net, int64_t n, int64_t m, int d, double* y_
             if (net->sub_graph) cudaGraphExecDestroy(net->sub_graph);
             net->sub_graph = nullptr;
             net->sub_key.clear();
-            prepare_gemm_attributes();  // function attributes are set outside the capture
+            for (int l = 0; l < net->nl; ++l) {  // function attributes are set outside the capture
+                const int cols = tile_cols(n, net->out[l], net->in[l]);
+                if (l + 1 < net->nl) prepare_gemm<EPI_BIAS_GELU>(cols);
+                else prepare_gemm<EPI_BIAS_F32>(cols);
+            }
             cudaGraph_t graph;
             CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
             try {
