@@ -79,16 +79,22 @@ struct View {  // a part of another buffer
     T* as() const { return static_cast<T*>(p); }
 };
 
-// All device storage of one planned batch, parts of one allocation (carve).
+// All device storage of one planned batch, parts of one allocation (carve), but for a resident batch's
+// fluxes: they have a buffer of their own, whose size no re-plan changes, since lcb_batch_results may ask
+// for the last run's after the tables have moved.
 struct DeviceSet {
-    DevBuf arena;
+    DevBuf arena, fluxes;
+    bool resident = false;
     // the plan's tables, uploaded as one piece
     View tables, models, segs, bands, rings, eblocks, rblocks, ablocks, units, dsub0;
     // what a run clears and what it returns, so that one memset and one copy do: [egrp | aux | counter |
-    // status | ecount | results | calc]
+    // status | ecount | results | calc], a resident batch's without calc
     View work, egrp, aux, counter, status, ecount, results, calc;
     View datum, rec, pos, p64, d64, ecl, spe, spphi, sptype, spw, slfac, partial, fcomp, svda, firsthit, episum, open;
-    void release() { arena.release(); }
+    void release() {
+        arena.release();
+        fluxes.release();
+    }
 };
 
 // Page-locked staging of host arrays: two slots used in turn, so that one fills while the other's copy
@@ -254,18 +260,19 @@ std::vector<Piece> plan_tables(const lcb::Plan& P, DeviceSet& D, void* base) {
 }
 
 // Sizes of the work buffer's parts, in its order.
-std::vector<size_t> work_sizes(const lcb::Plan& P) {
+std::vector<size_t> work_sizes(const lcb::Plan& P, const DeviceSet& D) {
     const size_t nm = P.models.size();
     return {ecl_groups(P) * sizeof(unsigned), nm * lcb::kNumAux * sizeof(double), sizeof(int) * 4, nm * sizeof(int),
-            sizeof(unsigned long long) * 8, nm * 12 * sizeof(double), P.ndatum * sizeof(double)};
+            sizeof(unsigned long long) * 8, nm * 12 * sizeof(double), D.resident ? 0 : P.ndatum * sizeof(double)};
 }
 void work_views(const lcb::Plan& P, DeviceSet& D, void* base) {
     View* v[7] = {&D.egrp, &D.aux, &D.counter, &D.status, &D.ecount, &D.results, &D.calc};
     size_t off = 0, k = 0;
-    for (size_t b : work_sizes(P)) {
+    for (size_t b : work_sizes(P, D)) {
         v[k++]->p = base ? (char*)base + off : nullptr;
         off += pad256(b);
     }
+    if (D.resident) D.calc.p = D.fluxes.p;
 }
 size_t total_of(const std::vector<size_t>& v) {
     size_t t = 0;
@@ -285,7 +292,7 @@ size_t carve(const lcb_ctx* C, const lcb::Plan& P, void* base, DeviceSet& D, siz
     for (const Piece& p : plan_tables(P, D, nullptr)) tables += pad256(p.bytes);
     take(D.tables, tables);
     plan_tables(P, D, D.tables.p);
-    take(D.work, total_of(work_sizes(P)));
+    take(D.work, total_of(work_sizes(P, D)));
     work_views(P, D, D.work.p);
     take(D.datum, P.data_count * sizeof(lcb_datum));
     take(D.rec, P.nelem * sizeof(float4));
@@ -438,12 +445,14 @@ void pull(lcb_ctx* C, void* dst, const void* src, size_t bytes) {
     C->d2h += (int64_t)bytes;
 }
 
-// The status words, search counters and results of a run, and with `calc` its fluxes: one copy.
+// The status words, search counters and results of a run, and with `calc` (not a resident batch's) its
+// fluxes: one copy.
 void fetch_results(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, std::vector<double>& res, std::vector<double>* calc,
                    std::vector<int>* status, unsigned long long* ecount = nullptr) {
     const int64_t nm = (int64_t)P.models.size();
     const char* base = (const char*)D.status.p;
-    const size_t head = (const char*)D.calc.p - base, tail = calc ? P.ndatum * sizeof(double) : 0;
+    const size_t head = (const char*)D.results.p + pad256(nm * 12 * sizeof(double)) - base;
+    const size_t tail = calc ? P.ndatum * sizeof(double) : 0;
     std::vector<char>& h = C->fetched;
     const bool one = head + tail <= Staging::kSlotMax;  // else the fluxes straight into their vector
     h.resize(head + (one ? tail : 0));
@@ -949,6 +958,8 @@ int lcb_batch_create(lcb_ctx* C, const lcb_model* const* models, int64_t nmodels
         std::vector<const lcb::Model*> mp(nmodels);
         for (int64_t i = 0; i < nmodels; ++i) mp[i] = &B->models[i];
         B->tune = engine_tuning();
+        B->dev.resident = true;
+        B->dev.fluxes.ensure(total * sizeof(double));
         lcb::plan_batch(mp.data(), nmodels, B->data.data(), B->start.data(), B->count.data(), C->num_sms, B->plan,
                         B->tune);
         upload_plan(C, B->dev, B->plan);
