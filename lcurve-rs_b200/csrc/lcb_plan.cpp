@@ -20,6 +20,7 @@
 #include <cmath>
 #include <cstring>
 #include <deque>
+#include <exception>
 #include <mutex>
 #include <thread>
 #include <unordered_map>
@@ -329,6 +330,7 @@ struct BandTable {
     int nlat = 0;
     int64_t count = 0, table = -1;  // elements; first band in the plan's table (-1: not in it)
     std::vector<Band> bands;
+    std::exception_ptr error;  // why it could not be built: the models that use it fail
 };
 
 struct ModelLayout {
@@ -477,6 +479,7 @@ void prepare_model(const Model& m, const lcb_datum* data, int64_t ndata, ModelLa
         } else {  // without infill the fill counts do not enter
             const auto t = std::lower_bound(tabs->begin(), tabs->end(), nlat,
                                             [](const BandTable& a, int v) { return a.nlat < v; });
+            if (t->error) std::rethrow_exception(t->error);
             s.table = (int32_t)(t - tabs->begin());
             s.count = t->count;
             s.ntable = -1;
@@ -825,7 +828,12 @@ void plan_batch(const Model* const* models, int64_t n, const lcb_datum* data, co
         parallel_for((int64_t)nl.size(), 8, [&](int64_t k) {
             BandTable& t = tabs[k];
             t.nlat = nl[k];
-            t.count = star_bands(*models[0], true, t.nlat, false, 0.0, 0.0, 0, 0, t.bands);
+            try {
+                t.count = star_bands(*models[0], true, t.nlat, false, 0.0, 0.0, 0, 0, t.bands);
+            } catch (...) {
+                std::vector<Band>().swap(t.bands);
+                t.error = std::current_exception();
+            }
         });
     }
     auto prep = [&](int64_t i) {
