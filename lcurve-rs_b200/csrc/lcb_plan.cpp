@@ -885,7 +885,7 @@ void plan_batch(const Model* const* models, int64_t n, const lcb_datum* data, co
         D.sub_begin = sbeg[i];
         D.nsub = sbeg[i + 1] - sbeg[i];
         D.ndiv = uniform[i];
-        irregular = irregular || (P.model_ok[i] && D.nsub > 0 && !D.ndiv);
+        irregular = irregular || (P.model_ok[i] && D.ndatum > 0 && !D.ndiv);
         P.most_data = std::max(P.most_data, D.ndatum);
     }
     if (tune.datum_tables || irregular) P.datum_sub0.resize(P.ndatum);

@@ -79,3 +79,55 @@ def test_a_grid_beyond_memory_fails_its_models_alone(grids, n, big):
     ok, err = r.stdout.split("\n")[:2]
     assert ok == "1" + "0" * big + "1" * (n - 1 - big)
     assert "bad_alloc" in err
+
+
+SUBS = r"""
+#include <cstdio>
+#include <fstream>
+#include <string>
+#include <vector>
+#include "lcb_plan.h"
+using namespace lcb;
+int main(int, char** argv) {
+    std::ifstream f(argv[1], std::ios::binary);
+    std::string text((std::istreambuf_iterator<char>(f)), std::istreambuf_iterator<char>());
+    const Model m = parse_model_text(text);
+    const int ndiv[4][3] = {{2, 2, 2}, {0, 0, 0}, {0, 1, 0}, {-1, -1, -1}};
+    int bad = 0;
+    for (int which = 0; which < 5; ++which) {  // each alone, then all together
+        std::vector<const Model*> mp;
+        std::vector<lcb_datum> data;
+        std::vector<int64_t> st, cnt;
+        for (int i = 0; i < 4; ++i) {
+            if (which < 4 && i != which) continue;
+            mp.push_back(&m);
+            st.push_back((int64_t)data.size());
+            cnt.push_back(3);
+            for (int k = 0; k < 3; ++k) {
+                lcb_datum d{};
+                d.time = 0.1 * k; d.ferr = 1.0; d.weight = 1.0; d.ndiv = ndiv[i][k];
+                data.push_back(d);
+            }
+        }
+        PlanTuning t;
+        t.datum_tables = false;
+        Plan P;
+        plan_batch(mp.data(), (int64_t)mp.size(), data.data(), st.data(), cnt.data(), 148, P, t);
+        for (const ModelDev& M : P.models)
+            for (int64_t d = 0; d < M.ndatum; ++d) {
+                // first_sub reads the table for this datum: it has to have the entry
+                if (M.ndiv <= 0 && M.datum_begin + d >= (int64_t)P.datum_sub0.size()) { ++bad; continue; }
+                const int64_t j = first_sub(M, P.datum_sub0.data(), d);
+                if (j < M.sub_begin || j + std::max(data[M.data_begin + d].ndiv, 0) > M.sub_begin + M.nsub) ++bad;
+            }
+    }
+    std::printf("%d\n", bad);
+    return 0;
+}
+"""
+
+
+def test_every_datum_has_a_first_sub_phase(build):
+    """Exposures with no sub-division (the data parser takes ndiv <= 0) among or instead of others."""
+    r = subprocess.run([*map(str, build("subs", SUBS))], capture_output=True, text=True, timeout=120)
+    assert r.stdout == "0\n", (r.stdout, r.stderr)
