@@ -446,9 +446,16 @@ void pull(lcb_ctx* C, void* dst, const void* src, size_t bytes) {
 }
 
 // The status words, search counters and results of a run, and with `calc` (not a resident batch's) its
-// fluxes: one copy.
+// fluxes: one copy, through the page-locked slots or (staged = false: they may have to be allocated) straight
+// into pageable memory.
 void fetch_results(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, std::vector<double>& res, std::vector<double>* calc,
-                   std::vector<int>* status, unsigned long long* ecount = nullptr) {
+                   std::vector<int>* status, unsigned long long* ecount = nullptr, bool staged = true) {
+    auto get = [&](void* dst, const void* src, size_t bytes) {
+        if (staged) return pull(C, dst, src, bytes);
+        CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, C->stream));
+        CUDA_TRY(cudaStreamSynchronize(C->stream));
+        C->d2h += (int64_t)bytes;
+    };
     const int64_t nm = (int64_t)P.models.size();
     const char* base = (const char*)D.status.p;
     const size_t head = (const char*)D.results.p + pad256(nm * 12 * sizeof(double)) - base;
@@ -456,7 +463,7 @@ void fetch_results(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, std::vector<dou
     std::vector<char>& h = C->fetched;
     const bool one = head + tail <= Staging::kSlotMax;  // else the fluxes straight into their vector
     h.resize(head + (one ? tail : 0));
-    pull(C, h.data(), base, h.size());
+    get(h.data(), base, h.size());
     auto part = [&](const View& v) { return h.data() + ((const char*)v.p - base); };
     res.resize(nm * 12);
     std::memcpy(res.data(), part(D.results), nm * 12 * sizeof(double));
@@ -468,7 +475,7 @@ void fetch_results(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, std::vector<dou
     if (calc) {
         calc->resize(P.ndatum);
         if (one) std::memcpy(calc->data(), part(D.calc), tail);
-        else pull(C, calc->data(), D.calc.p, tail);
+        else get(calc->data(), D.calc.p, tail);
     }
     CUDA_TRY(cudaStreamSynchronize(C->stream));
 }
@@ -1365,7 +1372,7 @@ extern "C" int lcb_light_curve_noalloc(lcb_ctx* C, const lcb_model* model, const
         try {
             noalloc_upload(C, D, P, data);
             enqueue_run(C, D, P, scale, rdata, false);
-            fetch_results(C, D, P, res, &calc, &status);  // ends with a stream synchronise
+            fetch_results(C, D, P, res, &calc, &status, nullptr, false);  // ends with a stream synchronise
         } catch (...) {
             cudaStreamSynchronize(C->stream);  // no work may touch the arena after the lock is released
             throw;

@@ -161,6 +161,29 @@ int main(int, char** argv) {
 }
 """
 
+# lcb_light_curve_noalloc on a fresh context allocates nothing, whatever the size of its results.
+NOALLOC = r"""
+int main(int, char** argv) {
+    lcb_ctx* C; lcb_model* m;
+    CHECK(lcb_ctx_create(0, &C) == LCB_OK && lcb_model_parse(read(argv[1]).c_str(), &m) == LCB_OK);
+    int r = 0;
+    for (int n : {500, 20000, 60000}) {
+        const auto d = times(n);
+        std::vector<double> f(n);
+        lcb_result res;
+        auto before = calls;
+        CHECK(lcb_light_curve_noalloc(C, m, d.data(), n, 0, 1, f.data(), &res) == LCB_OK);
+        for (const char* name : {"cudaMalloc", "cudaMallocHost", "cudaFree", "cudaFreeHost", "cudaEventCreate"})
+            CHECK(calls[name] == before[name]);
+        ++r;
+        CHECK(res.chisq == r && f[0] == 1000.0 * r && f[n - 1] == 1000.0 * r + n - 1);
+    }
+    lcb_ctx_destroy(C);
+    std::printf("ok\n");
+    return 0;
+}
+"""
+
 
 @pytest.fixture(scope="module")
 def host(tmp_path_factory):
@@ -190,3 +213,7 @@ DISC = dict(r2=-1.0, nlat1f=20, nlat2f=30, nlat1c=10, nlat2c=15, add_disc=1, opa
 
 def test_results_outlive_a_replan(host):
     host("replan", RESULTS_AFTER_REPLAN, **DISC)
+
+
+def test_noalloc_allocates_nothing(host):
+    host("noalloc", NOALLOC, **DISC)
