@@ -125,10 +125,10 @@ int lcb_light_curve(lcb_ctx* ctx, const lcb_model* model, const lcb_datum* data,
  * allocator, plugin hosts that forbid allocation inside callbacks, loops that
  * cannot afford the synchronisation cudaMalloc/cudaFree may imply).
  * Same arguments, results and errors as lcb_light_curve, but every device
- * buffer lives in one fixed arena of LCB_NOALLOC_ARENA_BYTES, a file-scope
- * device array that each device loading this library holds until the process
- * exits.  Nothing is allocated on the device: a model and data set needing
- * more scratch than the arena is rejected with LCB_ERR_INVALID and a message
+ * buffer lives in one fixed arena, a file-scope device array that each device
+ * loading this library holds until the process exits: LCB_NOALLOC_ARENA_BYTES
+ * and 7 MiB for lists that are sized for their longest and not counted.  Nothing is allocated on the device: a model and data set needing
+ * more scratch than LCB_NOALLOC_ARENA_BYTES is rejected with LCB_ERR_INVALID and a message
  * giving the bytes needed (a grid element takes about 160 B, a datum about
  * 80 B, each exposure sub-division about 40 B plus 8 B per 4,096 elements).
  * Every call looks up the arena's device address on the context's device and

@@ -1307,8 +1307,11 @@ int lcb_measure_fma_peak(lcb_ctx* C, int which, double* tflops) {
 // ===========================================================================
 // The limit on a call's scratch counts the tables, element, sub-phase and result arrays.  The list of
 // open elements (4 bytes per Roche thread: at most 8 per element of 160 or more) and the epilogue's
-// sums (about one byte per datum of 76 or more) come on top, under a sixteenth of the rest.
-static constexpr size_t kNoallocArena = (size_t)LCB_NOALLOC_ARENA_BYTES + LCB_NOALLOC_ARENA_BYTES / 16 + (64u << 10);
+// sums (about one byte per datum of 76 or more) come on top, under a sixteenth of the rest; and where no
+// split search was counted, the first hits of one on a short list (first_hits, 2.9 MiB on 148 SMs).
+static constexpr size_t kNoallocHits = (size_t)(lcb::split_target(148) / 2 + lcb::kRocheBlock) * sizeof(int);
+static constexpr size_t kNoallocArena =
+    (size_t)LCB_NOALLOC_ARENA_BYTES + LCB_NOALLOC_ARENA_BYTES / 16 + kNoallocHits + (64u << 10);
 static __device__ __align__(256) unsigned char g_noalloc_arena[kNoallocArena];
 
 namespace {
@@ -1360,10 +1363,12 @@ extern "C" int lcb_light_curve_noalloc(lcb_ctx* C, const lcb_model* model, const
         DeviceSet D;  // views into the static arena: its own is never allocated
         size_t need = 0;
         const size_t total = carve(C, P, nullptr, D, &need);
-        if (need > (size_t)LCB_NOALLOC_ARENA_BYTES || total > kNoallocArena)
-            throw Error(LCB_ERR_INVALID, "lcb_light_curve_noalloc: this model and data need " + std::to_string(need) +
+        const bool over = need > (size_t)LCB_NOALLOC_ARENA_BYTES;
+        if (over || total > kNoallocArena)
+            throw Error(LCB_ERR_INVALID, "lcb_light_curve_noalloc: this model and data need " +
+                                             std::to_string(over ? need : total) +
                                              " bytes of device scratch, more than the fixed arena's " +
-                                             std::to_string((size_t)LCB_NOALLOC_ARENA_BYTES) +
+                                             std::to_string(over ? (size_t)LCB_NOALLOC_ARENA_BYTES : kNoallocArena) +
                                              "; use lcb_light_curve (or coarser grids / fewer points)");
         std::lock_guard<std::mutex> lock(g_noalloc_mu[C->device]);
         carve(C, P, noalloc_arena(), D);

@@ -86,7 +86,7 @@ bool replan_models(const Model* const* models, int64_t n, const lcb_datum* data,
 void host_copy(void* dst, const void* src, size_t bytes);
 
 // Scan threads of the split eclipse search that fill the GPU: sixteen waves of five 128-thread blocks.
-inline int64_t split_target(int num_sms) { return (int64_t)(num_sms > 1 ? num_sms : 1) * 640 * 16; }
+constexpr int64_t split_target(int num_sms) { return (int64_t)(num_sms > 1 ? num_sms : 1) * 640 * 16; }
 
 // Host FP64 helpers also used by tests of the planner.
 double host_xl1(double q);

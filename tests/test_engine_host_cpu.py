@@ -184,6 +184,35 @@ int main(int, char** argv) {
 }
 """
 
+# lcb_light_curve_noalloc refuses a call for the scratch that its limit counts, and for nothing else:
+# discs from inside the limit to beyond it, in steps of less than its slack.
+NOALLOC_LIMIT = r"""
+int main(int, char** argv) {
+    lcb_ctx* C; lcb_model* m;
+    CHECK(lcb_ctx_create(0, &C) == LCB_OK && lcb_model_parse(read(argv[1]).c_str(), &m) == LCB_OK);
+    const auto d = times(10);
+    double f[10];
+    int taken = 0, refused = 0;
+    for (int nrad = 180; nrad <= 380; ++nrad) {
+        CHECK(lcb_model_set_comp(m, "nrad", std::to_string(nrad).c_str()) == LCB_OK);
+        const int rc = lcb_light_curve_noalloc(C, m, d.data(), 10, 0, 0, f, nullptr);
+        if (rc == LCB_OK) {
+            CHECK(refused == 0);
+            ++taken;
+        } else {
+            const std::string msg = lcb_last_error();
+            CHECK(rc == LCB_ERR_INVALID && msg.find("need ") != std::string::npos);
+            CHECK(std::atoll(msg.c_str() + msg.find("need ") + 5) > (long long)LCB_NOALLOC_ARENA_BYTES);
+            ++refused;
+        }
+    }
+    CHECK(taken > 5 && refused > 5);
+    lcb_ctx_destroy(C);
+    std::printf("ok\n");
+    return 0;
+}
+"""
+
 
 @pytest.fixture(scope="module")
 def host(tmp_path_factory):
@@ -217,3 +246,7 @@ def test_results_outlive_a_replan(host):
 
 def test_noalloc_allocates_nothing(host):
     host("noalloc", NOALLOC, **DISC)
+
+
+def test_noalloc_refuses_by_its_limit_alone(host):
+    host("limit", NOALLOC_LIMIT, **{**DISC, "roche1": 1, "r1": 0.3, "rdisc2": 0.35, "rdisc1": 0.1})
