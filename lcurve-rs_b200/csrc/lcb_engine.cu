@@ -1003,16 +1003,20 @@ static void replan_batch(lcb_batch* B, bool params_only) {
     for (int64_t i = 0; i < n; ++i) mp[i] = &B->models[i];
     Range r("lcb replan");
     // parameters that change no table (a sampler's, mostly) change the model table alone
-    if (params_only && !B->broken &&
-        lcb::replan_models(mp.data(), n, B->data.data(), B->start.data(), B->count.data(), B->plan)) {
-        push(C, C->stream, B->dev.models.p, {{B->plan.models.data(), n * sizeof(lcb::ModelDev)}});
-        return;
+    const bool models_only = params_only && !B->broken &&
+                             lcb::replan_models(mp.data(), n, B->data.data(), B->start.data(), B->count.data(), B->plan);
+    bool same = models_only;
+    if (!models_only) {
+        lcb::Plan& P = B->spare;
+        lcb::plan_batch(mp.data(), n, B->data.data(), B->start.data(), B->count.data(), C->num_sms, P, B->tune);
+        same = !B->broken && P.shape_key == B->plan.shape_key;
+        std::swap(B->plan, P);
     }
-    lcb::Plan& P = B->spare;
-    lcb::plan_batch(mp.data(), n, B->data.data(), B->start.data(), B->count.data(), C->num_sms, P, B->tune);
-    const bool same = !B->broken && P.shape_key == B->plan.shape_key;
-    std::swap(B->plan, P);
     try {
+        if (models_only) {
+            push(C, C->stream, B->dev.models.p, {{B->plan.models.data(), n * sizeof(lcb::ModelDev)}});
+            return;
+        }
         upload_plan(C, B->dev, B->plan);
         if (!same) upload_data(C, B->dev, B->plan, B->data.data());
         if (!same && B->graph) {

@@ -213,6 +213,43 @@ int main(int, char** argv) {
 }
 """
 
+# New parameters whose upload fails: the batch runs on neither the old nor the new ones until it is set again.
+FAILED_UPLOAD = r"""
+int main(int, char** argv) {
+    lcb_ctx* C; lcb_model* m;
+    CHECK(lcb_ctx_create(0, &C) == LCB_OK && lcb_model_parse(read(argv[1]).c_str(), &m) == LCB_OK);
+    const int n = 300;
+    const char* name = "t0";
+    for (const char* call : {"cudaMemcpyAsync", "cudaMallocHost"}) {
+        runs = 0;
+        lcb_batch* B = batch(C, m, 3, n);
+        CHECK(B && lcb_batch_run(B, 0) == LCB_OK && holds(B, 3, n, 1, 1));
+        const double v[3] = {0.25, 0.25, 0.25};
+        lcb_ctx* other = C;
+        if (std::string(call) == "cudaMallocHost") {  // staging to be allocated yet: a fresh context's batch
+            lcb_batch_destroy(B);
+            CHECK(lcb_ctx_create(0, &other) == LCB_OK);
+            fail_call = call; fail_at = calls[call] + 1;
+            CHECK(batch(other, m, 3, n) == nullptr);  // the creation itself reports it
+            fail_call = "";
+            B = batch(other, m, 3, n);
+            CHECK(B && lcb_batch_run(B, 0) == LCB_OK);
+        }
+        fail_call = "cudaMemcpyAsync"; fail_at = calls["cudaMemcpyAsync"] + 1;
+        CHECK(lcb_batch_set_params(B, &name, 1, v) == LCB_ERR_CUDA);
+        fail_call = "";
+        CHECK(lcb_batch_run(B, 0) == LCB_ERR_INVALID);
+        CHECK(lcb_batch_set_params(B, &name, 1, v) == LCB_OK && lcb_batch_run(B, 0) == LCB_OK);
+        CHECK(holds(B, 3, n, runs + 0.25, runs));
+        lcb_batch_destroy(B);
+        if (other != C) lcb_ctx_destroy(other);
+    }
+    lcb_ctx_destroy(C);
+    std::printf("ok\n");
+    return 0;
+}
+"""
+
 
 @pytest.fixture(scope="module")
 def host(tmp_path_factory):
@@ -250,3 +287,7 @@ def test_noalloc_allocates_nothing(host):
 
 def test_noalloc_refuses_by_its_limit_alone(host):
     host("limit", NOALLOC_LIMIT, **{**DISC, "roche1": 1, "r1": 0.3, "rdisc2": 0.35, "rdisc1": 0.1})
+
+
+def test_parameters_whose_upload_failed_are_not_run(host):
+    host("upload", FAILED_UPLOAD, **DISC)
