@@ -141,6 +141,34 @@ int32_t roche_convex(double own, double spin, double ffac) {
     return spin >= 1.0 && spin <= 6.0 && (own <= 0.5 || ffac <= 0.95);
 }
 
+// Where the eclipse search, which may evaluate the potential up to `acc` beyond the ends of a chord of
+// the bounding sphere, finds it below the surface value outside the star.  On a sphere of radius r about
+// the star's centre the potential is lowest in the orbital plane, and there a function of the distance t
+// to the companion (mass m) alone, const - m (1/t + t^2/2): lowest towards the companion, highest at t = 1.
+// Along a ray it rises from the surface and falls again, so that the sphere of radius rref + acc says it
+// all: below the surface value within an angle of the companion's direction.  Sets that angle, or returns
+// 0 where there is more: the far side lies below too, or acc is half a radius or more.
+int32_t roche_pad(RocheEcl& e, double delta) {
+    const double acc = 2.0 * std::sqrt(2.0 * kTwoPi * 2.0 * e.rref * delta) * 1.001;  // no chord is longer than 2 rref
+    const double own = e.primary ? e.comp : e.mu, m = 1.0 - own, r = e.rref + acc;
+    e.pad_cos = e.pad_sin = 0.0;
+    if (!(acc < 0.5 * e.rref) || !(m > 0.0) || r >= 1.0) return 0;
+    auto h = [](double t) { return 1.0 / t + 0.5 * t * t; };
+    const double at = -own / r - 0.5 * e.ssq * r * r + 0.5 * m * (1.0 + r * r) - (e.primary ? 0.0 : m) - e.pref;
+    const double low = at / m - 1e-9;  // below the surface value where h >= low
+    if (!(h(1.0 + r) < low && h(1.0) < low)) return 0;
+    if (h(1.0 - r) < low) return 1;
+    double lo = 1.0 - r, hi = 1.0;  // h falls
+    for (int k = 0; k < 24; ++k) {
+        const double mid = 0.5 * (lo + hi);
+        if (h(mid) >= low) lo = mid; else hi = mid;
+    }
+    const double u = (1.0 + r * r - hi * hi) / (2.0 * r);
+    e.pad_cos = r * u;
+    e.pad_sin = r * std::sqrt(std::fmax(1.0 - u * u, 0.0));
+    return 1;
+}
+
 // Planck function and its log-derivative (planck.rs:4-44).
 const double kFac1 = 2.0e27 * kH * kC;
 const double kFac2 = 1.0e9 * kH * kC / kK;
@@ -391,13 +419,14 @@ void prepare_model(const Model& m, const lcb_datum* data, int64_t ndata, ModelLa
     D.gref1 = m.roche1 ? face_gravity(true, q, spin1, {-1.0, 0.0, 0.0}, D.rref1, D.pref1, D.acc_face) : 1.0;
     D.gref2 = m.roche2 ? face_gravity(false, q, spin2, {1.0, 0.0, 0.0}, D.rref2, D.pref2, D.acc_face) : 1.0;
     double mu = q / (1.0 + q);
-    D.ecl1 = RocheEcl{mu, 1.0 - mu, sq(spin1), D.rref1, D.pref1, 0.0, 0.0, 0.0, 1, roche_convex(1.0 - mu, spin1, D.ffac1)};
-    D.ecl2 = RocheEcl{mu, 1.0 - mu, sq(spin2), D.rref2, D.pref2, 1.0, 0.0, 0.0, 0, roche_convex(mu, spin2, D.ffac2)};
+    D.ecl1 = RocheEcl{mu, 1.0 - mu, sq(spin1), D.rref1, D.pref1, 0.0, 0.0, 0.0, 0.0, 0.0, 1, roche_convex(1.0 - mu, spin1, D.ffac1)};
+    D.ecl2 = RocheEcl{mu, 1.0 - mu, sq(spin2), D.rref2, D.pref2, 1.0, 0.0, 0.0, 0.0, 0.0, 0, roche_convex(mu, spin2, D.ffac2)};
     for (RocheEcl* e : {&D.ecl1, &D.ecl2}) {
         const bool first = e == &D.ecl1;
         if (!(first ? m.roche1 : m.roche2)) continue;
         e->ry = face_radius(first, q, first ? spin1 : spin2, {0.0, 1.0, 0.0}, e->rref, e->pref);
         e->rz = face_radius(first, q, first ? spin1 : spin2, {0.0, 0.0, 1.0}, e->rref, e->pref);
+        e->convex = e->convex && roche_pad(*e, D.delta);
     }
     D.roche1 = m.roche1; D.roche2 = m.roche2; D.eclipse1 = m.eclipse1; D.eclipse2 = m.eclipse2;
     D.npole = m.npole; D.glens1 = m.glens1;

@@ -530,7 +530,10 @@ LCB_HD inline bool ingress_egress(const RocheEcl& s, double cosi, double sini, d
 //   - the tangent plane there supports the star, so every line of sight on its
 //     outer side misses: all phases from the start of the scan (or its end) up
 //     to c; the reference search returns true only at a point it has evaluated
-//     inside the star, hence "false" there.  kLimbEps keeps clear of rounding.
+//     below the surface value, in the chord or within acc of it, and where the
+//     plane has the companion's well behind it as well (well_behind; else the
+//     element is left to the general path) none is, hence "false" there.
+//     kLimbEps keeps clear of rounding.
 //   - on the inner side the line dips below pref by |dphi_min/dphase| (phase -
 //     c); dbrent ends within 2 acc of the minimum along the line, so it finds
 //     a point below pref once that depth exceeds phi'' (2 acc)^2 / 2.  Twice
@@ -597,6 +600,16 @@ LCB_HD inline bool limb_applies(const RocheEcl& s, const Geom& G) {
     return s.convex && G.cq > 4.0 * G.sc.acc * G.far;
 }
 
+// Whether the plane at (x, y, z) of the star's surface, outward normal n, has on its inner side all that
+// a search may reach of the companion's well (roche_pad): then a line of sight on its outer side meets no
+// potential below the surface value, in the chord or within acc of it.
+LCB_HD inline bool well_behind(const RocheEcl& s, const double* n, double x, double y, double z) {
+    const double along = s.primary ? n[0] : -n[0], aside = sqrt(n[1] * n[1] + n[2] * n[2]);
+    const double off = n[0] * (x - s.cofmx) + n[1] * y + n[2] * z;
+    return along * s.pad_sin <= aside * s.pad_cos &&
+           off > along * s.pad_cos + aside * s.pad_sin + 1e-6 * (fabs(along) + aside);
+}
+
 // First guess of the contacts: those of the ellipsoid with the star's half
 // widths ry (for x and y) and rz.  False: the ellipsoid is not touched.
 LCB_HD inline bool limb_guess(const RocheEcl& s, const Geom& G, double& half) {
@@ -640,6 +653,7 @@ LCB_HD inline Contact limb_contact(const RocheEcl& s, const Geom& G, bool egress
     const double end = egress ? G.sc.phi2 : G.sc.phi1;
     sincos(kTwoPi * end, &sn, &cs);
     if (!(G.sini * (P.g[0] * cs - P.g[1] * sn) + G.cosi * P.g[2] > 0.0) || fabs(end - phi) > 0.45) return c;
+    if (!well_behind(s, P.g, P.x[0], P.x[1], P.x[2])) return c;
     c.phi = phi;
     c.margin = kLimbEps + 4.0 * B * sq(G.sc.acc) / fabs(A);
     c.ok = true;
@@ -683,7 +697,8 @@ LCB_HD inline int limb_lowest(const RocheEcl& s, const Geom& G, double& lo, doub
             if (fabs(over) < 1e-10) break;
             r = fmin(fmax(r - over / (P.g[0] * w[0] + P.g[1] * w[1] + P.g[2] * w[2]), 0.2 * s.rref), s.rref);
         }
-        if (fabs(over) < 1e-10 && plane_clears(G, P.g, at.px, at.py, at.pz)) return LIMB_NONE;
+        if (fabs(over) < 1e-10 && plane_clears(G, P.g, at.px, at.py, at.pz) && well_behind(s, P.g, at.px, at.py, at.pz))
+            return LIMB_NONE;
     }
     double t = -(G.sini * (cs * (G.px - s.cofmx) - sn * G.py) + G.cosi * G.pz);
     double bend = 0.0;  // of the lowest potential in phase
@@ -731,7 +746,8 @@ LCB_HD inline int limb_lowest(const RocheEcl& s, const Geom& G, double& lo, doub
         const double m = over / (P.g[0] * P.g[0] + P.g[1] * P.g[1] + P.g[2] * P.g[2]);
         at.px -= m * P.g[0]; at.py -= m * P.g[1]; at.pz -= m * P.g[2];
     }
-    return fabs(over) < 1e-10 && plane_clears(G, P.g, at.px, at.py, at.pz) ? LIMB_NONE : LIMB_OPEN;
+    return fabs(over) < 1e-10 && plane_clears(G, P.g, at.px, at.py, at.pz) && well_behind(s, P.g, at.px, at.py, at.pz)
+               ? LIMB_NONE : LIMB_OPEN;
 }
 
 struct Limb {
