@@ -381,7 +381,7 @@ void enqueue_run(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, int scale, int rd
                      D.d64.as<double4>(), D.ecl.as<double2>(), D.egrp.as<unsigned>(), D.aux.as<double>(),
                      D.status.as<int>(), nblk, nrblk, (int64_t)P.ablocks.size(),
                      D.ecount.as<unsigned long long>(), D.open.as<unsigned>(), D.counter.as<unsigned>() + 1,
-                     D.firsthit.as<int>(), (unsigned)first_hits(C, P), P.split_fix, lcb::split_target(C->num_sms),
+                     D.firsthit.as<int>(), (unsigned)first_hits(C, P), P.split_fix, P.roche_split > 1, lcb::split_target(C->num_sms),
                      C->num_sms * 5, C->fblink_cap, sz};
     if (elem) CUDA_TRY(lcb::launch_elements(ea, s));
     if (timed) CUDA_TRY(cudaEventRecord(C->ev[1], s));

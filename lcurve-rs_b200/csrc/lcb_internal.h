@@ -45,7 +45,8 @@ struct RocheEcl {          // constants of a Roche-distorted eclipsing star
     double pad_cos, pad_sin;  // (roche_pad) what the search may reach of the companion's well lies within this
                               // angle of the direction to the companion; times the farthest distance
     int32_t primary;
-    int32_t convex;        // the star is convex (roche_convex): its limb decides most of the eclipse search
+    int32_t convex;        // the star is convex (roche_convex): its limb decides most of the eclipse search,
+    int32_t wide, unused;  // or, where that reach is wide, the search of the other star's elements
 };
 
 struct SpotDev {           // Gaussian star spot (brightness.rs:187-201)

@@ -69,7 +69,7 @@ constexpr int kRocheMinBlocks = LCB_ROCHE_MIN_BLOCKS;  // k_roche blocks per SM 
 #define LCB_SCAN_MIN_BLOCKS LCB_ROCHE_MIN_BLOCKS
 #endif
 #ifndef LCB_CHOP_MIN_BLOCKS
-#define LCB_CHOP_MIN_BLOCKS LCB_ROCHE_MIN_BLOCKS
+#define LCB_CHOP_MIN_BLOCKS 4
 #endif
 constexpr int kScanMinBlocks = LCB_SCAN_MIN_BLOCKS;  // the same for the split scan (small batches)
 constexpr int kChopMinBlocks = LCB_CHOP_MIN_BLOCKS;  // and for its bisection kernel
@@ -586,7 +586,9 @@ __global__ void __launch_bounds__(kRocheBlock, kRocheMinBlocks) k_roche(ElemArgs
     bool found = false, seek = false;  // both contacts known; guesses in c.phi to try
     Contact c{0.0, 0.0, false};
     bool crosses = false;  // the bounding sphere, at some phase
-    if (valid) {
+    if (!R.convex || (R.wide && sg.kind != SEG_STAR1 && sg.kind != SEG_STAR2)) {
+        open = true;  // the whole block, so that the list keeps its order and alignment
+    } else if (valid) {
         const double4 p = A.el_p64[e];
         crosses = geom_setup(R, M.cosi_e, M.sini_e, M.delta, p.x, p.y, p.z, G);
         open = crosses && !limb_applies(R, G);
@@ -643,15 +645,23 @@ __global__ void __launch_bounds__(kRocheBlock, kRocheMinBlocks) k_roche(ElemArgs
         bits = 1u << slot;
     }
     group_or_warp(A.ecl_grp, grp, bits);
-    // open elements to the list, one atomic per warp
+    // open elements to the list, a block's in their order (neighbours search alike: fragments of a warp's
+    // 16 cost k_roche_open a fifth)
     const unsigned mine = __ballot_sync(0xffffffffu, open && !egress);
-    if (mine) {
-        const int lane = threadIdx.x & 31, src = __ffs(mine) - 1;
-        unsigned base = 0;
-        if (lane == src) base = atomicAdd(A.nopen, (unsigned)__popc(mine));
-        base = __shfl_sync(0xffffffffu, base, src);
+    if (__syncthreads_or(mine != 0u)) {
+        __shared__ unsigned found_open[kRocheBlock / 32], list_at;
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        if (lane == 0) found_open[warp] = (unsigned)__popc(mine);
+        __syncthreads();
+        unsigned before = 0, total = 0;
+        for (int w = 0; w < kRocheBlock / 32; ++w) {
+            if (w < warp) before += found_open[w];
+            total += found_open[w];
+        }
+        if (threadIdx.x == 0) list_at = atomicAdd(A.nopen, total);
+        __syncthreads();
         if ((mine >> lane) & 1u) {
-            const unsigned k = base + __popc(mine & ((1u << lane) - 1u));
+            const unsigned k = list_at + before + __popc(mine & ((1u << lane) - 1u));
             A.open[k] = (unsigned)(rb * kRocheBlock + slot);
             if (k < A.nfirst) A.firsthit[k] = kNoHit;
         }
@@ -687,10 +697,11 @@ __device__ __forceinline__ OpenElem open_elem(const ElemArgs& A, unsigned item) 
     OpenElem o;
     o.M = A.models + sg.model;
     o.R = blk.by == 1 ? &o.M->ecl1 : &o.M->ecl2;
-    o.e = sg.first + blk.offset + item % kRocheBlock;
+    const int64_t i = blk.offset + item % kRocheBlock;
+    o.e = sg.first + i;
     o.model = sg.model;
     o.slot = roche_slot(sg.kind, blk.by);
-    o.valid = LCB_IN_BOUNDS(o.e < A.sz.nelem, A.status + sg.model);
+    o.valid = i < sg.count && LCB_IN_BOUNDS(o.e < A.sz.nelem, A.status + sg.model);
     return o;
 }
 
@@ -728,20 +739,32 @@ __device__ __forceinline__ void roche_counters(const ElemArgs& A, const EclCount
     }
 }
 
-// The general search of the open elements: persistent blocks over the list.
+// The warp's next group of open elements: searches differ in length many times
+// over, so that warps take them as they come.  (Strides instead gave a block the
+// same chunk of every scan it took, the grid being a multiple of `split`: 64
+// models of stars that are not convex 4.1 instead of 1.4 ms, 512 9.7 instead of 8.2.)
+__device__ __forceinline__ unsigned next_group(unsigned* counter) {
+    unsigned w = 0;
+    if ((threadIdx.x & 31) == 0) w = atomicAdd(counter, 1u);
+    return __shfl_sync(0xffffffffu, w, 0);
+}
+
+// The general search of the open elements: persistent warps over the list.
 // Unsplit, one thread runs an element's whole search (phase scan with block
 // proofs, then both bisections).  Split, the scans' chunks are spread over
 // `split` threads an element and k_roche_chop2 bisects from the first hit: the
-// time of a short list is otherwise its longest single scan.
+// time of a short list is otherwise its longest single scan.  kSplit: the batch is
+// small enough that its lists always split (the whole search is not compiled in).
+template <bool kSplit>
 __global__ void __launch_bounds__(kRocheBlock, kScanMinBlocks) k_roche_open(ElemArgs A) {
     const unsigned n = *A.nopen;
     if (n == 0) return;
     const int split = open_split(A, n);
-    const int64_t groups = (int64_t)((n + kRocheBlock - 1) / kRocheBlock) * split;
+    const unsigned groups = (n + 31) / 32 * split;
     EclCount cnt;
     cnt.cap = A.fblink_cap;
-    for (int64_t w = blockIdx.x; w < groups; w += gridDim.x) {
-        const unsigned k = (unsigned)(w / split) * kRocheBlock + threadIdx.x;
+    for (unsigned w; (w = next_group(A.nopen + 1)) < groups;) {
+        const unsigned k = w / split * 32 + (threadIdx.x & 31);
         int64_t g = -1;
         unsigned bits = 0u;
         if (k < n) {
@@ -749,7 +772,7 @@ __global__ void __launch_bounds__(kRocheBlock, kScanMinBlocks) k_roche_open(Elem
             bool capped = false;
             if (o.valid) {
                 const double4 p = A.el_p64[o.e];
-                if (split == 1) {
+                if (!kSplit && split == 1) {
                     double a, b;
                     if (ingress_egress<true>(*o.R, o.M->cosi_e, o.M->sini_e, o.M->delta, p.x, p.y, p.z, a, b, capped, cnt)) {
                         A.el_ecl[o.slot * A.sz.nelem + o.e] = make_double2(a, b);
@@ -765,7 +788,7 @@ __global__ void __launch_bounds__(kRocheBlock, kScanMinBlocks) k_roche_open(Elem
                 if (capped) atomicOr(A.status + o.model, kStatusIterCap);
             }
         }
-        if (split == 1) group_or_warp(A.ecl_grp, g, bits);
+        if (!kSplit && split == 1) group_or_warp(A.ecl_grp, g, bits);
     }
     roche_counters(A, cnt);
 }
@@ -780,8 +803,8 @@ __global__ void __launch_bounds__(kRocheBlock, kChopMinBlocks) k_roche_chop2(Ele
     const int part = threadIdx.x & 1;  // 0: ingress, 1: egress
     EclCount cnt;
     cnt.cap = A.fblink_cap;
-    for (int64_t k0 = (int64_t)blockIdx.x * (kRocheBlock / 2); k0 < n; k0 += (int64_t)gridDim.x * (kRocheBlock / 2)) {
-        const int64_t k = k0 + (threadIdx.x >> 1);
+    for (unsigned w; (w = next_group(A.nopen + 2)) < (n + 15) / 16;) {
+        const unsigned k = w * 16 + ((threadIdx.x & 31) >> 1);
         bool capped = false, found = false;
         double a = 0.0, b = 0.0;
         OpenElem o;
@@ -2179,7 +2202,8 @@ cudaError_t launch_roche(const ElemArgs& a, cudaStream_t s) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const unsigned grid = (unsigned)std::min<int64_t>(a.open_grid, 16 * a.nrblocks);
-    k_roche_open<<<grid, kRocheBlock, 0, s>>>(a);
+    if (a.split_all) k_roche_open<true><<<grid, kRocheBlock, 0, s>>>(a);
+    else k_roche_open<false><<<grid, kRocheBlock, 0, s>>>(a);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     k_roche_chop2<<<grid, kRocheBlock, 0, s>>>(a);

@@ -32,10 +32,11 @@ struct ElemArgs {
     int64_t nblocks, nrblocks, nablocks;
     unsigned long long* counters;  // [pot evals, dpot evals, fblink calls, bound nodes, proven misses] or null
     unsigned* open;      // elements left to the general search: Roche block x kRocheBlock + slot
-    unsigned* nopen;     // their number (zeroed before k_roche)
+    unsigned* nopen;     // their number, then the next group of k_roche_open and of k_roche_chop2 (zeroed before k_roche)
     int* firsthit;       // split scan: first hit per open element, set to kNoHit as it is listed
     unsigned nfirst;     // entries of firsthit: longer lists are not split
     int split_fix;       // threads per open element in the split scan; 0: by the list's length
+    int split_all;       // a list of every Roche thread would still be split
     int64_t split_target;  // scan threads that fill the GPU
     int open_grid;       // blocks of the two general kernels
     int fblink_cap;      // potential evaluations allowed in one line-of-sight search (kFblinkEvalCap)
