@@ -1138,7 +1138,10 @@ int lcb_mlp_create(int device, int n_in, int width, int n_hidden, int n_out, int
         int64_t nsplit = 0;
         for (int l = 0; l < N->nl; ++l) {
             N->wsplit_off.push_back(nsplit);
-            nsplit += (int64_t)max_split_count(N->out[l], N->in[l], N->sms) * N->out[l] * N->in[l];
+            // a layer of more tiles than half the SMs is never split (its GEMM writes the gradient itself), so
+            // that a layer's share is at most an SM's tile each, 9.7 MB
+            const int64_t most = max_split_count(N->out[l], N->in[l], N->sms);
+            if (most > 1) nsplit += most * N->out[l] * N->in[l];
         }
         N->wsplit_off.push_back(nsplit);
         N->wsplit.alloc(nsplit);
