@@ -480,10 +480,9 @@ void fetch_results(lcb_ctx* C, DeviceSet& D, const lcb::Plan& P, std::vector<dou
     CUDA_TRY(cudaStreamSynchronize(C->stream));
 }
 
-// Device checks that fail a whole call (as opposed to one model's NaN): a bounded
-// wait that gave up, or (LCURVE_DEBUG_BOUNDS build) an index out of range.
+// Device checks that fail a whole call (as opposed to one model's NaN): in the
+// LCURVE_DEBUG_BOUNDS build an index out of range.
 void check_device_status(int st) {
-    if (st & lcb::kStatusTmaTimeout) throw Error(LCB_ERR_DEVICE_CHECK, "a bounded device wait timed out");
     if (st & lcb::kStatusBounds) throw Error(LCB_ERR_DEVICE_CHECK, "a device-side bounds check failed");
 }
 
@@ -743,7 +742,7 @@ int lcb_model_grid(lcb_ctx* C, const lcb_model* model, int which, int64_t* n, do
         d.time = 0.0; d.expose = 0.0; d.ferr = 1.0; d.weight = 1.0; d.ndiv = 1;
         int64_t st = 0, cnt = 1;
         lcb::Plan P;
-        lcb::plan_batch(&mp, 1, &d, &st, &cnt, C->num_sms, P);
+        lcb::plan_batch(&mp, 1, &d, &st, &cnt, C->num_sms, P, engine_tuning());
         if (!P.model_ok[0]) throw Error(LCB_ERR_MODEL, P.model_err[0]);
         const lcb::SegDesc* g = nullptr;
         for (const auto& sg : P.segs) {
@@ -806,7 +805,7 @@ int lcb_model_elements(lcb_ctx* C, const lcb_model* model, int64_t first, int64_
         d.ferr = 1.0; d.weight = 1.0; d.ndiv = 1;
         int64_t st = 0, cnt = 1;
         lcb::Plan& P = C->plan;
-        lcb::plan_batch(&mp, 1, &d, &st, &cnt, C->num_sms, P);
+        lcb::plan_batch(&mp, 1, &d, &st, &cnt, C->num_sms, P, engine_tuning());
         if (!P.model_ok[0]) throw Error(LCB_ERR_MODEL, P.model_err[0]);
         *total = P.nelem;
         if (!rec_dev) return;
@@ -859,7 +858,7 @@ int lcb_light_curve_elements(lcb_ctx* C, const lcb_model* model, const lcb_datum
         const lcb::Model* mp = &model->m;
         int64_t st = 0, cnt = n;
         lcb::Plan& P = C->plan;
-        lcb::plan_batch(&mp, 1, data, &st, &cnt, C->num_sms, P);
+        lcb::plan_batch(&mp, 1, data, &st, &cnt, C->num_sms, P, engine_tuning());
         if (!P.model_ok[0]) throw Error(LCB_ERR_MODEL, P.model_err[0]);
         upload_plan(C, C->scratch, P);
         upload_data(C, C->scratch, P, data);
@@ -1245,7 +1244,7 @@ int lcb_model_work(const lcb_model* model, const lcb_datum* data, int64_t n, int
         const lcb::Model* mp = &model->m;
         int64_t st = 0, cnt = n;
         lcb::Plan P;
-        lcb::plan_batch(&mp, 1, data, &st, &cnt, 148, P);
+        lcb::plan_batch(&mp, 1, data, &st, &cnt, 148, P, engine_tuning());
         const bool ok = !P.model_ok.empty() && P.model_ok[0];
         int64_t v[4] = {ok ? P.nelem : 0, ok ? P.roche_elems : 0, ok ? P.nsub : 0, ok ? P.evals : 0};
         std::memcpy(out4, v, sizeof v);
@@ -1361,7 +1360,7 @@ extern "C" int lcb_light_curve_noalloc(lcb_ctx* C, const lcb_model* model, const
     return guarded(C, [&] {
         const lcb::Model* mp = &model->m;
         int64_t st = 0, cnt = n;
-        lcb::Plan P;
+        lcb::Plan P;  // with the table of first sub-phases, regular data or not: it is part of what the limit counts
         lcb::plan_batch(&mp, 1, data, &st, &cnt, C->num_sms, P);
         if (!P.model_ok[0]) throw Error(LCB_ERR_MODEL, P.model_err[0]);
         DeviceSet D;  // views into the static arena: its own is never allocated

@@ -962,7 +962,8 @@ __global__ void k_phase(PhaseArgs A) {
 }
 
 // ---------------------------------------------------------------------------
-// bounded waits
+// k_wait_probe: a bounded wait that runs out (no kernel of a light curve waits;
+// the surrogate's GEMMs have the same bounded waits of their own)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -977,10 +978,9 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait: gives up after `limit` SM clock cycles (by default about 2 s);
-// on time-out the caller records an error status instead of hanging.
-constexpr long long kWaitLimit = 4000000000LL;
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long long limit = kWaitLimit) {
+// Bounded wait: gives up after `limit` SM clock cycles; on time-out the caller
+// records an error status instead of hanging.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long long limit) {
     if (mbar_test(bar, parity)) return true;
     long long t0 = clock64();
     while (!mbar_test(bar, parity)) {
@@ -2215,8 +2215,6 @@ cudaError_t launch_aux(const ElemArgs& a, cudaStream_t s) {
     k_aux<<<(unsigned)a.nablocks, kElemThreads, 0, s>>>(a);
     return cudaGetLastError();
 }
-
-int roche_block_size() { return kRocheBlock; }
 
 cudaError_t launch_flux(const FluxArgs& a, int grid, cudaStream_t s) {
     if (a.nunits <= 0) return cudaSuccess;

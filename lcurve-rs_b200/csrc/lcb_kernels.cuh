@@ -101,7 +101,6 @@ cudaError_t launch_phase(const PhaseArgs& a, cudaStream_t s);
 cudaError_t launch_elements(const ElemArgs& a, cudaStream_t s);
 cudaError_t launch_roche(const ElemArgs& a, cudaStream_t s);
 cudaError_t launch_aux(const ElemArgs& a, cudaStream_t s);
-int roche_block_size();
 cudaError_t launch_flux(const FluxArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_epilogue(const EpiArgs& a, cudaStream_t s);
 int flux_blocks_per_sm();
