@@ -42,8 +42,9 @@ struct RocheEcl {          // constants of a Roche-distorted eclipsing star
     double rref, pref;     // reference sphere (surface.rs:14-39)
     double cofmx;          // 0 (primary) or 1 (secondary)
     double ry, rz;         // the surface's distance from the centre along y and z
-    double pad_cos, pad_sin;  // (roche_pad) what the search may reach of the companion's well lies within this
-                              // angle of the direction to the companion; times the farthest distance
+    // what the search may reach of the companion's well (roche_pad): towards the companion between pad_near
+    // and pad_far from the centre, aside up to pad_sin, there (on its rim) pad_cos towards the companion
+    double pad_near, pad_far, pad_cos, pad_sin;
     int32_t primary;
     int32_t convex;        // the star is convex (roche_convex): its limb decides most of the eclipse search,
     int32_t wide, unused;  // or, where that reach is wide, the search of the other star's elements

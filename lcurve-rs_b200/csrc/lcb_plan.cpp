@@ -151,7 +151,9 @@ int32_t roche_convex(double own, double spin, double ffac) {
 int32_t roche_pad(RocheEcl& e, double delta) {
     const double acc = 2.0 * std::sqrt(2.0 * kTwoPi * 2.0 * e.rref * delta) * 1.001;  // no chord is longer than 2 rref
     const double own = e.primary ? e.comp : e.mu, m = 1.0 - own, r = e.rref + acc;
-    e.pad_cos = e.pad_sin = 0.0;
+    constexpr double kClear = 1e-5;  // of a plane to the well: far above a contact's last Newton step
+    e.pad_near = 0.0;
+    e.pad_far = e.pad_cos = e.pad_sin = kClear;
     if (!(acc < 0.5 * e.rref) || !(m > 0.0) || r >= 1.0) return 0;
     auto h = [](double t) { return 1.0 / t + 0.5 * t * t; };
     const double at = -own / r - 0.5 * e.ssq * r * r + 0.5 * m * (1.0 + r * r) - (e.primary ? 0.0 : m) - e.pref;
@@ -167,8 +169,10 @@ int32_t roche_pad(RocheEcl& e, double delta) {
         if (h(mid) >= low) lo = mid; else hi = mid;
     }
     const double u = (1.0 + r * r - hi * hi) / (2.0 * r);
-    e.pad_cos = r * u;
-    e.pad_sin = r * std::sqrt(std::fmax(1.0 - u * u, 0.0));
+    e.pad_far = r + kClear;
+    e.pad_near = e.rref * u - kClear;
+    e.pad_cos = r * u + kClear;
+    e.pad_sin = r * std::sqrt(std::fmax(1.0 - u * u, 0.0)) + kClear;
     return 1;
 }
 
@@ -422,8 +426,8 @@ void prepare_model(const Model& m, const lcb_datum* data, int64_t ndata, ModelLa
     D.gref1 = m.roche1 ? face_gravity(true, q, spin1, {-1.0, 0.0, 0.0}, D.rref1, D.pref1, D.acc_face) : 1.0;
     D.gref2 = m.roche2 ? face_gravity(false, q, spin2, {1.0, 0.0, 0.0}, D.rref2, D.pref2, D.acc_face) : 1.0;
     double mu = q / (1.0 + q);
-    D.ecl1 = RocheEcl{mu, 1.0 - mu, sq(spin1), D.rref1, D.pref1, 0.0, 0.0, 0.0, 0.0, 0.0, 1, roche_convex(1.0 - mu, spin1, D.ffac1), 0, 0};
-    D.ecl2 = RocheEcl{mu, 1.0 - mu, sq(spin2), D.rref2, D.pref2, 1.0, 0.0, 0.0, 0.0, 0.0, 0, roche_convex(mu, spin2, D.ffac2), 0, 0};
+    D.ecl1 = RocheEcl{mu, 1.0 - mu, sq(spin1), D.rref1, D.pref1, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 1, roche_convex(1.0 - mu, spin1, D.ffac1), 0, 0};
+    D.ecl2 = RocheEcl{mu, 1.0 - mu, sq(spin2), D.rref2, D.pref2, 1.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0, roche_convex(mu, spin2, D.ffac2), 0, 0};
     for (RocheEcl* e : {&D.ecl1, &D.ecl2}) {
         const bool first = e == &D.ecl1;
         if (!(first ? m.roche1 : m.roche2)) continue;
@@ -1064,7 +1068,8 @@ void plan_batch(const Model* const* models, int64_t n, const lcb_datum* data, co
         const int64_t e = std::max<int64_t>(total / units, 1) / kFluxTile;
         return (std::min<int64_t>(std::max<int64_t>(e, kFluxChunk), 16 * kFluxChunk) + kFluxChunk - 1) / kFluxChunk * kFluxChunk;
     };
-    // a warp per unit where every resident warp (20 per SM) gets several, else a block per unit
+    // ranges for about 120 units an SM; a warp per unit where that gives at least 80, five to each of an
+    // SM's 16 resident warps, else a block per unit
     int64_t erange = range(sms * 20 * 6);
     P.flux_share = total / (erange * kFluxTile) < sms * 20 * 4;
     if (P.flux_share) erange = range(sms * 4 * 8);

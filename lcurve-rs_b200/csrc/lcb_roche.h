@@ -600,14 +600,21 @@ LCB_HD inline bool limb_applies(const RocheEcl& s, const Geom& G) {
     return s.convex && G.cq > 4.0 * G.sc.acc * G.far;
 }
 
-// Whether the plane at (x, y, z) of the star's surface, outward normal n, has on its inner side all that
+// Whether the star's tangent plane through (x, y, z), outward normal n, has on its inner side all that
 // a search may reach of the companion's well (roche_pad): then a line of sight on its outer side meets no
 // potential below the surface value, in the chord or within acc of it.
+LCB_ROCHE_CALL bool well_behind_rim(const RocheEcl& s, double along, double n1, double n2, double off) {
+    const double aside = sqrt(n1 * n1 + n2 * n2);
+    if (!(along > 0.0)) return off > along * s.pad_near + aside * s.pad_sin;
+    return along * s.pad_sin <= aside * s.pad_cos && off > along * s.pad_cos + aside * s.pad_sin;
+}
+// First by a box about the well, which does for most; then by its rim, the farthest of it towards a plane
+// whose normal is farther from the companion's direction than the rim.
 LCB_HD inline bool well_behind(const RocheEcl& s, const double* n, double x, double y, double z) {
-    const double along = s.primary ? n[0] : -n[0], aside = sqrt(n[1] * n[1] + n[2] * n[2]);
+    const double along = s.primary ? n[0] : -n[0], aside = fabs(n[1]) + fabs(n[2]);  // at least the normal's part
     const double off = n[0] * (x - s.cofmx) + n[1] * y + n[2] * z;
-    return along * s.pad_sin <= aside * s.pad_cos &&
-           off > along * s.pad_cos + aside * s.pad_sin + 1e-6 * (fabs(along) + aside);
+    return off > along * (along > 0.0 ? s.pad_far : s.pad_near) + aside * s.pad_sin ||
+           well_behind_rim(s, along, n[1], n[2], off);
 }
 
 // First guess of the contacts: those of the ellipsoid with the star's half
@@ -653,7 +660,7 @@ LCB_HD inline Contact limb_contact(const RocheEcl& s, const Geom& G, bool egress
     const double end = egress ? G.sc.phi2 : G.sc.phi1;
     sincos(kTwoPi * end, &sn, &cs);
     if (!(G.sini * (P.g[0] * cs - P.g[1] * sn) + G.cosi * P.g[2] > 0.0) || fabs(end - phi) > 0.45) return c;
-    if (!well_behind(s, P.g, P.x[0], P.x[1], P.x[2])) return c;
+    if (!well_behind(s, P.g, G.px, G.py, G.pz)) return c;  // the plane goes through the element
     c.phi = phi;
     c.margin = kLimbEps + 4.0 * B * sq(G.sc.acc) / fabs(A);
     c.ok = true;

@@ -60,7 +60,7 @@ int main(int argc, char** argv) {  // model file, models, log10 of the least and
         const ModelDev& D = P.models[0];
         const RocheEcl& s = by == 1 ? D.ecl1 : D.ecl2;
         if (!s.convex) continue;
-        const double half = std::atan2(s.pad_sin, s.pad_cos);
+        const double half = s.pad_far > s.rref ? std::asin(s.pad_sin / s.pad_far) : 0.0;  // or no such cap
         for (int i = 0; i < 1500; ++i) {  // a disc's and a gas stream's elements
             const double a = kTwoPi * U(g), r = l1 * (0.03 + 0.95 * U(g));
             double p[3] = {r * std::cos(a), r * std::sin(a), 0.15 * r * (2 * U(g) - 1)};
@@ -82,7 +82,7 @@ int main(int argc, char** argv) {  // model file, models, log10 of the least and
             const Los L{s.cofmx + (by == 1 ? r : -r) * std::cos(w), r * std::sin(w) * std::cos(az), r * std::sin(w) * std::sin(az), 0, 0, 0};
             if (los_pot(s, L, 0.0) > s.pref) continue;
             ++low;
-            outside += w > half;  // half is 0 where there is no such cap
+            outside += w > half;
         }
     }
     std::printf("total %ld hidden %ld open %ld bad %ld low %ld outside %ld\n", total, hidden, open, bad, low, outside);
