@@ -224,8 +224,10 @@ __device__ int disc_eclipse(const ModelDev& M, double rdisc1, double px, double 
 // radius lies on; away from the root by more than `tol` (the rounding of its
 // own potential evaluation, thousands of times over) the root tells, so the ~25
 // evaluations of two square roots and divisions each become ~5 of two
-// reciprocal square roots, and the radii keep their bits.  Not converged, or
-// too flat to trust (near L1): tol is infinite and every step evaluates.
+// reciprocal square roots, and the steps decide alike: the radius is the same
+// to the bit where they are taken one by one, to a unit or two in the last
+// place where `bisected` computes their end.  Not converged, or too flat to
+// trust (near L1): tol is infinite and every step evaluates.
 struct FaceRoot {
     double r, tol;
 };
@@ -1229,7 +1231,7 @@ __device__ __forceinline__ float rcp_normal(float x) {
 // Quotients and square roots, two at a time, of arguments far from the ends of
 // the range: a hardware estimate and one Newton correction from its exact FMA
 // residual (Markstein 1990), which rounds as / and sqrtf round but for a quotient
-// within the estimate's error squared (~2^-44) of a tie: one of 2.7 10^8 random ones.
+// within the estimate's error squared (~2^-44) of a tie.
 // The general ones test each argument for the ends; the generic stars' terms are
 // bound by issue slots, and by the special-function unit where they are lensed,
 // so a square root's estimate serves the divisions by it as well.  Beaming alone,
