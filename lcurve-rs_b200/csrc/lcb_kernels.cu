@@ -755,18 +755,20 @@ __device__ __forceinline__ unsigned next_group(unsigned* counter) {
 // Unsplit, one thread runs an element's whole search (phase scan with block
 // proofs, then both bisections).  Split, the scans' chunks are spread over
 // `split` threads an element and k_roche_chop2 bisects from the first hit: the
-// time of a short list is otherwise its longest single scan.  kSplit: the batch is
+// time of a short list is otherwise its longest single scan.  Every element's
+// first chunk comes before any second one: like work lies together, and a chunk
+// finds the hits of those before it (eight models: 0.24 -> 0.21 ms).  kSplit: the batch is
 // small enough that its lists always split (the whole search is not compiled in).
 template <bool kSplit>
 __global__ void __launch_bounds__(kRocheBlock, kScanMinBlocks) k_roche_open(ElemArgs A) {
     const unsigned n = *A.nopen;
     if (n == 0) return;
     const int split = open_split(A, n);
-    const unsigned groups = (n + 31) / 32 * split;
+    const unsigned lists = (n + 31) / 32, groups = lists * split;
     EclCount cnt;
     cnt.cap = A.fblink_cap;
     for (unsigned w; (w = next_group(A.nopen + 1)) < groups;) {
-        const unsigned k = w / split * 32 + (threadIdx.x & 31);
+        const unsigned chunk = w / lists, k = (w - chunk * lists) * 32 + (threadIdx.x & 31);
         int64_t g = -1;
         unsigned bits = 0u;
         if (k < n) {
@@ -783,7 +785,7 @@ __global__ void __launch_bounds__(kRocheBlock, kScanMinBlocks) k_roche_open(Elem
                     }
                 } else {
                     const int fbl = cnt.fbl;  // k_roche_chop2 counts the reference's scan searches
-                    scan_chunk(*o.R, o.M->cosi_e, o.M->sini_e, o.M->delta, p.x, p.y, p.z, (int)(w % split), split,
+                    scan_chunk(*o.R, o.M->cosi_e, o.M->sini_e, o.M->delta, p.x, p.y, p.z, (int)chunk, split,
                                A.firsthit + k, capped, cnt);
                     cnt.fbl = fbl;
                 }
