@@ -193,8 +193,9 @@ int lcb_chisq_batch_ragged(lcb_ctx* ctx, const lcb_model* const* models, int64_t
  * lcb_batch_set_params changes physical parameters (names x values, row-major,
  * one row per model) without re-uploading data; lcb_batch_run evaluates on the
  * device (the launch sequence is captured once in a CUDA graph and replayed);
- * lcb_batch_results copies results back.  Changing a parameter that alters an
- * element count (disc/edge sizes) re-plans the batch transparently. */
+ * lcb_batch_results copies the last run's results back.  Changing a parameter
+ * that alters an element count (disc/edge sizes) re-plans the batch
+ * transparently; the last run's results stay until the next run. */
 int  lcb_batch_create(lcb_ctx* ctx, const lcb_model* const* models, int64_t nmodels,
                       const lcb_datum* data, const int64_t* offsets, lcb_batch** out);
 void lcb_batch_destroy(lcb_batch* b);
